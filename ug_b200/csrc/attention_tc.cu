@@ -150,7 +150,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer --
-    if (lane == 0) {
+    if (elect_one()) {
       int g = 0;
       bool alive = true;
       int idx = blockIdx.x;
@@ -192,7 +192,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer --
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = make_idesc(BQ, BKV, false);          // Q and K both K-major (rows of 64 dims)
       const uint32_t idesc_o = make_idesc(BQ, DV, true);            // P K-major, V MN-major ([key][dim] rows)
       bool alive = true;

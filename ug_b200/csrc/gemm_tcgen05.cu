@@ -217,7 +217,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer --
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool alive = true;
@@ -279,7 +279,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // -------------------------------------------------------- MMA issuer --
-    if (lane == 0 && rank == 0) {
+    // One elected lane (elect.sync, not lane == 0: see elect_one).
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc = make_idesc(TILE_M, BN, !p.b_is_nk, p.f16 != 0);
       auto mma = [&](uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t acc_in) {
         if constexpr (PAIR) umma_bf16_pair(d, a_desc, b_desc, idesc, acc_in);
@@ -289,6 +290,13 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if constexpr (PAIR) umma_commit_pair(bar);
         else umma_commit(bar);
       };
+      // Descriptors of ring stage 0; a stage or a k step only moves their start address (units of 16 bytes, and the
+      // ring ends below the 256 KiB the field reaches).  A, and B when k-major: rows of 128 B, 8-row groups 1024 B
+      // apart; a k step of 16 elements moves 32 B inside the swizzled row.  B n-major: 64-wide n chunks 8 KiB apart
+      // (LBO), 8-k groups 1024 B apart (SBO); a k step moves 16 rows of 128 B.
+      const uint64_t a_desc0 = make_smem_desc(smem_u32(smem), 0, 1024);
+      const uint64_t b_desc0 = make_smem_desc(smem_u32(smem) + A_BYTES, p.b_is_nk ? 0 : 64 * BK * 2, 1024);
+      const uint32_t b_step = p.b_is_nk ? UMMA_K * 2 >> 4 : UMMA_K * 128 >> 4;
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool alive = true;
@@ -305,19 +313,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if (!mbar_wait(smem_u32(&full[stage]), phase, abort_flag, p.status, 3)) { alive = false; break; }
           if (tile == cta0) UGB_TC_STAMP(UGB_TC_PROF_KBLOCK0 + (kb - kb0));
           tcgen05_fence_after();
-          const uint32_t a_addr = smem_u32(smem + stage * STAGE_BYTES);
-          const uint32_t b_addr = a_addr + A_BYTES;
+          const uint64_t a_desc = a_desc0 + (uint32_t)stage * (STAGE_BYTES >> 4);
+          const uint64_t b_desc = b_desc0 + (uint32_t)stage * (STAGE_BYTES >> 4);
 #pragma unroll
-          for (int j = 0; j < BK / UMMA_K; ++j) {
-            // A, and B when k-major: rows of 128 B, 8-row groups 1024 B apart; a
-            // k step of 16 bf16 moves 32 B inside the swizzled row.
-            const uint64_t a_desc = make_smem_desc(a_addr + j * (UMMA_K * 2), 0, 1024);
-            // B n-major: 64-wide n chunks 8 KiB apart (LBO), 8-k groups 1024 B
-            // apart (SBO); a k step of 16 moves 16 rows of 128 B.
-            const uint64_t b_desc = p.b_is_nk ? make_smem_desc(b_addr + j * (UMMA_K * 2), 0, 1024)
-                                              : make_smem_desc(b_addr + j * (UMMA_K * 128), 64 * BK * 2, 1024);
-            mma(d_tmem, a_desc, b_desc, (kb > kb0 || j > 0) ? 1u : 0u);
-          }
+          for (int j = 0; j < BK / UMMA_K; ++j)
+            mma(d_tmem, a_desc + j * (UMMA_K * 2 >> 4), b_desc + j * b_step, (kb > kb0 || j > 0) ? 1u : 0u);
           commit(smem_u32(&empty[stage]));           // frees the smem stage when the MMAs retire
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
