@@ -1,0 +1,21 @@
+// Interface of the product kernel for few rows (gemm_skinny.cu).
+#pragma once
+#include "gemm_tcgen05.cuh"
+
+constexpr int UGB_SKINNY_ROWS = 8;      // most rows of A it takes
+constexpr int UGB_SKINNY_SPLITS = 8;     // most partials it writes
+
+// Whether a decode step of `rows` rows runs its products on this kernel.  Measured at 8 rows: a 2048 x 2048 projection
+// takes 2.5 us in the chain of a step against 4.5 on 64-row tcgen05 tiles; beyond 8 rows the activations no longer fit
+// the registers beside the weights in flight (with half of those in flight 16 rows took 1.22 ms a step against 1.16).
+inline bool ugb_skinny_rows(size_t rows) { return rows >= 1 && rows <= (size_t)UGB_SKINNY_ROWS; }
+
+// k splits of a product with a f32 result that the consumer sums: 2048 inputs or fewer each, more where the columns alone do
+// not fill the SMs.
+int ugb_skinny_splits(int sm_count, size_t n, size_t k);
+
+// out = A . W^T for up to 8 rows, arguments and epilogues as ugb_tc_gemm (no rope, no n-major B, no pair_k); `splits` as
+// given, rounded as ugb_skinny_effective_splits says.  Grouped rows: tiles of g.tile_m rows of which the first
+// `rows_per_tile` may hold something; m is their total.  UGB_ERR_UNSUPPORTED (last_error untouched) for what it does not take.
+int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &g, int rows_per_tile = 0);
+int ugb_skinny_effective_splits(size_t k, int splits);

@@ -26,6 +26,7 @@
 
 #include "attention_tc.cuh"
 #include "decode_kernels.cuh"
+#include "gemm_skinny.cuh"
 #include "gemm_tcgen05.cuh"
 #include "grouped_attention.cuh"
 #include "hybrid_engine.cuh"
@@ -76,6 +77,10 @@ int32_t ugb_hybrid_matmul(ugb_hybrid *m, const Mat &x) {
   if (x.silu_mul) g.c_ld = x.c_ld == x.n / 2 ? 0 : (long long)x.c_ld;
   g.splits = x.splits; g.bn = x.bn; g.b_static = x.groups == nullptr; g.pdl = m->pdl != 0; g.late_trigger = true;
   g.groups = x.groups; g.n_groups = x.n_groups; g.tile_m = x.tile;
+  if (ugb_skinny_rows(x.groups ? (size_t)x.tile_rows : x.m)) {
+    const int32_t rc = ugb_skinny_gemm(dev, g, x.tile_rows);
+    if (rc != UGB_ERR_UNSUPPORTED) return rc;
+  }
   g.smem_kib = x.m <= 64 || (x.groups && x.tile == 64) ? 144 : 0;
   if (!x.f32_out && !x.groups && x.batch == 1 && x.nk && x.m <= 64 && x.k >= 256) {
     // a T result cannot be split into partials: the two k halves of a tile on a pair of CTAs, with the narrowest tile that fits the SMs
@@ -99,6 +104,7 @@ int32_t ugb_hybrid_matmul(ugb_hybrid *m, const Mat &x) {
 // As many CTAs as SMs, no fewer than two k blocks each
 Tiling ugb_hybrid_tile(const ugb_hybrid *m, size_t n, size_t k) {
   if (m->f32 || m->batch > 64) return {0, 1};
+  if (ugb_skinny_rows(m->batch)) return {0, ugb_skinny_splits(m->dev->sm_count, n, k)};
   // A CTA's time goes with its k blocks and hardly with its tile width (an MMA of 64 rows costs the same up to 160
   // columns), so: the fewest k blocks per CTA over widths and splits that fit one wave, then the fewest partials,
   // then the narrowest tile.

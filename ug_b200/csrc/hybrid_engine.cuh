@@ -78,6 +78,7 @@ struct ugb_hybrid_mat {            // out[b, m, n] = a . w
   bool silu_mul = false;           // columns are (gate, up) pairs; T result of n / 2 columns
   const int *groups = nullptr;     // rows in tiles of `tile`, tile i against weights groups[i]
   int tile = 0, n_groups = 0;
+  int tile_rows = 0;               // rows of a tile that may hold something (0: all)
   int splits = 1, bn = 0;
 };
 

@@ -259,6 +259,7 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
       }
       Mat g{w.xmid, w.xin, L.x_up, xrows, 2 * (size_t)L.ef, (size_t)wl};
       g.groups = w.map; g.n_groups = d.experts; g.tile = tile;
+      g.tile_rows = decode ? rows : 0;                       // a token chooses an expert once
       g.bn = tile == 64 ? 128 : 256;
       if (m->on(UGB_HYBRID_K_EXPERT_UP) && (rc = gated_product(m, w, g))) return rc;
       g.out = w.xout; g.a = w.xmid; g.w = L.x_down; g.n = wl; g.k = L.ef;

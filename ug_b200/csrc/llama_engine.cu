@@ -29,6 +29,7 @@
 
 #include "decode_kernels.cuh"
 #include "engine_core.cuh"
+#include "gemm_skinny.cuh"
 #include "gemm_tcgen05.cuh"
 #include "tp_kernels.cuh"
 #include "attention_tc.cuh"
@@ -129,6 +130,9 @@ int32_t put_vector(ugb_llama *m, const ugb_slice *w, float *dst, size_t n, const
   return UGB_OK;
 }
 
+// Few rows run on the register-streaming kernel; option gemm_profile asks for the tcgen05 kernel's timeline.
+bool skinny(const ugb_llama *m, size_t rows) { return ugb_skinny_rows(rows) && !m->gemm_prof; }
+
 // out[rows, n] = a[rows, k] . w[n, k]^T on the tensor-core kernel (weights are the static operand).
 int32_t gemm_rows(ugb_llama *m, size_t rows, void *out, const __nv_bfloat16 *a, const __nv_bfloat16 *w, size_t n,
                   size_t k, int epi, int splits, int bn, const ugb_tc_rope_epilogue *rope = nullptr, int *query_grid = nullptr,
@@ -142,6 +146,12 @@ int32_t gemm_rows(ugb_llama *m, size_t rows, void *out, const __nv_bfloat16 *a, 
   g.a_batch = 0; g.b_batch = 0; g.b_is_nk = true;
   g.epi = epi; g.splits = splits; g.bn = bn; g.b_static = true; g.pdl = m->pdl != 0;
   g.smem_kib = rows <= 64 ? m->gemm_smem_kib : 0;
+  if (skinny(m, rows)) {
+    g.late_trigger = true;              // see early_ok in llama_step
+    const int32_t rc = ugb_skinny_gemm(m->dev, g);
+    if (rc != UGB_ERR_UNSUPPORTED) return rc;
+    g.late_trigger = false;
+  }
   if (m->gemm_prof && rows <= 64) {     // qkv, o, gate|up, down, lm_head
     const int kind = epi == UGB_EPI_SILU_MUL_BF16 ? 2 : n == (size_t)m->qkv_dim ? 0 : n == (size_t)m->vl ? 4 : k == (size_t)m->lc.ffn ? 3 : 1;
     g.prof = m->gemm_prof + (size_t)kind * UGB_TC_PROF_SLOTS;
@@ -160,6 +170,11 @@ int32_t gemm_rows(ugb_llama *m, size_t rows, void *out, const __nv_bfloat16 *a, 
   if (rc == UGB_ERR_UNSUPPORTED)
     return ugb_fail(m->dev, rc, "GEMM m=%zu n=%zu k=%zu does not meet the tensor-core kernel's shape rules", rows, n, k);
   return rc;
+}
+
+// Partials that a step's projection writes for the split factor `option`.
+int step_splits(const ugb_llama *m, size_t n, size_t k, int option) {
+  return skinny(m, m->batch) ? ugb_skinny_splits(m->dev->sm_count, n, k) : ugb_tc_gemm_effective_splits(k, option);
 }
 
 int32_t gemm(ugb_llama *m, void *out, const __nv_bfloat16 *a, const __nv_bfloat16 *w, size_t n, size_t k,
@@ -398,9 +413,8 @@ int32_t llama_step(ugb_llama *m, const int *tok) {
   cudaError_t e = ugb_launch(embed_gather_kernel, dim3(B), dim3(256), 0, st, pdl, m->embed, tok, m->x, H, c.vocab, dev->status_dev, 1, 1, 0);
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of embed_gather_kernel failed: %s", cudaGetErrorString(e));
   if ((rc = ugb_after_launch(dev, "embed_gather_kernel"))) return rc;
-  const int s_qkv = ugb_tc_gemm_effective_splits(H, m->splits_qkv);
-  const int s_o = ugb_tc_gemm_effective_splits(AW, m->splits_o);
-  const int s_down = ugb_tc_gemm_effective_splits(c.ffn, m->splits_down);
+  const int s_qkv = step_splits(m, m->qkv_dim, H, m->splits_qkv), s_o = step_splits(m, H, AW, m->splits_o);
+  const int s_down = step_splits(m, H, c.ffn, m->splits_down);
   const float scale = powf((float)c.head_dim, -0.5f);   // model.rs:236
   float *po = o_out(m, m->part), *pd = down_out(m, m->part);
   // Work done before griddepcontrol.wait (the attention kernel's K/V ring, the norm kernel's residual row)
@@ -412,31 +426,34 @@ int32_t llama_step(ugb_llama *m, const int *tok) {
   // everything before it -- the writer included -- has completed.  Both facts are taken from the launches
   // themselves (the grid each projection gets, the residency the occupancy calculator gives its kernel with
   // its shared memory), not from the tuning options, so a retune that breaks the argument switches this off.
+  // Up to 8 rows the projections let their successor start only after their own wait has returned, and one of them
+  // comes right before every kernel that reads ahead: everything before that projection has completed.
   const int sms = dev->sm_count;
   int c_qkv = 0, c_o = 0, c_gu = 0, c_down = 0, o_qkv = 0, o_o = 0, o_gu = 0, o_down = 0;
   bool early = m->att_early && m->pdl && m->skip == 0;
-  if (early) {
+  const bool few = skinny(m, B);
+  if (early && !few) {
     const LayerW &w0 = m->layers[0];
-    if (gemm_rows(m, B, m->part, m->xn, w0.wqkv, m->qkv_dim, H, UGB_EPI_F32, m->splits_qkv, m->bn_qkv, nullptr, &c_qkv, &o_qkv) ||
-        gemm_rows(m, B, po, m->att, w0.wo, H, AW, UGB_EPI_F32, m->splits_o, m->bn_o, nullptr, &c_o, &o_o) ||
+    if (gemm_rows(m, B, m->part, m->xn, w0.wqkv, m->qkv_dim, H, UGB_EPI_F32, s_qkv, m->bn_qkv, nullptr, &c_qkv, &o_qkv) ||
+        gemm_rows(m, B, po, m->att, w0.wo, H, AW, UGB_EPI_F32, s_o, m->bn_o, nullptr, &c_o, &o_o) ||
         gemm_rows(m, B, m->h, m->xn, w0.wgu, 2 * (size_t)c.ffn, H, UGB_EPI_SILU_MUL_BF16, 1, m->bn_gate_up, nullptr, &c_gu, &o_gu) ||
-        gemm_rows(m, B, pd, m->h, w0.wdown, H, c.ffn, UGB_EPI_F32, m->splits_down, m->bn_down, nullptr, &c_down, &o_down))
+        gemm_rows(m, B, pd, m->h, w0.wdown, H, c.ffn, UGB_EPI_F32, s_down, m->bn_down, nullptr, &c_down, &o_down))
       early = false;
   }
-  m->early_ok = early && o_qkv == 1 && o_o == 1 && o_gu == 1 && o_down == 1 && c_qkv <= sms && c_o <= sms && c_gu <= sms &&
+  m->early_ok = few ? early : early && o_qkv == 1 && o_o == 1 && o_gu == 1 && o_down == 1 && c_qkv <= sms && c_o <= sms && c_gu <= sms &&
                 c_down <= sms && c_qkv + c_o > sms && c_gu + c_down > sms && c_down + c_qkv > sms;
   const int early_i = m->early_ok ? 1 : 0;
   for (int l = 0; l < c.layers; ++l) {
     const LayerW &w = m->layers[l];
     if (!(m->skip & 1) && (rc = launch_reduce(m, B, m->x, m->xn, l == 0 ? RED_NONE : RED_DOWN, pd, l == 0 ? 0 : s_down, w.rms1, l > 0 ? early_i : 0))) return rc;
-    if (!(m->skip & 2) && (rc = gemm(m, m->part, m->xn, w.wqkv, m->qkv_dim, H, UGB_EPI_F32, m->splits_qkv, m->bn_qkv))) return rc;
+    if (!(m->skip & 2) && (rc = gemm(m, m->part, m->xn, w.wqkv, m->qkv_dim, H, UGB_EPI_F32, s_qkv, m->bn_qkv))) return rc;
     __nv_bfloat16 *kc = m->kcache + (size_t)l * m->kv_layer_stride;
     __nv_bfloat16 *vc = m->vcache + (size_t)l * m->kv_layer_stride;
     if (!(m->skip & 8) && (rc = launch_attention(m, l, scale, s_qkv, true))) return rc;   // rope + append + attention
-    if (!(m->skip & 16) && (rc = gemm(m, po, m->att, w.wo, H, AW, UGB_EPI_F32, m->splits_o, m->bn_o))) return rc;
+    if (!(m->skip & 16) && (rc = gemm(m, po, m->att, w.wo, H, AW, UGB_EPI_F32, s_o, m->bn_o))) return rc;
     if (!(m->skip & 1) && (rc = launch_reduce(m, B, m->x, m->xn, RED_O, po, s_o, w.rms2, early_i))) return rc;
     if (!(m->skip & 32) && (rc = gemm(m, m->h, m->xn, w.wgu, 2 * (size_t)c.ffn, H, UGB_EPI_SILU_MUL_BF16, 1, m->bn_gate_up))) return rc;
-    if (!(m->skip & 64) && (rc = gemm(m, pd, m->h, w.wdown, H, c.ffn, UGB_EPI_F32, m->splits_down, m->bn_down))) return rc;
+    if (!(m->skip & 64) && (rc = gemm(m, pd, m->h, w.wdown, H, c.ffn, UGB_EPI_F32, s_down, m->bn_down))) return rc;
   }
   if ((rc = launch_reduce(m, B, m->x, m->xn, RED_DOWN, pd, s_down, m->ln_f, early_i))) return rc;
   return launch_lm_head_argmax(m, true);
@@ -982,6 +999,8 @@ int32_t ugb_llama_time_kernel(ugb_llama *m, int32_t which, int32_t iters, float 
   const ugb_llama_config &c = m->lc;
   const int H = c.hidden, AW = c.n_heads * c.head_dim;
   const float scale = powf((float)c.head_dim, -0.5f);
+  const int s_qkv = step_splits(m, m->qkv_dim, H, m->splits_qkv), s_o = step_splits(m, H, AW, m->splits_o);
+  const int s_down = step_splits(m, H, c.ffn, m->splits_down);
   int32_t rc = UGB_OK;
   // the kernels read the device-side position; during timing it must name the last cached position
   const int last = m->host_pos - 1;
@@ -991,14 +1010,14 @@ int32_t ugb_llama_time_kernel(ugb_llama *m, int32_t which, int32_t iters, float 
     for (int l = 0; l < c.layers && rc == UGB_OK; ++l) {
       const LayerW &w = m->layers[(m->skip & 256) ? 0 : l];   // bit 8: reuse layer 0 (weights stay in L2)
       switch (which) {
-        case UGB_LLAMA_K_QKV: rc = gemm(m, m->part, m->xn, w.wqkv, m->qkv_dim, H, UGB_EPI_F32, m->splits_qkv, m->bn_qkv); break;
+        case UGB_LLAMA_K_QKV: rc = gemm(m, m->part, m->xn, w.wqkv, m->qkv_dim, H, UGB_EPI_F32, s_qkv, m->bn_qkv); break;
         case UGB_LLAMA_K_ATTENTION: {
-          rc = launch_attention(m, l, scale, ugb_tc_gemm_effective_splits(H, m->splits_qkv), false);
+          rc = launch_attention(m, l, scale, s_qkv, false);
           break;
         }
-        case UGB_LLAMA_K_O: rc = gemm(m, m->part, m->att, w.wo, H, AW, UGB_EPI_F32, m->splits_o, m->bn_o); break;
+        case UGB_LLAMA_K_O: rc = gemm(m, m->part, m->att, w.wo, H, AW, UGB_EPI_F32, s_o, m->bn_o); break;
         case UGB_LLAMA_K_GATE_UP: rc = gemm(m, m->h, m->xn, w.wgu, 2 * (size_t)c.ffn, H, UGB_EPI_SILU_MUL_BF16, 1, m->bn_gate_up); break;
-        case UGB_LLAMA_K_DOWN: rc = gemm(m, m->part, m->h, w.wdown, H, c.ffn, UGB_EPI_F32, m->splits_down, m->bn_down); break;
+        case UGB_LLAMA_K_DOWN: rc = gemm(m, m->part, m->h, w.wdown, H, c.ffn, UGB_EPI_F32, s_down, m->bn_down); break;
         case UGB_LLAMA_K_LM_HEAD:
           if (l == 0) rc = gemm(m, m->logits, m->xn, m->embed + (size_t)m->tp_rank * m->vl * H, (size_t)m->vl, H, UGB_EPI_F32, 1, m->bn_lm_head);
           break;

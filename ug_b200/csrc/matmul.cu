@@ -13,6 +13,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "gemm_skinny.cuh"
 #include "gemm_tcgen05.cuh"
 #include "ugb_internal.h"
 
@@ -464,6 +465,17 @@ int32_t ugb_matmul(ugb_device *dev, ugb_slice *dst, const ugb_slice *lhs, const 
   const char *lp = (const char *)lhs->ptr + lhs_off * es;
   const char *rp = (const char *)rhs->ptr + rhs_off * es;
 
+  // Few rows against [n, k] rows: the kernel that streams the matrix through registers, whatever n (it reads every step of a
+  // batch that shares its matrix again, so those go on as one tall product).
+  if ((dt == UGB_BF16 || dt == UGB_F16) && !L.transposed && R.transposed && ugb_skinny_rows(R.batch == 0 ? b * m : m)) {
+    ugb_tc_gemm_args g;
+    g.out = dst->ptr; g.a = lp; g.b = rp;
+    g.batch = b; g.m = m; g.n = n; g.k = k;
+    g.a_batch = L.batch; g.b_batch = R.batch; g.b_is_nk = true; g.f16 = dt == UGB_F16;
+    g.epi = UGB_EPI_BF16; g.splits = 1; g.bn = 0; g.b_static = false; g.pdl = false;
+    const int32_t src = ugb_skinny_gemm(dev, g);
+    if (src != UGB_ERR_UNSUPPORTED) return src;
+  }
   // Tiny products do not fill a 128-row tensor-core tile; the strided kernel handles them.
   if ((dt == UGB_BF16 || dt == UGB_F16) && !L.transposed && m >= 16 && m * n >= 128 * 64) {
     // tensor-core path (bf16 and f16 are the same tcgen05.mma.kind::f16 instruction with another format field, as
