@@ -7,11 +7,13 @@
 //   * the tcgen05 / TMEM tensor-core kernel (bf16 operands, fp32 accumulate),
 //     declared in gemm_tcgen05.cuh, and
 //   * for f32 (the dtype ug-llama casts every weight to, model.rs:118,140,313) two FP32-pipe kernels: a
-//     warp-per-column streaming kernel for the skinny products of a decode step and a 128 x 128 register-blocked
-//     FFMA kernel for the rest, and
+//     warp-per-column streaming kernel for the skinny products of a decode step and a register-blocked FFMA kernel
+//     for the rest, and
 //   * a strided SIMT kernel with fp32 accumulation for bf16 / f16 shapes the tensor-core kernel does not take.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <algorithm>
 
 #include "gemm_skinny.cuh"
 #include "gemm_tcgen05.cuh"
@@ -211,106 +213,246 @@ f32_skinny_n_kernel(float *__restrict__ C, const float *__restrict__ A, const fl
   }
 }
 
-// (2) Everything else in f32: 128 x 128 output tile per CTA, k slices of 8, 256 threads with 8 x 8 outputs each in
-// registers (64 FFMA per 16 shared-memory values read), global loads one slice ahead of the arithmetic, 128-bit
-// global and shared accesses where the layout allows (VEC), zero fill at the m / n / k tails.
-template <bool VEC>
-__global__ void __launch_bounds__(256, 2)
-f32_tile_kernel(float *__restrict__ C, const float *__restrict__ A, const float *__restrict__ B, int m, int n, int k,
-                long long a_rs, long long a_cs, long long a_b, long long b_rs, long long b_cs, long long b_b,
-                long long c_rs, long long c_b) {
-  constexpr int BM = 128, BN = 128, BK = 8;
-  __shared__ __align__(16) float As[2][BK][BM + 4];
-  __shared__ __align__(16) float Bs[2][BK][BN + 4];
-  const int batch = blockIdx.z, t = threadIdx.x;
-  const float *Ab = A + (long long)batch * a_b;
-  const float *Bb = B + (long long)batch * b_b;
-  float *Cb = C + (long long)batch * c_b;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  // one 4-element piece of each tile per thread: along the operand's contiguous direction
-  const bool a_kc = a_cs == 1, b_nc = b_cs == 1;       // A: k contiguous?  B: n contiguous?
-  const int a_i = a_kc ? t >> 1 : (t & 31) * 4, a_p = a_kc ? (t & 1) * 4 : t >> 5;
-  const int b_j = b_nc ? (t & 31) * 4 : t >> 1, b_p = b_nc ? t >> 5 : (t & 1) * 4;
-  float ra[4], rb[4];
-  auto fetch = [&](int k0) {
+// (2) Everything else in f32.  A warp owns 32 x 128 outputs, a thread 8 x 16 of them; of the four warps of a CTA, WM lie side by
+// side over rows and WK take parts of every k slice.  With p.split > 1 the CTAs of a cluster take equal parts of k as well.
+// All partial sums meet in shared memory, in a fixed order.
+//
+// Bound: the FP32 pipe (74 TFLOP/s), with the shared-memory reads close behind: a 16-byte read of a warp takes four passes
+// whatever its lanes have in common, so 8 x 8 outputs per thread (4 reads per 64 FFMA) leave no room above 100 % of both, 8 x 16
+// (6 reads per 128) a quarter.  Two products per instruction (fma.rn.f32x2: the same roundings) halve the issue slots that the
+// products take; the column pairs come out of shared memory as they are needed, the eight row values are doubled by moves.
+// k slices of 16 go through registers into one of two buffers, 16-byte global reads where the layout allows (VEC), zeros behind
+// the edges; the columns of slice k are permuted by 8 (k / 4 mod 4), so that four lanes along k and eight along the rows write
+// without conflicts.
+//
+// [2048, 2048] x [4096, 2048]^T runs at 50 TFLOP/s, FMA pipe 75 % busy while its CTAs run (two CTAs of 256 threads with 8 x 8
+// outputs on 128 x 128 tiles: 41 and 64 %).  Against those: [257, 2048] x [5632, 2048]^T 310 -> 179 us, [1619, 1768] x
+// [984, 1768]^T 243 -> 140, [120, 7144] x [1352, 7144]^T 957 -> 114, [2, 6045] x [338, 6045]^T 951 -> 83.  Slices of 8 were
+// slower (683 -> 770 us on the first), and CTAs whose warps lie over columns no faster than these.
+template <int WM, int WK> struct F32Tile {
+  static constexpr int BM = 32 * WM, BN = 128, BK = 16, THREADS = 32 * WM * WK;
+  static constexpr int STAGE = BK * (BM + BN);                                     // floats
+  static constexpr int SMEM = 2 * STAGE * 4, SMEM_REDUCE = WK * BM * BN * 4;       // bytes; the sums come after the slices
+};
+struct F32Params {
+  float *c;
+  const float *a, *b;
+  int m, n, k;
+  long long a_rs, a_cs, a_b, b_rs, b_cs, b_b, c_rs, c_b;
+  int split, k_per_split;                              // CTAs of a cluster along k
+};
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint64_t twice(float x) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 halves(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
+template <int WM, int WK, bool VEC>
+__global__ void __launch_bounds__(128, 2)
+f32_tile_kernel(const F32Params p) {
+  using T = F32Tile<WM, WK>;
+  constexpr int BM = T::BM, BN = T::BN, BK = T::BK, QK = BK / 4, SW = 32 / QK;
+  static_assert(T::THREADS == 128, "four warps");
+  extern __shared__ __align__(16) float smem[];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int rank = p.split > 1 ? (int)(blockIdx.x % p.split) : 0, n0 = (int)(p.split > 1 ? blockIdx.x / p.split : blockIdx.x) * BN;
+  const int m0 = blockIdx.y * BM;
+  const float *A = p.a + (long long)blockIdx.z * p.a_b, *B = p.b + (long long)blockIdx.z * p.b_b;
+  const int k_lo = rank * p.k_per_split, k_hi = min(p.k, k_lo + p.k_per_split);
+
+  // One operand's slice: R rows of 16 k, in pieces of four values along the contiguous direction
+  auto fetch = [&](auto &reg, const float *src, long long rs, long long ks, int r0, int rows, int R, int k0) {
+    const bool kc = ks == 1;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int gi = m0 + a_i + (a_kc ? 0 : e), gp = k0 + a_p + (a_kc ? e : 0);
-      ra[e] = (gi < m && gp < k) ? __ldg(Ab + gi * a_rs + gp * a_cs) : 0.f;
-      const int gj = n0 + b_j + (b_nc ? e : 0), gq = k0 + b_p + (b_nc ? 0 : e);
-      rb[e] = (gj < n && gq < k) ? __ldg(Bb + gq * b_rs + gj * b_cs) : 0.f;
+    for (int i = 0; i < (int)(sizeof(reg) / sizeof(float4)); ++i) {
+      const int q = t + i * 128;
+      const int r = r0 + (kc ? q / QK : q % (R / 4) * 4), k = k0 + (kc ? q % QK * 4 : q / (R / 4));
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      const float *at = src + r * rs + k * ks;
+      if (VEC) {                                       // a piece is all in or all out
+        if (r < rows && k < k_hi) {
+          const float4 w = __ldg(reinterpret_cast<const float4 *>(at));
+          v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (kc ? r < rows && k + e < k_hi : r + e < rows && k < k_hi) v[e] = __ldg(at + e * (kc ? ks : rs));
+      }
+      reg[i] = make_float4(v[0], v[1], v[2], v[3]);
     }
   };
-  auto fetch_vec = [&](int k0) {       // whole pieces inside the matrix, 16-byte aligned (checked by the host)
-    const int gi = m0 + a_i, gp = k0 + a_p;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (gi < m && gp < k) v = __ldg(reinterpret_cast<const float4 *>(Ab + gi * a_rs + gp * a_cs));
-    ra[0] = v.x; ra[1] = v.y; ra[2] = v.z; ra[3] = v.w;
-    const int gj = n0 + b_j, gq = k0 + b_p;
-    v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (gj < n && gq < k) v = __ldg(reinterpret_cast<const float4 *>(Bb + gq * b_rs + gj * b_cs));
-    rb[0] = v.x; rb[1] = v.y; rb[2] = v.z; rb[3] = v.w;
-  };
-  auto stage = [&](int buf) {
+  auto stage = [&](const auto &reg, float *dst, long long ks, int R) {
+    const bool kc = ks == 1;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      As[buf][a_p + (a_kc ? e : 0)][a_i + (a_kc ? 0 : e)] = ra[e];
-      Bs[buf][b_p + (b_nc ? 0 : e)][b_j + (b_nc ? e : 0)] = rb[e];
+    for (int i = 0; i < (int)(sizeof(reg) / sizeof(float4)); ++i) {
+      const int q = t + i * 128;
+      if (kc) {
+        const int r = q / QK ^ q % QK * SW, k = q % QK * 4;
+        dst[k * R + r] = reg[i].x; dst[(k + 1) * R + r] = reg[i].y; dst[(k + 2) * R + r] = reg[i].z; dst[(k + 3) * R + r] = reg[i].w;
+      } else {
+        const int k = q / (R / 4), r = q % (R / 4) * 4 ^ (k >> 2) * SW;
+        *reinterpret_cast<float4 *>(dst + k * R + r) = reg[i];
+      }
     }
   };
-  const int tx = t & 15, ty = t >> 4;
-  float acc[8][8];
+  float4 ra[BM * BK / 512], rb[BN * BK / 512];
+  auto fetch_both = [&](int k0) {
+    fetch(ra, A, p.a_rs, p.a_cs, m0, p.m, BM, k0);
+    fetch(rb, B, p.b_cs, p.b_rs, n0, p.n, BN, k0);
+  };
+  auto stage_both = [&](int buf) {
+    stage(ra, smem + buf * T::STAGE, p.a_cs, BM);
+    stage(rb, smem + buf * T::STAGE + BK * BM, p.b_rs, BN);
+  };
+
+  const int wk = warp % WK, wm = warp / WK;
+  const int ty = lane >> 3, tx = lane & 7;
+  uint64_t acc[8][8];                                  // columns in pairs
 #pragma unroll
   for (int u = 0; u < 8; ++u)
 #pragma unroll
-    for (int v = 0; v < 8; ++v) acc[u][v] = 0.f;
-  if (VEC) fetch_vec(0); else fetch(0);
-  stage(0);
+    for (int v = 0; v < 8; ++v) acc[u][v] = 0ull;
+  if (k_lo < k_hi) {
+    fetch_both(k_lo);
+    stage_both(0);
+  }
   __syncthreads();
   int buf = 0;
-  for (int k0 = 0; k0 < k; k0 += BK) {
-    const bool more = k0 + BK < k;
-    if (more) { if (VEC) fetch_vec(k0 + BK); else fetch(k0 + BK); }
+  for (int k0 = k_lo; k0 < k_hi; k0 += BK) {
+    const bool more = k0 + BK < k_hi;
+    if (more) fetch_both(k0 + BK);
+    const float *as = smem + buf * T::STAGE, *bs = as + BK * BM;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h)                        // rolled, or the compiler moves the global reads down to their use
 #pragma unroll
-    for (int p = 0; p < BK; ++p) {
-      // rows ty*4 .. +3 and 64 + ty*4 .. +3, columns tx*4 .. +3 and 64 + tx*4 .. +3: conflict-free 128-bit reads
-      const float4 a0 = *reinterpret_cast<const float4 *>(&As[buf][p][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4 *>(&As[buf][p][64 + ty * 4]);
-      const float4 b0 = *reinterpret_cast<const float4 *>(&Bs[buf][p][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4 *>(&Bs[buf][p][64 + tx * 4]);
+    for (int j = 0; j < BK / WK / 2; ++j) {
+      const int kk = wk * (BK / WK) + h * (BK / WK / 2) + j, x = (kk >> 2) * SW;
+      const float *ar = as + kk * BM + wm * 32, *br = bs + kk * BN + (tx * 4 ^ x);
+      const float4 a0 = *reinterpret_cast<const float4 *>(ar + (ty * 4 ^ x)), a1 = *reinterpret_cast<const float4 *>(ar + (16 + ty * 4 ^ x));
       const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+      uint64_t b[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
+      for (int g = 0; g < 4; ++g) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(br + g * 32);
+        b[2 * g] = w.x; b[2 * g + 1] = w.y;
+      }
 #pragma unroll
-        for (int v = 0; v < 8; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
+      for (int u = 0; u < 8; ++u) {
+        const uint64_t aa = twice(a[u]);
+#pragma unroll
+        for (int v = 0; v < 8; ++v) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[u][v]) : "l"(aa), "l"(b[v]));
+      }
     }
     if (more) {
-      stage(buf ^ 1);
+      stage_both(buf ^ 1);
       __syncthreads();
       buf ^= 1;
     }
   }
+
+  float *C = p.c + (long long)blockIdx.z * p.c_b;
+  auto store = [&](int row, int col, float4 v) {       // row, col inside the tile
+    const int gi = m0 + row, gj = n0 + col;
+    if (gi >= p.m) return;
+    float *at = C + gi * p.c_rs + gj;
+    if (VEC && gj + 3 < p.n) {
+      *reinterpret_cast<float4 *>(at) = v;
+    } else {
+      const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (gj + e < p.n) at[e] = w[e];
+    }
+  };
+  const bool alone = WK == 1 && p.split == 1;
+  if (!alone) __syncthreads();                         // the sums take the place of the slices
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
-    const int gi = m0 + (u < 4 ? ty * 4 + u : 64 + ty * 4 + (u - 4));
-    if (gi >= m) continue;
+    const int row = wm * 32 + ty * 4 + (u & 3) + (u >> 2) * 16;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int gj = n0 + h * 64 + tx * 4;
-      float *crow = Cb + (long long)gi * c_rs + gj;
-      if (VEC && gj + 3 < n) {
-        *reinterpret_cast<float4 *>(crow) = make_float4(acc[u][4 * h], acc[u][4 * h + 1], acc[u][4 * h + 2], acc[u][4 * h + 3]);
-      } else {
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          if (gj + v < n) crow[v] = acc[u][4 * h + v];
-      }
+    for (int g = 0; g < 4; ++g) {
+      const int col = g * 32 + tx * 4;
+      const float2 lo = halves(acc[u][2 * g]), hi = halves(acc[u][2 * g + 1]);
+      const float4 v = make_float4(lo.x, lo.y, hi.x, hi.y);
+      if (alone) store(row, col, v);
+      else *reinterpret_cast<float4 *>(smem + (wk * BM + row) * BN + col) = v;
     }
   }
+  if (alone) return;
+  if (p.split > 1) cluster_barrier(); else __syncthreads();
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+  for (int i = rank * 128 + t; i < BM * BN / 4; i += p.split * 128) {
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < p.split; ++s) {
+      uint32_t from = base;
+      if (p.split > 1) asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(from) : "r"(base), "r"(s));
+#pragma unroll
+      for (int w = 0; w < WK; ++w) {
+        float4 v;
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(from + (uint32_t)(w * BM * BN + 4 * i) * 4u) : "memory");
+        sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+      }
+    }
+    store(4 * i / BN, 4 * i % BN, sum);
+  }
+  if (p.split > 1) cluster_barrier();                  // the others have read this CTA's sums
 }
 
 inline bool al16(const void *p) { return ((uintptr_t)p & 15) == 0; }
+
+// Warps over rows and over a slice's k, and CTAs along k, for a product on f32_tile_kernel: the least time of the fullest SM.
+// In SM cycles, fitted to 49 timed combinations of eight products of 40-2048 rows (off by 4 % on average): the share of the FMA
+// pipe that one CTA on an SM or several reach, what the k split inside a CTA costs of it, and what a CTA spends besides.
+struct F32Shape { int wm, wk, split; };
+F32Shape f32_shape(int sm_count, size_t b, size_t m, size_t n, size_t k) {
+  constexpr double ONE = 0.62, SEVERAL = 0.75, SHARE[] = {1.0, 0.85, 0.72}, CTA = 1300, REDUCE = 2600, RANK = 400;
+  F32Shape best{4, 1, 1};
+  double least = 0;
+  for (int i = 0; i < 3; ++i) {
+    const int wm = 4 >> i, wk = 1 << i;
+    const size_t rows = (m + 32 * wm - 1) / (32 * wm), tiles = rows * ((n + 127) / 128) * b;
+    if (rows > 65535) continue;
+    for (int split = 1; split == 1 || (split <= 8 && k / split >= 64); split *= 2) {
+      const double ctas = (double)((tiles * split + sm_count - 1) / sm_count);
+      const double mma = 32.0 * wm * ((k + split - 1) / split) / (SHARE[i] * (ctas < 2 ? ONE : SEVERAL));
+      const double cost = ctas * (mma + CTA + (wk * split > 1 ? REDUCE : 0) + (split > 1 ? RANK * split : 0));
+      if (least == 0 || cost < least) { least = cost; best = {wm, wk, split}; }
+    }
+  }
+  return best;
+}
+
+template <int WM, int WK, bool VEC>
+int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b) {
+  using T = F32Tile<WM, WK>;
+  const dim3 grid((unsigned)((p.n + T::BN - 1) / T::BN * p.split), (unsigned)((p.m + T::BM - 1) / T::BM), (unsigned)b);
+  const size_t smem = WK * p.split > 1 ? std::max(T::SMEM, T::SMEM_REDUCE) : T::SMEM;
+  if (smem > 48 * 1024) UGB_CUDA(dev, cudaFuncSetAttribute(f32_tile_kernel<WM, WK, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const cudaError_t e = ugb_launch_cluster(f32_tile_kernel<WM, WK, VEC>, grid, dim3(T::THREADS), smem, dev->stream, false, p.split, p);
+  if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of f32_tile_kernel failed: %s", cudaGetErrorString(e));
+  return ugb_after_launch(dev, "f32_tile_kernel");
+}
+
+int32_t launch_f32_tile(ugb_device *dev, F32Params p, size_t b, bool vec) {
+  const F32Shape s = f32_shape(dev->sm_count, b, p.m, p.n, p.k);
+  UGB_REQUIRE(dev, b <= 65535 && ((size_t)p.m + 127) / 128 <= 65535, UGB_ERR_UNSUPPORTED, "matmul: m too large for the f32 kernel");
+  p.split = s.split;
+  p.k_per_split = (int)((((size_t)p.k + s.split - 1) / s.split + 15) / 16 * 16);
+  if (s.wk == 4) return vec ? launch_f32_shape<1, 4, true>(dev, p, b) : launch_f32_shape<1, 4, false>(dev, p, b);
+  if (s.wk == 2) return vec ? launch_f32_shape<2, 2, true>(dev, p, b) : launch_f32_shape<2, 2, false>(dev, p, b);
+  return vec ? launch_f32_shape<4, 1, true>(dev, p, b) : launch_f32_shape<4, 1, false>(dev, p, b);
+}
 
 int32_t launch_f32(ugb_device *dev, float *dst, const float *lhs, const float *rhs, size_t b, size_t m, size_t n, size_t k,
                    const MatLayout &L, const MatLayout &R) {
@@ -336,15 +478,11 @@ int32_t launch_f32(ugb_device *dev, float *dst, const float *lhs, const float *r
 #undef UGB_SKINNY_N
     return ugb_after_launch(dev, "f32_skinny_n_kernel");
   }
-  const dim3 grid((unsigned)((n + 127) / 128), (unsigned)((m + 127) / 128), (unsigned)b);
-  UGB_REQUIRE(dev, grid.y <= 65535, UGB_ERR_UNSUPPORTED, "matmul: m too large for the f32 kernel");
   // 128-bit pieces: the contiguous extent and the leading stride of each operand in whole float4s
   const size_t a_c = L.transposed ? m : k, a_ld = (size_t)(L.transposed ? L.cs : L.rs);
   const size_t b_c = R.transposed ? k : n, b_ld = (size_t)(R.transposed ? R.cs : R.rs);
   const bool vec = bases && a_c % 4 == 0 && a_ld % 4 == 0 && b_c % 4 == 0 && b_ld % 4 == 0 && n % 4 == 0;
-  if (vec) f32_tile_kernel<true><<<grid, 256, 0, dev->stream>>>(dst, lhs, rhs, (int)m, (int)n, (int)k, L.rs, L.cs, L.batch, R.rs, R.cs, R.batch, (long long)n, (long long)(m * n));
-  else f32_tile_kernel<false><<<grid, 256, 0, dev->stream>>>(dst, lhs, rhs, (int)m, (int)n, (int)k, L.rs, L.cs, L.batch, R.rs, R.cs, R.batch, (long long)n, (long long)(m * n));
-  return ugb_after_launch(dev, "f32_tile_kernel");
+  return launch_f32_tile(dev, {dst, lhs, rhs, (int)m, (int)n, (int)k, L.rs, L.cs, L.batch, R.rs, R.cs, R.batch, (long long)n, (long long)(m * n), 1, 0}, b, vec);
 }
 
 template <typename T>
@@ -413,15 +551,12 @@ int32_t ugb_f32_gemm(ugb_device *dev, float *c, const float *a, const float *b, 
     const MatLayout L{(long long)k, 1, (long long)a_batch, false}, R{1, (long long)k, (long long)b_batch, true};
     return launch_f32(dev, c, a, b, batch, m, n, k, L, R);
   }
-  const dim3 grid((unsigned)((n + 127) / 128), (unsigned)((m + 127) / 128), (unsigned)batch);
-  UGB_REQUIRE(dev, batch <= 65535 && grid.y <= 65535 && m < (1u << 31) && n < (1u << 31) && k < (1u << 31), UGB_ERR_UNSUPPORTED,
+  UGB_REQUIRE(dev, batch <= 65535 && (m + 127) / 128 <= 65535 && m < (1u << 31) && n < (1u << 31) && k < (1u << 31), UGB_ERR_UNSUPPORTED,
               "f32 product: extent too large");
   const bool vec = al16(c) && al16(a) && al16(b) && k % 4 == 0 && n % 4 == 0 && a_ld % 4 == 0 && c_ld % 4 == 0 &&
                    a_batch % 4 == 0 && b_batch % 4 == 0 && c_batch % 4 == 0;
   const long long b_rs = b_is_nk ? 1 : (long long)n, b_cs = b_is_nk ? (long long)k : 1;
-  if (vec) f32_tile_kernel<true><<<grid, 256, 0, dev->stream>>>(c, a, b, (int)m, (int)n, (int)k, (long long)a_ld, 1, (long long)a_batch, b_rs, b_cs, (long long)b_batch, (long long)c_ld, (long long)c_batch);
-  else f32_tile_kernel<false><<<grid, 256, 0, dev->stream>>>(c, a, b, (int)m, (int)n, (int)k, (long long)a_ld, 1, (long long)a_batch, b_rs, b_cs, (long long)b_batch, (long long)c_ld, (long long)c_batch);
-  return ugb_after_launch(dev, "f32_tile_kernel");
+  return launch_f32_tile(dev, {c, a, b, (int)m, (int)n, (int)k, (long long)a_ld, 1, (long long)a_batch, b_rs, b_cs, (long long)b_batch, (long long)c_ld, (long long)c_batch, 1, 0}, batch, vec);
 }
 
 extern "C" {
