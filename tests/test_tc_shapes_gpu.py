@@ -1,0 +1,30 @@
+"""16-bit products of more than 64 rows at sizes for which each tile shape of the tensor-core kernel is chosen (128- and 256-row
+tiles, 64 to 256 columns), ragged in every direction, and Llama prompts whose o and down products split k."""
+import numpy as np
+import pytest
+
+from ug_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k,kn", [
+    (65, 72, 64, False), (100, 2040, 200, False), (129, 2056, 520, True), (300, 2048, 2048, False),       # 64 columns
+    (100, 11256, 2040, False), (777, 2056, 2040, False), (500, 2560, 1000, True),                         # 128
+    (777, 11256, 520, False), (200, 11264, 2056, True), (1023, 2552, 2048, False),                        # 192
+    (300, 11264, 2040, False),                                                                            # 256, 128 rows
+    (1023, 2040, 5640, False), (511, 11256, 2040, False), (1500, 2040, 5632, False), (2040, 2056, 264, False), (2047, 2048, 2048, True)])  # pairs
+def test_shapes(dev, m, n, k, kn):
+    ab, wb = synth.to_bf16_bits(synth.normal(m, (m, k), 0.5)), synth.to_bf16_bits(synth.normal(n, (k, n) if kn else (n, k), 0.5))
+    guard = 64
+    out = dev.slice_from_values(synth.to_bf16_bits(np.full(m * n + guard, 3.0, np.float32)), bf16=True)
+    dev.matmul(out, dev.slice_from_values(ab.ravel(), bf16=True), dev.slice_from_values(wb.ravel(), bf16=True), (1, m, n, k),
+               ([1, m, k], [m * k, k, 1], 0), ([1, k, n], [n * k, n, 1] if kn else [n * k, 1, k], 0))
+    got = synth.bf16_bits_to_f32(out.to_vec())
+    assert np.all(got[m * n:] == 3.0)
+    rows = np.unique(np.r_[np.arange(0, m, 37), m - 1, min(m - 1, 127), min(m - 1, 128), min(m - 1, 255), min(m - 1, 256)])
+    a = synth.bf16_bits_to_f32(ab)[rows].astype(np.float64)
+    w = synth.bf16_bits_to_f32(wb).astype(np.float64)
+    w = w if kn else w.T
+    # one rounding of the result (half a unit, 2^-9) plus f32 sums of k products
+    assert np.all(np.abs(got[:m * n].reshape(m, n)[rows] - a @ w) <= np.abs(a @ w) * 2.0 ** -8 + np.abs(a) @ np.abs(w) * k * 2.0 ** -24 + 1e-6)

@@ -43,7 +43,7 @@ struct ugb_tc_gemm_args {
   bool b_is_nk;
   int epi;              // UGB_EPI_*
   int splits;           // split-K factor (only with UGB_EPI_F32); the kernel may use fewer
-  int bn;               // tile width: 64, 128, 256 (80, 96, 160 too when m <= 64 and b_is_nk), or 0 = choose from m
+  int bn;               // tile width: 64, 128, 192 (m > 64), 256 (80, 96, 160 too when m <= 64 and b_is_nk), or 0 = choose the shape
   bool b_static;        // no kernel on the stream writes b (weights): fetch it before waiting for the predecessor
   bool pdl;             // launch with programmatic stream serialization (see ugb_launch)
   bool late_trigger = false;   // let the next kernel start only once the wait for the preceding one has returned: a kernel
@@ -71,6 +71,10 @@ struct ugb_tc_gemm_args {
 // does not meet the kernel's alignment rules so that the caller can fall back
 // to the strided kernel.
 int32_t ugb_tc_gemm(ugb_device *dev, const ugb_tc_gemm_args &args);
+// Tile shape for more than 64 rows: width, 256-row tiles on pairs of CTAs, and a k split where the caller takes f32 partials
+// (max_splits > 1; the pair shapes do not split).  `pairs`: pairs may be chosen at all.
+struct ugb_tc_plan { int bn = 0, splits = 1; bool pair = false; };
+ugb_tc_plan ugb_tc_gemm_plan(int sm_count, size_t batch, size_t m, size_t n, size_t k, bool b_is_nk, bool pairs, int max_splits);
 // Number of partials ugb_tc_gemm writes for a requested split factor.
 int ugb_tc_gemm_effective_splits(size_t k, int splits);
 // C[b, m, n] = A . B with the default epilogue, all three bf16 (f16 = false) or IEEE f16.

@@ -497,11 +497,20 @@ int32_t llama_prefill_chunk(ugb_llama *m, const int *tok, int t, int c0, int tc,
   if ((rc = ugb_after_launch(dev, "embed_gather_kernel"))) return rc;
   const int rope_items = ((c.n_heads + c.n_kv_heads) * c.head_dim / 2 + c.n_kv_heads * c.head_dim) / 4;   // 4 pairs / values per thread
   float *po = o_out(m, m->pf_f32), *pd = down_out(m, m->pf_f32);
+  // The reduce kernel adds partials, so the two products before it may split k where their tiles leave SMs idle, as far as the
+  // buffer (and the exchange block, which holds no fewer rows) takes the partials.  Several ranks read one partial of each other.
+  const size_t pf_cap = m->tp_size > 1 ? 1 : (size_t)m->pf_rows / (size_t)rows;
+  auto split_plan = [&](size_t k) {
+    const int most = (int)std::min<size_t>(4, pf_cap);
+    return rows > 64 && most > 1 ? ugb_tc_gemm_plan(dev->sm_count, 1, rows, H, k, true, dev->gemm_pair != 0, most) : ugb_tc_plan{};
+  };
+  const ugb_tc_plan plan_o = split_plan(AW), plan_down = split_plan(c.ffn);
+  auto bn_of = [](const ugb_tc_plan &x) { return x.splits > 1 ? x.bn : 0; };
   for (int l = 0; l < c.layers; ++l) {
     const LayerW &w = m->layers[l];
     __nv_bfloat16 *kc = m->kcache + (size_t)l * m->kv_layer_stride;
     __nv_bfloat16 *vc = m->vcache + (size_t)l * m->kv_layer_stride;
-    if ((rc = launch_reduce(m, rows, m->pf_x, m->pf_xn, l == 0 ? RED_NONE : RED_DOWN, pd, l == 0 ? 0 : 1, w.rms1))) return rc;
+    if ((rc = launch_reduce(m, rows, m->pf_x, m->pf_xn, l == 0 ? RED_NONE : RED_DOWN, pd, l == 0 ? 0 : plan_down.splits, w.rms1))) return rc;
     if (rows > 64) {
       // qkv projection with the rotation and the cache append in its epilogue: no fp32 round trip, no rope kernel
       ugb_tc_rope_epilogue re;
@@ -527,14 +536,14 @@ int32_t llama_prefill_chunk(ugb_llama *m, const int *tok, int t, int c0, int tc,
           m->pf_q, kc, vc, m->pf_att, tc, m->host_pos + c0, c.n_heads, c.n_kv_heads, m->t_max, scale);
       if ((rc = ugb_after_launch(dev, "prefill_attention_kernel"))) return rc;
     }
-    if ((rc = gemm_rows(m, rows, po, m->pf_att, w.wo, H, AW, UGB_EPI_F32, 1, 0))) return rc;
-    if ((rc = launch_reduce(m, rows, m->pf_x, m->pf_xn, RED_O, po, 1, w.rms2))) return rc;
+    if ((rc = gemm_rows(m, rows, po, m->pf_att, w.wo, H, AW, UGB_EPI_F32, plan_o.splits, bn_of(plan_o)))) return rc;
+    if ((rc = launch_reduce(m, rows, m->pf_x, m->pf_xn, RED_O, po, plan_o.splits, w.rms2))) return rc;
     if ((rc = gemm_rows(m, rows, m->pf_h, m->pf_xn, w.wgu, 2 * (size_t)c.ffn, H, UGB_EPI_SILU_MUL_BF16, 1, 0))) return rc;
-    if ((rc = gemm_rows(m, rows, pd, m->pf_h, w.wdown, H, c.ffn, UGB_EPI_F32, 1, 0))) return rc;
+    if ((rc = gemm_rows(m, rows, pd, m->pf_h, w.wdown, H, c.ffn, UGB_EPI_F32, plan_down.splits, bn_of(plan_down)))) return rc;
   }
   // The last down_proj output is folded into the residual stream here (every rank's partial under tensor
   // parallelism), so that what follows -- all-position logits, the last-position step -- sees the final x.
-  if ((rc = launch_reduce(m, rows, m->pf_x, m->pf_xn, RED_DOWN, pd, 1, m->ln_f))) return rc;
+  if ((rc = launch_reduce(m, rows, m->pf_x, m->pf_xn, RED_DOWN, pd, plan_down.splits, m->ln_f))) return rc;
   if (all_logits) {
     // logits[b, c0 + i, rank's vocabulary slice] for the chunk as one GEMM batched over sequences
     ugb_tc_gemm_args g;
