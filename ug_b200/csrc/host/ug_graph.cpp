@@ -497,6 +497,11 @@ Opts b200_opts(const op::Kernel &k) {
 CompiledSchedule Schedule::compile_with_cache(CompilationCache &cache) const {
   CompiledSchedule out;
   out.device = device;
+  out.funcs.reserve(items.size());
+  // Kernels of this schedule that a shape-generic function serves.  Every layer of a model has the same ones, and finding the
+  // function takes a lowering and a pass over its text (about 35 us); they are new in the next schedule, so nothing is kept.
+  struct Served { std::shared_ptr<Func> func; uint32_t grid; int64_t t; };
+  std::map<NormalizedKernel, Served> served_here;
   for (const ScheduleItem &item : items) {
     CompiledFunc cf;
     switch (item.kind) {
@@ -538,6 +543,12 @@ CompiledSchedule Schedule::compile_with_cache(CompilationCache &cache) const {
         }
         auto it = cache.op_cache.find(norm);
         if (it != cache.op_cache.end()) { cf.func = it->second; cache.hits++; break; }
+        auto again = served_here.find(norm);
+        if (again != served_here.end()) {
+          cf.func = again->second.func; cf.dyn = true; cf.dyn_grid = again->second.grid; cf.dyn_t = again->second.t;
+          cache.hits++; cache.poly_hits++;
+          break;
+        }
         const std::string name = kernel.ops.empty() ? std::string() : kernel.ops[0].name();
         kernel = optimize(std::move(kernel));
         if (device->launch_policy() == LaunchPolicy::B200 && cache.polymorphic) {
@@ -563,7 +574,10 @@ CompiledSchedule Schedule::compile_with_cache(CompilationCache &cache) const {
                 served = true;
                 break;
               }
-            if (served) break;
+            if (served) {
+              served_here.emplace(std::move(norm), Served{cf.func, cf.dyn_grid, cf.dyn_t});
+              break;
+            }
             if (!pe.failed && pe.have_pending && pe.generics.size() < 8) {
               std::string generic;
               PolyGeneric g;
@@ -585,6 +599,7 @@ CompiledSchedule Schedule::compile_with_cache(CompilationCache &cache) const {
                 pe.pending.clear();
                 pe.have_pending = false;
                 cache.misses++;
+                served_here.emplace(std::move(norm), Served{cf.func, cf.dyn_grid, cf.dyn_t});
                 break;
               }
               pe.failed = true;

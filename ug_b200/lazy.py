@@ -54,9 +54,18 @@ def _chk(rc):
         raise UgError(rc, _err())
 
 
+_SIZES = [C.c_size_t * max(n, 1) for n in range(9)]       # ctypes looks an array type up at every product
+
+
 def _dims(shape):
-    shape = tuple(int(d) for d in (shape if hasattr(shape, "__len__") else (shape,)))
-    return (C.c_size_t * max(len(shape), 1))(*shape), len(shape)
+    if not hasattr(shape, "__len__"):
+        shape = (shape,)
+    n = len(shape)
+    t = _SIZES[n] if n < len(_SIZES) else C.c_size_t * n
+    try:
+        return t(*shape), n
+    except TypeError:                                      # numpy integers and the like
+        return t(*[int(d) for d in shape]), n
 
 
 class UnaryOp(enum.IntEnum):
@@ -188,15 +197,18 @@ class LazyBuffer:
     """ug::LazyBuffer (ug-core/src/lazy_buffer.rs)."""
 
     def __init__(self, handle, device):
-        self._h, self.device = handle, device
+        self._h, self.device, self._shape = handle, device, None
 
-    def __del__(self):
-        h, self._h = getattr(self, "_h", None), None
+    def __del__(self, _free=host.ugh_lb_free):
+        try:
+            h, self._h = self._h, None
+        except AttributeError:
+            return
         if h:
-            host.ugh_lb_free(h)
+            _free(h)
 
     def _new(self, h):
-        return LazyBuffer(_ptr(h), self.device)
+        return LazyBuffer(h or _ptr(h), self.device)
 
     # ---- constructors
     @staticmethod
@@ -307,10 +319,12 @@ class LazyBuffer:
 
     # ---- queries
     def dims(self):
-        r = host.ugh_lb_rank(self._h)
-        out = (C.c_size_t * max(r, 1))()
-        host.ugh_lb_dims(self._h, out)
-        return tuple(out[i] for i in range(r))
+        if self._shape is None:                            # a node's shape never changes
+            r = host.ugh_lb_rank(self._h)
+            out = (C.c_size_t * max(r, 1))()
+            host.ugh_lb_dims(self._h, out)
+            self._shape = tuple(out[:r])
+        return self._shape
 
     shape = dims
 
