@@ -36,7 +36,7 @@ struct Params {
   void *out;
   long long w_batch, a_ld, a_batch, c_ld, c_batch, c_split;      // elements
   int rows, n, k, tiles, splits, chunks, chunks_per_split, spans, units;
-  int epi, late_trigger;
+  int epi, late_trigger, wait_first;       // wait_first: a kernel of the stream may write W
   const int *groups;                       // expert of group tile i, -1 behind the last; or null
   int n_groups_tiles, tile_m;
 };
@@ -79,6 +79,7 @@ skinny_gemm_kernel(const Params p) {
     units = live * p.tiles;
   }
   if (!p.late_trigger) ugb_pdl_trigger();
+  if (p.wait_first) ugb_pdl_wait();
   const int u1 = (int)((long long)(blockIdx.x + 1) * units / gridDim.x);
   int u = (int)((long long)blockIdx.x * units / gridDim.x), s = 0;
 
@@ -234,6 +235,7 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
   p.spans = (p.chunks_per_split + kc * WARPS - 1) / (kc * WARPS);
   p.epi = g.epi;
   p.late_trigger = g.late_trigger ? 1 : 0;
+  p.wait_first = !g.b_static && !g.groups ? 1 : 0;
   p.groups = g.groups; p.tile_m = g.tile_m;
   p.n_groups_tiles = g.groups ? (int)(g.m / g.tile_m) : 0;
   const long long units = (long long)p.tiles * (g.groups ? p.n_groups_tiles : (long long)p.splits * (long long)g.batch);

@@ -886,7 +886,7 @@ int32_t ugb_tc_gemm_bf16(ugb_device *dev, void *c, const void *a, const void *b_
   g.out = c; g.a = a; g.b = b_;
   g.batch = batch; g.m = m; g.n = n; g.k = k;
   g.a_batch = a_batch; g.b_batch = b_batch; g.b_is_nk = b_is_nk;
-  g.epi = UGB_EPI_BF16; g.splits = 1; g.bn = 0; g.b_static = false; g.pdl = false;
+  g.epi = UGB_EPI_BF16; g.splits = 1; g.bn = 0; g.b_static = false; g.pdl = true;
   return ugb_tc_gemm(dev, g);
 }
 

@@ -137,6 +137,8 @@ template <int MR>
 __global__ void __launch_bounds__(256)
 f32_skinny_kernel(float *__restrict__ C, const float *__restrict__ A, const float *__restrict__ B, int m, int n, int k,
                   long long a_b, long long b_b) {
+  ugb_pdl_trigger();
+  ugb_pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 8 + warp;
   if (col >= n) return;
@@ -177,6 +179,8 @@ f32_skinny_n_kernel(float *__restrict__ C, const float *__restrict__ A, const fl
                     long long a_rs, long long a_b, long long b_rs, long long b_b) {
   constexpr int WARPS = MR <= 2 ? 32 : (MR <= 4 ? 16 : 8);       // 32 KiB of partial sums at most
   __shared__ __align__(16) float red[WARPS][MR][128];
+  ugb_pdl_trigger();
+  ugb_pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int batch = blockIdx.y, col = blockIdx.x * 128 + lane * 4;
   const float *a = A + (long long)batch * a_b;
@@ -263,6 +267,8 @@ f32_tile_kernel(const F32Params p) {
   constexpr int BM = T::BM, BN = T::BN, BK = T::BK, QK = BK / 4, SW = 32 / QK;
   static_assert(T::THREADS == 128, "four warps");
   extern __shared__ __align__(16) float smem[];
+  ugb_pdl_trigger();
+  ugb_pdl_wait();
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int rank = p.split > 1 ? (int)(blockIdx.x % p.split) : 0, n0 = (int)(p.split > 1 ? blockIdx.x / p.split : blockIdx.x) * BN;
   const int m0 = blockIdx.y * BM;
@@ -439,7 +445,7 @@ int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b) {
   const dim3 grid((unsigned)((p.n + T::BN - 1) / T::BN * p.split), (unsigned)((p.m + T::BM - 1) / T::BM), (unsigned)b);
   const size_t smem = WK * p.split > 1 ? std::max(T::SMEM, T::SMEM_REDUCE) : T::SMEM;
   if (smem > 48 * 1024) UGB_CUDA(dev, cudaFuncSetAttribute(f32_tile_kernel<WM, WK, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const cudaError_t e = ugb_launch_cluster(f32_tile_kernel<WM, WK, VEC>, grid, dim3(T::THREADS), smem, dev->stream, false, p.split, p);
+  const cudaError_t e = ugb_launch_cluster(f32_tile_kernel<WM, WK, VEC>, grid, dim3(T::THREADS), smem, dev->stream, true, p.split, p);
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of f32_tile_kernel failed: %s", cudaGetErrorString(e));
   return ugb_after_launch(dev, "f32_tile_kernel");
 }
@@ -464,7 +470,7 @@ int32_t launch_f32(ugb_device *dev, float *dst, const float *lhs, const float *r
   const bool bases = al16(dst) && al16(lhs) && al16(rhs) && L.batch % 4 == 0 && R.batch % 4 == 0;
   if (m <= 16 && !L.transposed && R.transposed && k % 4 == 0 && bases) {
     const dim3 grid((unsigned)((n + 7) / 8), (unsigned)b);
-#define UGB_SKINNY(MR) f32_skinny_kernel<MR><<<grid, 256, 0, dev->stream>>>(dst, lhs, rhs, (int)m, (int)n, (int)k, L.batch, R.batch)
+#define UGB_SKINNY(MR) ugb_launch(f32_skinny_kernel<MR>, grid, dim3(256), 0, dev->stream, true, dst, lhs, rhs, (int)m, (int)n, (int)k, L.batch, R.batch)
     if (m <= 1) UGB_SKINNY(1); else if (m <= 2) UGB_SKINNY(2); else if (m <= 4) UGB_SKINNY(4); else if (m <= 8) UGB_SKINNY(8); else UGB_SKINNY(16);
 #undef UGB_SKINNY
     return ugb_after_launch(dev, "f32_skinny_kernel");
@@ -473,7 +479,7 @@ int32_t launch_f32(ugb_device *dev, float *dst, const float *lhs, const float *r
   if (m <= 8 && !L.transposed && !R.transposed && (L.cs == 1 || k == 1) && (R.cs == 1 || n == 1) && n % 4 == 0 &&
       R.rs % 4 == 0 && R.batch % 4 == 0 && al16(rhs)) {
     const dim3 grid((unsigned)((n + 127) / 128), (unsigned)b);
-#define UGB_SKINNY_N(MR) f32_skinny_n_kernel<MR><<<grid, (MR) <= 2 ? 1024 : ((MR) <= 4 ? 512 : 256), 0, dev->stream>>>(dst, lhs, rhs, (int)m, (int)n, (int)k, L.rs, L.batch, R.rs, R.batch)
+#define UGB_SKINNY_N(MR) ugb_launch(f32_skinny_n_kernel<MR>, grid, dim3((MR) <= 2 ? 1024 : ((MR) <= 4 ? 512 : 256)), 0, dev->stream, true, dst, lhs, rhs, (int)m, (int)n, (int)k, L.rs, L.batch, R.rs, R.batch)
     if (m <= 1) UGB_SKINNY_N(1); else if (m <= 2) UGB_SKINNY_N(2); else if (m <= 4) UGB_SKINNY_N(4); else UGB_SKINNY_N(8);
 #undef UGB_SKINNY_N
     return ugb_after_launch(dev, "f32_skinny_n_kernel");
@@ -607,7 +613,7 @@ int32_t ugb_matmul(ugb_device *dev, ugb_slice *dst, const ugb_slice *lhs, const 
     g.out = dst->ptr; g.a = lp; g.b = rp;
     g.batch = b; g.m = m; g.n = n; g.k = k;
     g.a_batch = L.batch; g.b_batch = R.batch; g.b_is_nk = true; g.f16 = dt == UGB_F16;
-    g.epi = UGB_EPI_BF16; g.splits = 1; g.bn = 0; g.b_static = false; g.pdl = false;
+    g.epi = UGB_EPI_BF16; g.splits = 1; g.bn = 0; g.b_static = false; g.pdl = true;
     const int32_t src = ugb_skinny_gemm(dev, g);
     if (src != UGB_ERR_UNSUPPORTED) return src;
   }

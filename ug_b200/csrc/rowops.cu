@@ -12,6 +12,10 @@
 //   CTA-per-row    n_cols <= 8192, multiple of 4     (row in registers)
 //   general        anything else                      (row in shared memory when
 //                  it fits, otherwise re-read from global memory)
+//
+// Every kernel is a dependent launch: its CTAs come to the SMs while the last wave of the kernel before still runs and wait
+// there, so that a chain of small operators does not pay a launch between two of them ([1024, 4096] softmax 8.80 -> 7.23 us,
+// [107, 40] 5.5 -> 3.6, [28239, 104] rms_silu 8.7 -> 6.7).
 #include <cfloat>
 
 #include "ugb_internal.h"
@@ -67,6 +71,8 @@ __device__ __forceinline__ float silu(float g) { return g / (expf(-g) + 1.0f); }
 template <int OP, int VPT, int THREADS, int LANES>
 __global__ void __launch_bounds__(THREADS) row_reg_kernel(RowArgs a) {
   __shared__ float sm[32];
+  ugb_pdl_trigger();
+  ugb_pdl_wait();
   constexpr int ROWS_PER_CTA = THREADS / LANES;
   const int lane = threadIdx.x % LANES;
   const int sub = threadIdx.x / LANES;
@@ -154,6 +160,8 @@ template <int OP, int THREADS>
 __global__ void __launch_bounds__(THREADS) row_general_kernel(RowArgs a, int cache_cols) {
   extern __shared__ float row_cache[];
   __shared__ float sm[32];
+  ugb_pdl_trigger();
+  ugb_pdl_wait();
   const bool cached = cache_cols >= a.n_cols;
   for (size_t row = blockIdx.x; row < a.n_rows; row += gridDim.x) {
     const float *xr = a.x + row * a.n_cols;
@@ -198,7 +206,7 @@ int32_t launch_warp_rows(ugb_device *dev, const RowArgs &a) {
   size_t ctas = (a.n_rows + THREADS / 32 - 1) / (THREADS / 32);
   size_t cap = (size_t)dev->sm_count * 32;
   unsigned grid = (unsigned)(ctas < cap ? ctas : cap);
-  row_reg_kernel<OP, VPT, THREADS, 32><<<grid, THREADS, 0, dev->stream>>>(a);
+  ugb_launch(row_reg_kernel<OP, VPT, THREADS, 32>, dim3(grid), dim3(THREADS), 0, dev->stream, true, a);
   return ugb_after_launch(dev, "row_reg_kernel");
 }
 
@@ -206,7 +214,7 @@ template <int OP, int VPT, int THREADS>
 int32_t launch_cta_rows(ugb_device *dev, const RowArgs &a) {
   size_t cap = (size_t)dev->sm_count * 64;
   unsigned grid = (unsigned)(a.n_rows < cap ? a.n_rows : cap);
-  row_reg_kernel<OP, VPT, THREADS, THREADS><<<grid, THREADS, 0, dev->stream>>>(a);
+  ugb_launch(row_reg_kernel<OP, VPT, THREADS, THREADS>, dim3(grid), dim3(THREADS), 0, dev->stream, true, a);
   return ugb_after_launch(dev, "row_reg_kernel");
 }
 
@@ -249,7 +257,7 @@ int32_t launch_row(ugb_device *dev, const RowArgs &a) {
     UGB_CUDA(dev, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_cache));
   size_t cap = (size_t)dev->sm_count * 4;
   unsigned grid = (unsigned)(a.n_rows < cap ? a.n_rows : cap);
-  k<<<grid, THREADS, smem, dev->stream>>>(a, cache_cols);
+  ugb_launch(k, dim3(grid), dim3(THREADS), smem, dev->stream, true, a, cache_cols);
   return ugb_after_launch(dev, "row_general_kernel");
 }
 
