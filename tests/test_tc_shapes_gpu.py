@@ -28,3 +28,23 @@ def test_shapes(dev, m, n, k, kn):
     w = w if kn else w.T
     # one rounding of the result (half a unit, 2^-9) plus f32 sums of k products
     assert np.all(np.abs(got[:m * n].reshape(m, n)[rows] - a @ w) <= np.abs(a @ w) * 2.0 ** -8 + np.abs(a) @ np.abs(w) * k * 2.0 ** -24 + 1e-6)
+
+
+@pytest.mark.parametrize("f16", [False, True])
+@pytest.mark.parametrize("b,m,n,k,kn", [(1, 14, 520, 2048, False), (3, 9, 136, 264, True), (2, 4, 128, 880, True), (1, 1, 9, 7, True), (1, 15, 4096, 520, True),   # few rows
+                                        (1, 37, 333, 777, True), (2, 100, 255, 129, False), (1, 130, 129, 1001, False), (1, 3, 8, 2, True)])                   # no 16-byte rows
+def test_few_rows_and_odd_sizes(dev, b, m, n, k, kn, f16):
+    def bits(x):
+        return x.astype(np.float16) if f16 else synth.to_bf16_bits(x)
+
+    def wide(x):
+        return x.astype(np.float64) if f16 else synth.bf16_bits_to_f32(x).astype(np.float64)
+    ab, wb = bits(synth.normal(m, (b, m, k), 0.5)), bits(synth.normal(n, (b, k, n) if kn else (b, n, k), 0.5))
+    out = dev.slice_from_values(bits(np.full(b * m * n + 64, 3.0, np.float32)), bf16=not f16)
+    dev.matmul(out, dev.slice_from_values(ab.ravel(), bf16=not f16), dev.slice_from_values(wb.ravel(), bf16=not f16), (b, m, n, k),
+               ([b, m, k], [m * k, k, 1], 0), ([b, k, n], [n * k, n, 1] if kn else [n * k, 1, k], 0))
+    got = wide(out.to_vec())
+    assert np.all(got[b * m * n:] == 3.0)
+    a, w = wide(ab), wide(wb) if kn else wide(wb).transpose(0, 2, 1)
+    # one rounding of the result (half a unit, 2^-12 in f16, 2^-9 in bf16) plus f32 sums of k products
+    assert np.all(np.abs(got[:b * m * n].reshape(b, m, n) - a @ w) <= np.abs(a @ w) * 2.0 ** (-11 if f16 else -8) + np.abs(a) @ np.abs(w) * k * 2.0 ** -24 + 1e-6)

@@ -9,7 +9,7 @@
 //   * for f32 (the dtype ug-llama casts every weight to, model.rs:118,140,313) two FP32-pipe kernels: a
 //     warp-per-column streaming kernel for the skinny products of a decode step and a register-blocked FFMA kernel
 //     for the rest, and
-//   * a strided SIMT kernel with fp32 accumulation for bf16 / f16 shapes the tensor-core kernel does not take.
+//   * the same FFMA kernel on 16-bit operands for the shapes and layouts the tensor-core kernels do not take.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -69,63 +69,6 @@ template <typename T> __device__ __forceinline__ T from_f32(float v);
 template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
-
-// 64x64 output tile, 16-deep k slices, 256 threads, 4x4 outputs per thread.
-template <typename T>
-__global__ void __launch_bounds__(256)
-simt_gemm_kernel(T *__restrict__ C, const T *__restrict__ A, const T *__restrict__ B, int m, int n,
-                 int k, long long a_rs, long long a_cs, long long a_b, long long b_rs,
-                 long long b_cs, long long b_b) {
-  constexpr int BM = 64, BN = 64, BK = 16;
-  __shared__ float As[BK][BM + 1];
-  __shared__ float Bs[BK][BN + 1];
-  const int batch = blockIdx.z;
-  const T *Ab = A + (long long)batch * a_b;
-  const T *Bb = B + (long long)batch * b_b;
-  T *Cb = C + (long long)batch * m * n;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < k; k0 += BK) {
-    for (int e = threadIdx.x; e < BM * BK; e += 256) {
-      // walk the contiguous direction of each operand with consecutive threads
-      int i, p;
-      if (a_cs == 1) { p = e % BK; i = e / BK; } else { i = e % BM; p = e / BM; }
-      const int gi = m0 + i, gp = k0 + p;
-      As[p][i] = (gi < m && gp < k) ? to_f32<T>(Ab[gi * a_rs + gp * a_cs]) : 0.f;
-    }
-    for (int e = threadIdx.x; e < BN * BK; e += 256) {
-      int j, p;
-      if (b_cs == 1) { j = e % BN; p = e / BN; } else { p = e % BK; j = e / BK; }
-      const int gj = n0 + j, gp = k0 + p;
-      Bs[p][j] = (gj < n && gp < k) ? to_f32<T>(Bb[gp * b_rs + gj * b_cs]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < BK; ++p) {
-      float a[4], b[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) a[u] = As[p][ty * 4 + u];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) b[u] = Bs[p][tx * 4 + u];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int gi = m0 + ty * 4 + u;
-    if (gi >= m) continue;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int gj = n0 + tx * 4 + v;
-      if (gj < n) Cb[(long long)gi * n + gj] = from_f32<T>(acc[u][v]);
-    }
-  }
-}
 
 // ---- fp32 on the FP32 pipe (the reference's default for f32 is CUBLAS_COMPUTE_32F, gemm.rs:87-128: no reduced
 // precision), two shapes -------------------------------------------------------------------------------------
@@ -233,14 +176,16 @@ f32_skinny_n_kernel(float *__restrict__ C, const float *__restrict__ A, const fl
 // outputs on 128 x 128 tiles: 41 and 64 %).  Against those: [257, 2048] x [5632, 2048]^T 310 -> 179 us, [1619, 1768] x
 // [984, 1768]^T 243 -> 140, [120, 7144] x [1352, 7144]^T 957 -> 114, [2, 6045] x [338, 6045]^T 951 -> 83.  Slices of 8 were
 // slower (683 -> 770 us on the first), and CTAs whose warps lie over columns no faster than these.
+// 16-bit operands (E) that no tensor-core kernel takes, odd rows above all: [500, 999] x [1001, 999]^T 169 -> 46 us, [11, 2001] x
+// [200, 2001]^T 267 -> 38 on 64 x 64 tiles of one 16-deep buffer before.
 template <int WM, int WK> struct F32Tile {
   static constexpr int BM = 32 * WM, BN = 128, BK = 16, THREADS = 32 * WM * WK;
   static constexpr int STAGE = BK * (BM + BN);                                     // floats
   static constexpr int SMEM = 2 * STAGE * 4, SMEM_REDUCE = WK * BM * BN * 4;       // bytes; the sums come after the slices
 };
 struct F32Params {
-  float *c;
-  const float *a, *b;
+  void *c;
+  const void *a, *b;
   int m, n, k;
   long long a_rs, a_cs, a_b, b_rs, b_cs, b_b, c_rs, c_b;
   int split, k_per_split;                              // CTAs of a cluster along k
@@ -260,7 +205,7 @@ __device__ __forceinline__ float2 halves(uint64_t v) {
   return r;
 }
 
-template <int WM, int WK, bool VEC>
+template <typename E, int WM, int WK, bool VEC>
 __global__ void __launch_bounds__(128, 2)
 f32_tile_kernel(const F32Params p) {
   using T = F32Tile<WM, WK>;
@@ -272,19 +217,20 @@ f32_tile_kernel(const F32Params p) {
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int rank = p.split > 1 ? (int)(blockIdx.x % p.split) : 0, n0 = (int)(p.split > 1 ? blockIdx.x / p.split : blockIdx.x) * BN;
   const int m0 = blockIdx.y * BM;
-  const float *A = p.a + (long long)blockIdx.z * p.a_b, *B = p.b + (long long)blockIdx.z * p.b_b;
+  const E *A = (const E *)p.a + (long long)blockIdx.z * p.a_b, *B = (const E *)p.b + (long long)blockIdx.z * p.b_b;
+  static_assert(!VEC || sizeof(E) == 4, "16-byte pieces are four floats");
   const int k_lo = rank * p.k_per_split, k_hi = min(p.k, k_lo + p.k_per_split);
 
   // One operand's slice: R rows of 16 k, in pieces of four values along the contiguous direction
-  auto fetch = [&](auto &reg, const float *src, long long rs, long long ks, int r0, int rows, int R, int k0) {
+  auto fetch = [&](auto &reg, const E *src, long long rs, long long ks, int r0, int rows, int R, int k0) {
     const bool kc = ks == 1;
 #pragma unroll
     for (int i = 0; i < (int)(sizeof(reg) / sizeof(float4)); ++i) {
       const int q = t + i * 128;
       const int r = r0 + (kc ? q / QK : q % (R / 4) * 4), k = k0 + (kc ? q % QK * 4 : q / (R / 4));
       float v[4] = {0.f, 0.f, 0.f, 0.f};
-      const float *at = src + r * rs + k * ks;
-      if (VEC) {                                       // a piece is all in or all out
+      const E *at = src + r * rs + k * ks;
+      if constexpr (VEC) {                             // a piece is all in or all out
         if (r < rows && k < k_hi) {
           const float4 w = __ldg(reinterpret_cast<const float4 *>(at));
           v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
@@ -292,7 +238,7 @@ f32_tile_kernel(const F32Params p) {
       } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (kc ? r < rows && k + e < k_hi : r + e < rows && k < k_hi) v[e] = __ldg(at + e * (kc ? ks : rs));
+          if (kc ? r < rows && k + e < k_hi : r + e < rows && k < k_hi) v[e] = to_f32<E>(__ldg(at + e * (kc ? ks : rs)));
       }
       reg[i] = make_float4(v[0], v[1], v[2], v[3]);
     }
@@ -366,18 +312,18 @@ f32_tile_kernel(const F32Params p) {
     }
   }
 
-  float *C = p.c + (long long)blockIdx.z * p.c_b;
+  E *C = (E *)p.c + (long long)blockIdx.z * p.c_b;
   auto store = [&](int row, int col, float4 v) {       // row, col inside the tile
     const int gi = m0 + row, gj = n0 + col;
     if (gi >= p.m) return;
-    float *at = C + gi * p.c_rs + gj;
+    E *at = C + gi * p.c_rs + gj;
     if (VEC && gj + 3 < p.n) {
-      *reinterpret_cast<float4 *>(at) = v;
+      if constexpr (VEC) *reinterpret_cast<float4 *>(at) = v;
     } else {
       const float w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        if (gj + e < p.n) at[e] = w[e];
+        if (gj + e < p.n) at[e] = from_f32<E>(w[e]);
     }
   };
   const bool alone = WK == 1 && p.split == 1;
@@ -439,25 +385,26 @@ F32Shape f32_shape(int sm_count, size_t b, size_t m, size_t n, size_t k) {
   return best;
 }
 
-template <int WM, int WK, bool VEC>
+template <typename E, int WM, int WK, bool VEC>
 int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b) {
   using T = F32Tile<WM, WK>;
   const dim3 grid((unsigned)((p.n + T::BN - 1) / T::BN * p.split), (unsigned)((p.m + T::BM - 1) / T::BM), (unsigned)b);
   const size_t smem = WK * p.split > 1 ? std::max(T::SMEM, T::SMEM_REDUCE) : T::SMEM;
-  if (smem > 48 * 1024) UGB_CUDA(dev, cudaFuncSetAttribute(f32_tile_kernel<WM, WK, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const cudaError_t e = ugb_launch_cluster(f32_tile_kernel<WM, WK, VEC>, grid, dim3(T::THREADS), smem, dev->stream, true, p.split, p);
+  if (smem > 48 * 1024) UGB_CUDA(dev, cudaFuncSetAttribute(f32_tile_kernel<E, WM, WK, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const cudaError_t e = ugb_launch_cluster(f32_tile_kernel<E, WM, WK, VEC>, grid, dim3(T::THREADS), smem, dev->stream, true, p.split, p);
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of f32_tile_kernel failed: %s", cudaGetErrorString(e));
   return ugb_after_launch(dev, "f32_tile_kernel");
 }
 
-int32_t launch_f32_tile(ugb_device *dev, F32Params p, size_t b, bool vec) {
+template <typename E, bool VEC>
+int32_t launch_f32_tile(ugb_device *dev, F32Params p, size_t b) {
   const F32Shape s = f32_shape(dev->sm_count, b, p.m, p.n, p.k);
-  UGB_REQUIRE(dev, b <= 65535 && ((size_t)p.m + 127) / 128 <= 65535, UGB_ERR_UNSUPPORTED, "matmul: m too large for the f32 kernel");
+  UGB_REQUIRE(dev, b <= 65535 && ((size_t)p.m + 127) / 128 <= 65535, UGB_ERR_UNSUPPORTED, "matmul: m or batch too large for the FP32-pipe kernel");
   p.split = s.split;
   p.k_per_split = (int)((((size_t)p.k + s.split - 1) / s.split + 15) / 16 * 16);
-  if (s.wk == 4) return vec ? launch_f32_shape<1, 4, true>(dev, p, b) : launch_f32_shape<1, 4, false>(dev, p, b);
-  if (s.wk == 2) return vec ? launch_f32_shape<2, 2, true>(dev, p, b) : launch_f32_shape<2, 2, false>(dev, p, b);
-  return vec ? launch_f32_shape<4, 1, true>(dev, p, b) : launch_f32_shape<4, 1, false>(dev, p, b);
+  if (s.wk == 4) return launch_f32_shape<E, 1, 4, VEC>(dev, p, b);
+  if (s.wk == 2) return launch_f32_shape<E, 2, 2, VEC>(dev, p, b);
+  return launch_f32_shape<E, 4, 1, VEC>(dev, p, b);
 }
 
 int32_t launch_f32(ugb_device *dev, float *dst, const float *lhs, const float *rhs, size_t b, size_t m, size_t n, size_t k,
@@ -488,19 +435,10 @@ int32_t launch_f32(ugb_device *dev, float *dst, const float *lhs, const float *r
   const size_t a_c = L.transposed ? m : k, a_ld = (size_t)(L.transposed ? L.cs : L.rs);
   const size_t b_c = R.transposed ? k : n, b_ld = (size_t)(R.transposed ? R.cs : R.rs);
   const bool vec = bases && a_c % 4 == 0 && a_ld % 4 == 0 && b_c % 4 == 0 && b_ld % 4 == 0 && n % 4 == 0;
-  return launch_f32_tile(dev, {dst, lhs, rhs, (int)m, (int)n, (int)k, L.rs, L.cs, L.batch, R.rs, R.cs, R.batch, (long long)n, (long long)(m * n), 1, 0}, b, vec);
-}
-
-template <typename T>
-int32_t launch_simt(ugb_device *dev, void *dst, const void *lhs, const void *rhs, size_t b, size_t m,
-                    size_t n, size_t k, const MatLayout &L, const MatLayout &R) {
-  dim3 grid((unsigned)((n + 63) / 64), (unsigned)((m + 63) / 64), (unsigned)b);
-  UGB_REQUIRE(dev, grid.y <= 65535 && grid.z <= 65535, UGB_ERR_UNSUPPORTED,
-              "matmul: m or batch too large for the SIMT kernel");
-  simt_gemm_kernel<T><<<grid, 256, 0, dev->stream>>>((T *)dst, (const T *)lhs, (const T *)rhs,
-                                                     (int)m, (int)n, (int)k, L.rs, L.cs, L.batch,
-                                                     R.rs, R.cs, R.batch);
-  return ugb_after_launch(dev, "simt_gemm_kernel");
+  {
+    const F32Params p{dst, lhs, rhs, (int)m, (int)n, (int)k, L.rs, L.cs, L.batch, R.rs, R.cs, R.batch, (long long)n, (long long)(m * n), 1, 0};
+    return vec ? launch_f32_tile<float, true>(dev, p, b) : launch_f32_tile<float, false>(dev, p, b);
+  }
 }
 
 }  // namespace
@@ -562,7 +500,10 @@ int32_t ugb_f32_gemm(ugb_device *dev, float *c, const float *a, const float *b, 
   const bool vec = al16(c) && al16(a) && al16(b) && k % 4 == 0 && n % 4 == 0 && a_ld % 4 == 0 && c_ld % 4 == 0 &&
                    a_batch % 4 == 0 && b_batch % 4 == 0 && c_batch % 4 == 0;
   const long long b_rs = b_is_nk ? 1 : (long long)n, b_cs = b_is_nk ? (long long)k : 1;
-  return launch_f32_tile(dev, {c, a, b, (int)m, (int)n, (int)k, (long long)a_ld, 1, (long long)a_batch, b_rs, b_cs, (long long)b_batch, (long long)c_ld, (long long)c_batch, 1, 0}, batch, vec);
+  {
+    const F32Params p{c, a, b, (int)m, (int)n, (int)k, (long long)a_ld, 1, (long long)a_batch, b_rs, b_cs, (long long)b_batch, (long long)c_ld, (long long)c_batch, 1, 0};
+    return vec ? launch_f32_tile<float, true>(dev, p, batch) : launch_f32_tile<float, false>(dev, p, batch);
+  }
 }
 
 extern "C" {
@@ -617,8 +558,8 @@ int32_t ugb_matmul(ugb_device *dev, ugb_slice *dst, const ugb_slice *lhs, const 
     const int32_t src = ugb_skinny_gemm(dev, g);
     if (src != UGB_ERR_UNSUPPORTED) return src;
   }
-  // Tiny products do not fill a 128-row tensor-core tile; the strided kernel handles them.
-  if ((dt == UGB_BF16 || dt == UGB_F16) && !L.transposed && m >= 16 && m * n >= 128 * 64) {
+  // Few results of a short k finish on the FFMA kernel before a tensor-core tile is set up ([1, 3, 1616] x [1616, 328]: 28 us there).
+  if ((dt == UGB_BF16 || dt == UGB_F16) && !L.transposed && (m * n >= 128 * 64 || k >= 256)) {
     // tensor-core path (bf16 and f16 are the same tcgen05.mma.kind::f16 instruction with another format field, as
     // both go to cublasGemmStridedBatchedEx in the reference, gemm.rs:130-232): A [m,k] row-major, B either
     // [n,k] row-major ("TN", matmul_t with a weight) or [k,n] row-major ("NN").
@@ -627,8 +568,14 @@ int32_t ugb_matmul(ugb_device *dev, ugb_slice *dst, const ugb_slice *lhs, const 
   }
   switch (dt) {
     case UGB_F32: return launch_f32(dev, (float *)dst->ptr, (const float *)lp, (const float *)rp, b, m, n, k, L, R);
-    case UGB_BF16: return launch_simt<__nv_bfloat16>(dev, dst->ptr, lp, rp, b, m, n, k, L, R);
-    default: return launch_simt<__half>(dev, dst->ptr, lp, rp, b, m, n, k, L, R);
+    default: {
+      if (k == 0) {
+        UGB_CUDA(dev, cudaMemsetAsync(dst->ptr, 0, b * m * n * es, dev->stream));
+        return UGB_OK;
+      }
+      const F32Params p{dst->ptr, lp, rp, (int)m, (int)n, (int)k, L.rs, L.cs, L.batch, R.rs, R.cs, R.batch, (long long)n, (long long)(m * n), 1, 0};
+      return dt == UGB_BF16 ? launch_f32_tile<__nv_bfloat16, false>(dev, p, b) : launch_f32_tile<__half, false>(dev, p, b);
+    }
   }
 }
 
