@@ -55,7 +55,8 @@ embed_gather_kernel(const __nv_bfloat16 *__restrict__ embed, const int *__restri
 // x[b, :] += sum_s part[s][b][:]   (split-K partials of the previous projection,
 // summed in a fixed order), then xn = bf16(x / sqrt(mean(x^2) + eps) * alpha).
 // One CTA of 256 threads per row; hidden <= 8192, hidden % 4 == 0.
-template <int VPT>
+// FEW: few rows, each alone on its SM: many partials in flight; otherwise occupancy hides their latency.
+template <int VPT, bool FEW>
 __global__ void __launch_bounds__(256)
 reduce_rmsnorm_kernel(float *__restrict__ x, const float *__restrict__ part, int n_part,
                       size_t part_stride, const float *__restrict__ alpha,
@@ -100,15 +101,30 @@ reduce_rmsnorm_kernel(float *__restrict__ x, const float *__restrict__ part, int
         ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
       }
     }
-  } else
+  } else {
+    // split-K partials, U of them in flight, added in order
+    constexpr int U = !FEW ? 2 : VPT <= 2 ? 8 : (VPT <= 4 ? 4 : 2);
+    for (int s = 0; s < n_part; s += U) {
+      float4 q[U][VPT];
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int c = threadIdx.x + i * 256;
-    if (c < nvec) {
-      for (int s = 0; s < n_part; ++s) {
-        const float4 p = __ldcs(reinterpret_cast<const float4 *>(part + s * part_stride + (size_t)b * hidden) + c);
-        v[i].x += p.x; v[i].y += p.y; v[i].z += p.z; v[i].w += p.w;
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+          const int c = threadIdx.x + i * 256;
+          q[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (c < nvec && s + u < n_part) q[u][i] = __ldcs(reinterpret_cast<const float4 *>(part + (s + u) * part_stride + (size_t)b * hidden) + c);
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (s + u >= n_part) break;
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) { v[i].x += q[u][i].x; v[i].y += q[u][i].y; v[i].z += q[u][i].z; v[i].w += q[u][i].w; }
       }
+    }
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int c = threadIdx.x + i * 256;
+      if (c >= nvec) continue;
       if (n_part > 0) xr[c] = v[i];
       ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
     }

@@ -207,15 +207,25 @@ row_update_kernel(RowArgs<T> a) {
         for (int i = 0; i < VPT; ++i) { y[i].x += q[u][i].x; y[i].y += q[u][i].y; y[i].z += q[u][i].z; y[i].w += q[u][i].w; }
     }
   }
-  for (int k = 0; k < a.top; ++k) {
-    const int to = __ldcg(a.slot + (size_t)r * a.top + k);
-    if (to < 0) continue;
+  // the experts' rows: first all places, then all rows, so that a step pays two round trips and not two for each expert
+  constexpr int EX = STEP ? (VPT <= 2 ? 4 : 2) : 1;
+  for (int k = 0; k < a.top; k += EX) {
+    int to[EX];
+    float4 q[EX][VPT];
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * 256;
-      if (c >= nvec) continue;
-      const float4 q = __ldcs(reinterpret_cast<const float4 *>(a.routed + (size_t)to * a.ld) + c);
-      y[i].x += q.x; y[i].y += q.y; y[i].z += q.z; y[i].w += q.w;
+    for (int e = 0; e < EX; ++e) to[e] = k + e < a.top ? __ldcg(a.slot + (size_t)r * a.top + k + e) : -1;
+#pragma unroll
+    for (int e = 0; e < EX; ++e)
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int c = threadIdx.x + i * 256;
+        q[e][i] = to[e] >= 0 && c < nvec ? __ldcs(reinterpret_cast<const float4 *>(a.routed + (size_t)to[e] * a.ld) + c) : zero;
+      }
+#pragma unroll
+    for (int e = 0; e < EX; ++e) {
+      if (to[e] < 0) continue;
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) { y[i].x += q[e][i].x; y[i].y += q[e][i].y; y[i].z += q[e][i].z; y[i].w += q[e][i].w; }
     }
   }
   if (a.bias) {

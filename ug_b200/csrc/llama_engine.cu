@@ -192,10 +192,15 @@ int32_t launch_reduce_rmsnorm_rows(ugb_llama *m, int rows, float *x, __nv_bfloat
   cudaStream_t st = m->dev->stream;
   const bool pdl = m->pdl != 0;
   cudaError_t e;
-  if (nvec <= 256) e = ugb_launch(reduce_rmsnorm_kernel<1>, grid, dim3(256), 0, st, pdl, x, part, n_part, stride, alpha, xn, hidden, inv_d, eps, early);
-  else if (nvec <= 512) e = ugb_launch(reduce_rmsnorm_kernel<2>, grid, dim3(256), 0, st, pdl, x, part, n_part, stride, alpha, xn, hidden, inv_d, eps, early);
-  else if (nvec <= 1024) e = ugb_launch(reduce_rmsnorm_kernel<4>, grid, dim3(256), 0, st, pdl, x, part, n_part, stride, alpha, xn, hidden, inv_d, eps, early);
-  else e = ugb_launch(reduce_rmsnorm_kernel<8>, grid, dim3(256), 0, st, pdl, x, part, n_part, stride, alpha, xn, hidden, inv_d, eps, early);
+  const bool few = rows <= 2 * m->dev->sm_count;
+#define UGB_REDUCE(VPT) \
+  e = few ? ugb_launch(reduce_rmsnorm_kernel<VPT, true>, grid, dim3(256), 0, st, pdl, x, part, n_part, stride, alpha, xn, hidden, inv_d, eps, early) \
+          : ugb_launch(reduce_rmsnorm_kernel<VPT, false>, grid, dim3(256), 0, st, pdl, x, part, n_part, stride, alpha, xn, hidden, inv_d, eps, early)
+  if (nvec <= 256) UGB_REDUCE(1);
+  else if (nvec <= 512) UGB_REDUCE(2);
+  else if (nvec <= 1024) UGB_REDUCE(4);
+  else UGB_REDUCE(8);
+#undef UGB_REDUCE
   if (e != cudaSuccess) return ugb_fail(m->dev, UGB_ERR_CUDA, "launch of reduce_rmsnorm_kernel failed: %s", cudaGetErrorString(e));
   return ugb_after_launch(m->dev, "reduce_rmsnorm_kernel");
 }
