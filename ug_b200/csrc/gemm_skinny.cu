@@ -39,6 +39,7 @@ struct Params {
   int epi, late_trigger, wait_first;       // wait_first: a kernel of the stream may write W
   const int *groups;                       // expert of group tile i, -1 behind the last; or null
   int n_groups_tiles, tile_m;
+  ugb_skinny_gate gate;                    // GATE: where the activations come from
 };
 
 static __device__ __forceinline__ uint4 ld_stream(const void *p) {     // read once: past L1
@@ -60,8 +61,40 @@ template <bool F16> static __device__ __forceinline__ void store16(void *out, lo
   else reinterpret_cast<__nv_bfloat16 *>(out)[i] = __float2bfloat16_rn(v);
 }
 
+// Activations k .. k + 7 of row r, formed from the product before: gelu_tanh(sum of its partials) * the row's token in the table,
+// rounded to bf16.  Every CTA does it again for all of its k (2048 values of 1024 bytes of partials and table each); what it
+// saves is a kernel between two products of 1 MB (Zidevik, 8 sequences: 28 of them a step, request of 32 steps 96.4 -> 95.0 ms).
+static __device__ __forceinline__ uint4 gated_act(const ugb_skinny_gate &q, int r, int k) {
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const int id = q.tok[r];
+  uint4 e = make_uint4(0, 0, 0, 0);
+  if (id >= 0 && id < q.vocab) e = __ldg(reinterpret_cast<const uint4 *>(q.table + (size_t)id * q.table_ld + q.off + k));
+  const float *row = q.part + (size_t)r * q.ld + k;
+  for (int p = 0; p < q.n_part; p += 4) {  // the partials are added in order
+    float4 v[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        v[j][h] = p + j < q.n_part ? __ldcg(reinterpret_cast<const float4 *>(row + (size_t)(p + j) * q.part_stride) + h) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) { s[4 * h] += v[j][h].x; s[4 * h + 1] += v[j][h].y; s[4 * h + 2] += v[j][h].z; s[4 * h + 3] += v[j][h].w; }
+  }
+  const uint32_t w[4] = {e.x, e.y, e.z, e.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w[j]));
+    const __nv_bfloat162 y = __floats2bfloat162_rn(ugb_gelu_tanh(s[2 * j]) * t.x, ugb_gelu_tanh(s[2 * j + 1]) * t.y);
+    o[j] = *reinterpret_cast<const uint32_t *>(&y);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // KC: chunks of a warp per piece; a unit whose split is longer runs in p.spans pieces.
-template <int KC, bool F16>
+template <int KC, bool F16, bool GATE = false>
 __global__ void __launch_bounds__(THREADS, 2)
 skinny_gemm_kernel(const Params p) {
   __shared__ float red[2][WARPS][8 * RED_LD];
@@ -136,6 +169,11 @@ skinny_gemm_kernel(const Params p) {
       for (int i = 0; i < KC; ++i) {
         const int c = lc + i * WARPS, k = c * CHUNK + 8 * t;
         const bool on = g < p.rows && c < lc1;
+        if constexpr (GATE) {
+          act[i][0] = on && k < p.k ? gated_act(p.gate, g, k) : make_uint4(0, 0, 0, 0);
+          act[i][1] = on && k + 32 < p.k ? gated_act(p.gate, g, k + 32) : make_uint4(0, 0, 0, 0);
+          continue;
+        }
         act[i][0] = on && k < p.k ? __ldcg(reinterpret_cast<const uint4 *>(row + 2 * (size_t)k)) : make_uint4(0, 0, 0, 0);
         act[i][1] = on && k + 32 < p.k ? __ldcg(reinterpret_cast<const uint4 *>(row + 2 * (size_t)k + 64)) : make_uint4(0, 0, 0, 0);
       }
@@ -202,7 +240,7 @@ int ugb_skinny_splits(int sm_count, size_t n, size_t k) {
   return ugb_skinny_effective_splits(k, std::min(UGB_SKINNY_SPLITS, std::max(need, fill)));
 }
 
-int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_per_tile) {
+int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_per_tile, const ugb_skinny_gate *gate) {
   ugb_tc_gemm_args g = args;
   const long long dense_c = (long long)g.m * (long long)(g.epi == UGB_EPI_SILU_MUL_BF16 ? g.n / 2 : g.n);
   if (g.batch > 1 && g.b_batch == 0 && g.a_ld == 0 && g.c_ld == 0 && g.a_batch == (long long)(g.m * g.k) && (g.c_batch == 0 || g.c_batch == dense_c)) {
@@ -233,6 +271,13 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
   p.chunks_per_split = (p.chunks + p.splits - 1) / p.splits;
   const int kc = std::min(MAX_CHUNKS, (p.chunks_per_split + WARPS - 1) / WARPS);
   p.spans = (p.chunks_per_split + kc * WARPS - 1) / (kc * WARPS);
+  if (gate) {                              // 16-byte pieces of the table's and the partials' rows, all of k in registers
+    if (g.groups || g.f16 || g.batch != 1 || p.splits != 1 || kc != 1 || p.spans != 1 || gate->n_part < 1) return UGB_ERR_UNSUPPORTED;
+    if (((uintptr_t)gate->part | (uintptr_t)gate->table) & 15 || gate->part_stride % 4 != 0 || gate->ld % 4 != 0 || gate->table_ld % 8 != 0 || gate->off % 8 != 0 ||
+        gate->n % 8 != 0 || (size_t)gate->n != g.k)
+      return UGB_ERR_UNSUPPORTED;
+    p.gate = *gate;
+  }
   p.epi = g.epi;
   p.late_trigger = g.late_trigger ? 1 : 0;
   p.wait_first = !g.b_static && !g.groups ? 1 : 0;
@@ -255,7 +300,8 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
 #define UGB_SKINNY(KC) \
   e = g.f16 ? ugb_launch(skinny_gemm_kernel<KC, true>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p) \
             : ugb_launch(skinny_gemm_kernel<KC, false>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p)
-  switch (kc) { case 1: UGB_SKINNY(1); break; case 2: UGB_SKINNY(2); break; case 3: UGB_SKINNY(3); break; default: UGB_SKINNY(4); }
+  if (gate) e = ugb_launch(skinny_gemm_kernel<1, false, true>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p);
+  else switch (kc) { case 1: UGB_SKINNY(1); break; case 2: UGB_SKINNY(2); break; case 3: UGB_SKINNY(3); break; default: UGB_SKINNY(4); }
 #undef UGB_SKINNY
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of skinny_gemm_kernel failed: %s", cudaGetErrorString(e));
   return ugb_after_launch(dev, "skinny_gemm_kernel");

@@ -14,8 +14,25 @@ inline bool ugb_skinny_rows(size_t rows) { return rows >= 1 && rows <= (size_t)U
 // not fill the SMs.
 int ugb_skinny_splits(int sm_count, size_t n, size_t k);
 
+// gelu_tanh
+static __device__ __forceinline__ float ugb_gelu_tanh(float x) { return 0.5f * x * (1.0f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x))); }
+
+// Activations that the kernel forms itself: A[r, j] = bf16(gelu_tanh(sum_p part[p][r][j]) * table[tok[r]][off + j]), j < n = k; 0 for a
+// token outside the table.
+struct ugb_skinny_gate {
+  const float *part;
+  int n_part;
+  size_t part_stride;
+  int ld, n;
+  const int *tok;
+  const __nv_bfloat16 *table;
+  size_t table_ld;
+  int off, vocab;
+};
+
 // out = A . W^T for up to 8 rows, arguments and epilogues as ugb_tc_gemm (no rope, no n-major B, no pair_k); `splits` as
 // given, rounded as ugb_skinny_effective_splits says.  Grouped rows: tiles of g.tile_m rows of which the first
 // `rows_per_tile` may hold something; m is their total.  UGB_ERR_UNSUPPORTED (last_error untouched) for what it does not take.
-int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &g, int rows_per_tile = 0);
+// With `gate`, g.a is not read (f32 or bf16 result, k of 512 at most).
+int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &g, int rows_per_tile = 0, const ugb_skinny_gate *gate = nullptr);
 int ugb_skinny_effective_splits(size_t k, int splits);

@@ -78,9 +78,10 @@ int32_t ugb_hybrid_matmul(ugb_hybrid *m, const Mat &x) {
   g.splits = x.splits; g.bn = x.bn; g.b_static = x.groups == nullptr; g.pdl = m->pdl != 0; g.late_trigger = true;
   g.groups = x.groups; g.n_groups = x.n_groups; g.tile_m = x.tile;
   if (ugb_skinny_rows(x.groups ? (size_t)x.tile_rows : x.m)) {
-    const int32_t rc = ugb_skinny_gemm(dev, g, x.tile_rows);
+    const int32_t rc = ugb_skinny_gemm(dev, g, x.tile_rows, x.gate);
     if (rc != UGB_ERR_UNSUPPORTED) return rc;
   }
+  if (x.gate) return UGB_ERR_UNSUPPORTED;                    // the caller forms them itself
   g.smem_kib = x.m <= 64 || (x.groups && x.tile == 64) ? 144 : 0;
   if (!x.f32_out && !x.groups && x.batch == 1 && x.nk && x.m <= 64 && x.k >= 256) {
     // a T result cannot be split into partials: the two k halves of a tile on a pair of CTAs, with the narrowest tile that fits the SMs

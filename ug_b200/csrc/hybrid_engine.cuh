@@ -69,6 +69,7 @@ struct ugb_hybrid_work {
   float4 *choice = nullptr;                                // {expert, place, weight}
 };
 
+struct ugb_skinny_gate;
 struct ugb_hybrid_mat {            // out[b, m, n] = a . w
   void *out; const void *a, *w;
   size_t m, n, k, batch = 1, a_ld = 0, a_batch = 0, w_batch = 0, c_ld = 0, c_batch = 0;
@@ -80,6 +81,7 @@ struct ugb_hybrid_mat {            // out[b, m, n] = a . w
   int tile = 0, n_groups = 0;
   int tile_rows = 0;               // rows of a tile that may hold something (0: all)
   int splits = 1, bn = 0;
+  const ugb_skinny_gate *gate = nullptr;   // up to 8 rows: activations formed inside the product (see gemm_skinny.cuh)
 };
 
 struct ugb_hybrid_tiling { int bn, splits; };

@@ -14,7 +14,7 @@
 //   GEMM cat -> f32                                     output projections of mixer and feed-forward as one product
 //   row_update      stream += product + experts' rows;  copy -> T (token input or loop) or norm -> h
 //   (a step runs feed-forward and experts ahead of the scan, see run())
-//   [token input]  GEMM gate;  token_gate;  GEMM proj -> f32;  row_update  stream += norm(product);  copy or norm
+//   [token input]  GEMM gate;  token_gate (a step of few rows: inside proj);  GEMM proj -> f32;  row_update  stream += norm(product);  copy or norm
 // The factors of attention and scan are applied where their f32 results are rounded to T.  Products with a f32 result are
 // split over k in a step; the consumer sums the partials.
 //
@@ -26,6 +26,7 @@
 #include <string>
 
 #include "attention_tc.cuh"
+#include "gemm_skinny.cuh"
 #include "gemm_tcgen05.cuh"
 #include "grouped_attention.cuh"
 #include "hybrid_engine.cuh"
@@ -297,18 +298,26 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
         g.splits = g_t.splits; g.bn = !decode && g_t.splits > 1 ? 256 : g_t.bn;
         if ((rc = ugb_hybrid_matmul(m, g))) return rc;
       }
-      if (m->on(UGB_HYBRID_K_SIDE_GATE)) {
+      Mat g{w.prod, w.side_h, L.side_proj, (size_t)rows, (size_t)wl, (size_t)m->sl};
+      g.splits = p_t.splits; g.bn = p_t.bn;
+      bool formed = false;                                   // a step of few rows forms the gate inside the second product
+      if (decode && !m->f32 && m->only == UGB_HYBRID_K_ALL && t_block == 1) {
+        const ugb_skinny_gate q{(const float *)w.side, g_t.splits, (size_t)rows * m->sl, m->sl, m->cfg.side_dim, tok, (const __nv_bfloat16 *)m->side_embed,
+                                (size_t)m->cfg.layers * m->cfg.side_dim, R.layer * m->cfg.side_dim, m->cfg.vocab};
+        g.gate = &q;
+        rc = ugb_hybrid_matmul(m, g);
+        if (rc != UGB_OK && rc != UGB_ERR_UNSUPPORTED) return rc;
+        formed = rc == UGB_OK;
+        g.gate = nullptr;
+      }
+      if (!formed && m->on(UGB_HYBRID_K_SIDE_GATE)) {
         e = ugb_launch(token_gate_kernel<T>, dim3((unsigned)(((size_t)rows * m->sl / 4 + 255) / 256)), dim3(256), 0, dev->stream, pdl, w.side, g_t.splits,
                        (size_t)rows * m->sl, (size_t)rows * m->sl / 4, m->sl, m->cfg.side_dim, tok, t, t_block, off, (const T *)m->side_embed, (size_t)m->cfg.layers * m->cfg.side_dim,
                        R.layer * m->cfg.side_dim, m->cfg.vocab, (T *)w.side_h);
         if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of token_gate_kernel failed: %s", cudaGetErrorString(e));
         if ((rc = ugb_after_launch(dev, "token_gate_kernel"))) return rc;
       }
-      if (m->on(UGB_HYBRID_K_SIDE)) {
-        Mat g{w.prod, w.side_h, L.side_proj, (size_t)rows, (size_t)wl, (size_t)m->sl};
-        g.splits = p_t.splits; g.bn = p_t.bn;
-        if ((rc = ugb_hybrid_matmul(m, g))) return rc;
-      }
+      if (!formed && m->on(UGB_HYBRID_K_SIDE) && (rc = ugb_hybrid_matmul(m, g))) return rc;
       RowArgs<T> s;
       s.part = w.prod; s.n_part = p_t.splits; s.part_stride = (size_t)rows * wl; s.x = w.x; s.post_gain = L.side_gain;
       prepare(s, i + 1);

@@ -2,6 +2,7 @@
 // its attention, scan and experts, and the token input behind a layer.  T is the activation type; rotations, norms,
 // router scores and gates are f32 whatever T is.
 #pragma once
+#include "gemm_skinny.cuh"
 #include "hybrid_kernels.cuh"
 
 namespace ugb_hybrid_k {
@@ -363,8 +364,7 @@ token_gate_kernel(const float *__restrict__ part, int n_part, size_t part_stride
         if (j + k < n) e[k] = (float)src[k];
     }
   }
-  auto gelu = [](float x) { return 0.5f * x * (1.0f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x))); };
-  Act<T>::st4(out + (size_t)r * ld + j, make_float4(gelu(s.x) * e[0], gelu(s.y) * e[1], gelu(s.z) * e[2], gelu(s.w) * e[3]));
+  Act<T>::st4(out + (size_t)r * ld + j, make_float4(ugb_gelu_tanh(s.x) * e[0], ugb_gelu_tanh(s.y) * e[1], ugb_gelu_tanh(s.z) * e[2], ugb_gelu_tanh(s.w) * e[3]));
 }
 
 // ------------------------------------------------------- logits, loading ----
