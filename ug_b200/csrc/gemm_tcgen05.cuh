@@ -69,7 +69,7 @@ struct ugb_tc_gemm_args {
 
 // Returns UGB_ERR_UNSUPPORTED (without touching last_error) when the shape
 // does not meet the kernel's alignment rules so that the caller can fall back
-// to the strided kernel.
+// to the FFMA kernel.
 int32_t ugb_tc_gemm(ugb_device *dev, const ugb_tc_gemm_args &args);
 // Tile shape for more than 64 rows: width, 256-row tiles on pairs of CTAs, and a k split where the caller takes f32 partials
 // (max_splits > 1; the pair shapes do not split).  `pairs`: pairs may be chosen at all.
