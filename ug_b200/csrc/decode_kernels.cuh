@@ -29,7 +29,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // One CTA per row; ids outside the table raise the status word and leave the row
 // untouched.
 static __global__ void __launch_bounds__(256)
-embed_gather_kernel(const __nv_bfloat16 *__restrict__ embed, const int *__restrict__ tok,
+embed_gather_kernel(const __nv_bfloat16 *__restrict__ embed, const int *tok,
                     float *__restrict__ x, int hidden, int vocab, ugb_status_word *status,
                     int t, int tok_stride, int tok_off) {
   ugb_pdl_trigger();
@@ -58,7 +58,7 @@ embed_gather_kernel(const __nv_bfloat16 *__restrict__ embed, const int *__restri
 // FEW: few rows, each alone on its SM: many partials in flight; otherwise occupancy hides their latency.
 template <int VPT, bool FEW>
 __global__ void __launch_bounds__(256)
-reduce_rmsnorm_kernel(float *__restrict__ x, const float *__restrict__ part, int n_part,
+reduce_rmsnorm_kernel(float *__restrict__ x, const float *part, int n_part,
                       size_t part_stride, const float *__restrict__ alpha,
                       __nv_bfloat16 *__restrict__ xn, int hidden, float inv_d, float eps, int early) {
   __shared__ float sm[8];
@@ -159,9 +159,9 @@ reduce_rmsnorm_kernel(float *__restrict__ x, const float *__restrict__ part, int
 // sums and of the cos / sin rows, 64- or 128-bit bf16 stores -- so that all of a
 // thread's loads are independent and issued at once.  hd % 8 == 0.
 static __global__ void __launch_bounds__(256)
-rope_append_kernel(const float *__restrict__ part, int n_part, size_t part_stride,
+rope_append_kernel(const float *part, int n_part, size_t part_stride,
                    const float *__restrict__ cos_, const float *__restrict__ sin_,
-                   const int *__restrict__ pos_p, __nv_bfloat16 *__restrict__ q_out,
+                   const int *pos_p, __nv_bfloat16 *__restrict__ q_out,
                    __nv_bfloat16 *__restrict__ kcache, __nv_bfloat16 *__restrict__ vcache,
                    int n_heads, int n_kv, int hd, int t_max, int interleaved, int t, int pos_off) {
   ugb_pdl_trigger();
@@ -296,8 +296,8 @@ constexpr int att_dyn_smem(int stages, bool tma) {
 
 template <int NSTAGE, bool TMA = false>
 __global__ void __launch_bounds__(ATT_WARPS * 32)
-decode_attention_kernel_t(const __nv_bfloat16 *__restrict__ q, __nv_bfloat16 *__restrict__ kcache,
-                        __nv_bfloat16 *__restrict__ vcache, const int *__restrict__ pos_p,
+decode_attention_kernel_t(const __nv_bfloat16 *q, __nv_bfloat16 *__restrict__ kcache,
+                        __nv_bfloat16 *__restrict__ vcache, const int *pos_p,
                         float *__restrict__ part_o, float *__restrict__ part_ml,
                         unsigned int *__restrict__ counters, __nv_bfloat16 *__restrict__ out,
                         int n_heads, int n_kv, int group, int t_max, float scale, AttRope rope,
@@ -357,8 +357,8 @@ decode_attention_kernel_t(const __nv_bfloat16 *__restrict__ q, __nv_bfloat16 *__
     uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
     if (g < group) {
       const uint4 *qp = reinterpret_cast<const uint4 *>(q + ((size_t)b * n_heads + kvh * group + g) * ATT_HD + 16 * t);
-      lo = __ldg(qp);
-      hi = __ldg(qp + 1);
+      lo = qp[0];
+      hi = qp[1];
     }
     qa[0] = lo.x; qa[1] = lo.y; qa[2] = lo.z; qa[3] = lo.w;
     qa[4] = hi.x; qa[5] = hi.y; qa[6] = hi.z; qa[7] = hi.w;
@@ -708,7 +708,7 @@ decode_attention_kernel_t(const __nv_bfloat16 *__restrict__ q, __nv_bfloat16 *__
 // advances the shared position counter.  One CTA of 1024 threads per row,
 // 128-bit loads; rows of `vocab` values, ld elements apart (ld % 4 == 0).
 static __global__ void __launch_bounds__(1024)
-argmax_rows_kernel(const float *__restrict__ logits, int vocab, int ld, int *__restrict__ next, int *pos_p) {
+argmax_rows_kernel(const float *logits, int vocab, int ld, int *__restrict__ next, int *pos_p) {
   __shared__ float sv[32];
   __shared__ int si[32];
   ugb_pdl_trigger();

@@ -42,9 +42,15 @@ struct Params {
   ugb_skinny_gate gate;                    // GATE: where the activations come from
 };
 
-static __device__ __forceinline__ uint4 ld_stream(const void *p) {     // read once: past L1
+// A piece of W, read once: past L1.  FIXED: nothing writes it as long as the kernel lives, as the non-coherent load wants it.  A
+// kernel that a W's writer may still run beside (Params::wait_first) takes the ordinary load.
+template <bool FIXED>
+static __device__ __forceinline__ uint4 ld_stream(const void *p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  if constexpr (FIXED)
+    asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  else
+    asm volatile("ld.global.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
 template <bool F16>
@@ -93,8 +99,8 @@ static __device__ __forceinline__ uint4 gated_act(const ugb_skinny_gate &q, int 
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// KC: chunks of a warp per piece; a unit whose split is longer runs in p.spans pieces.
-template <int KC, bool F16, bool GATE = false>
+// KC: chunks of a warp per piece; a unit whose split is longer runs in p.spans pieces.  FIXED: no kernel of the stream writes W.
+template <int KC, bool F16, bool FIXED, bool GATE = false>
 __global__ void __launch_bounds__(THREADS, 2)
 skinny_gemm_kernel(const Params p) {
   __shared__ float red[2][WARPS][8 * RED_LD];
@@ -140,10 +146,10 @@ skinny_gemm_kernel(const Params p) {
     const int c = lc + i * WARPS, k = c * CHUNK + 8 * t;
     const bool lo = c < lc1 && k < p.k, hi = c < lc1 && k + 32 < p.k;
     const uint4 z = make_uint4(0, 0, 0, 0);
-    w[i][0] = lo ? ld_stream(r0 + 2 * (size_t)k) : z;
-    w[i][1] = lo ? ld_stream(r1 + 2 * (size_t)k) : z;
-    w[i][2] = hi ? ld_stream(r0 + 2 * (size_t)k + 64) : z;
-    w[i][3] = hi ? ld_stream(r1 + 2 * (size_t)k + 64) : z;
+    w[i][0] = lo ? ld_stream<FIXED>(r0 + 2 * (size_t)k) : z;
+    w[i][1] = lo ? ld_stream<FIXED>(r1 + 2 * (size_t)k) : z;
+    w[i][2] = hi ? ld_stream<FIXED>(r0 + 2 * (size_t)k + 64) : z;
+    w[i][3] = hi ? ld_stream<FIXED>(r1 + 2 * (size_t)k + 64) : z;
   };
   if (u < u1) {
     aim(u, 0);
@@ -273,7 +279,7 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
   p.spans = (p.chunks_per_split + kc * WARPS - 1) / (kc * WARPS);
   if (gate) {                              // 16-byte pieces of the table's and the partials' rows, all of k in registers
     if (g.groups || g.f16 || g.batch != 1 || p.splits != 1 || kc != 1 || p.spans != 1 || gate->n_part < 1) return UGB_ERR_UNSUPPORTED;
-    if (((uintptr_t)gate->part | (uintptr_t)gate->table) & 15 || gate->part_stride % 4 != 0 || gate->ld % 4 != 0 || gate->table_ld % 8 != 0 || gate->off % 8 != 0 ||
+    if (!g.b_static || ((uintptr_t)gate->part | (uintptr_t)gate->table) & 15 || gate->part_stride % 4 != 0 || gate->ld % 4 != 0 || gate->table_ld % 8 != 0 || gate->off % 8 != 0 ||
         gate->n % 8 != 0 || (size_t)gate->n != g.k)
       return UGB_ERR_UNSUPPORTED;
     p.gate = *gate;
@@ -298,9 +304,10 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
   }
   cudaError_t e = cudaErrorInvalidValue;
 #define UGB_SKINNY(KC) \
-  e = g.f16 ? ugb_launch(skinny_gemm_kernel<KC, true>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p) \
-            : ugb_launch(skinny_gemm_kernel<KC, false>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p)
-  if (gate) e = ugb_launch(skinny_gemm_kernel<1, false, true>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p);
+  e = g.f16          ? ugb_launch(skinny_gemm_kernel<KC, true, false>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p) \
+      : p.wait_first ? ugb_launch(skinny_gemm_kernel<KC, false, false>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p) \
+                     : ugb_launch(skinny_gemm_kernel<KC, false, true>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p)
+  if (gate) e = ugb_launch(skinny_gemm_kernel<1, false, true, true>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p);
   else switch (kc) { case 1: UGB_SKINNY(1); break; case 2: UGB_SKINNY(2); break; case 3: UGB_SKINNY(3); break; default: UGB_SKINNY(4); }
 #undef UGB_SKINNY
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of skinny_gemm_kernel failed: %s", cudaGetErrorString(e));

@@ -433,7 +433,7 @@ causal_conv_kernel(const T *__restrict__ h, size_t h_ld, const float *__restrict
 // One new position per sequence: one thread per 4 channels, state [rows][ld] in place.
 template <typename T>
 __global__ void __launch_bounds__(128)
-min_gru_step_kernel(const float *__restrict__ pre, int n_part, size_t part_stride, const float *__restrict__ bz,
+min_gru_step_kernel(const float *pre, int n_part, size_t part_stride, const float *__restrict__ bz,
                     const float *__restrict__ bu, float *__restrict__ state, T *__restrict__ out, int ld) {
   const int r = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
   const bool on = c < ld >> 2;
@@ -630,9 +630,9 @@ min_gru_scan_kernel(const TI *__restrict__ pre, const float *__restrict__ bz, co
 // columns per thread (the segments are multiples of 8 wide), U split-K partials in flight.
 template <typename T, int PER, int U>
 __global__ void __launch_bounds__(512)
-latent_inputs_kernel(const float *__restrict__ pre, int n_part, size_t part_stride, const float *__restrict__ q_gain,
+latent_inputs_kernel(const float *pre, int n_part, size_t part_stride, const float *__restrict__ q_gain,
                      const float *__restrict__ c_gain, T *__restrict__ cq, T *__restrict__ cache, float *__restrict__ gate,
-                     const int *__restrict__ pos_p, int pos_off, int t, int t_max, int q_ld, int c_ld, int g_ld,
+                     const int *pos_p, int pos_off, int t, int t_max, int q_ld, int c_ld, int g_ld,
                      float inv_q, float inv_c, float eps, ugb_status_word *status) {
   __shared__ float sm[2][16];
   const int r = blockIdx.x, n = q_ld + c_ld + g_ld, tid = threadIdx.x, bd = blockDim.x;

@@ -70,6 +70,10 @@ template <> __device__ __forceinline__ float from_f32<float>(float v) { return v
 template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
 
+// The kernels below are dependent launches: they are resident while the kernels that write their operands may still run.  So
+// no operand is read through the non-coherent path (__ldg, or const __restrict__), which wants memory that nothing writes as
+// long as the kernel lives; ordinary loads behind the wait see what was written before it.
+
 // ---- fp32 on the FP32 pipe (the reference's default for f32 is CUBLAS_COMPUTE_32F, gemm.rs:87-128: no reduced
 // precision), two shapes -------------------------------------------------------------------------------------
 // (1) Skinny products, m <= 16 rows against a [n, k] operand with k contiguous (Linear::fwd = matmul_t with a
@@ -78,8 +82,7 @@ template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return
 // partial dot products are summed by warp shuffles.
 template <int MR>
 __global__ void __launch_bounds__(256)
-f32_skinny_kernel(float *__restrict__ C, const float *__restrict__ A, const float *__restrict__ B, int m, int n, int k,
-                  long long a_b, long long b_b) {
+f32_skinny_kernel(float *C, const float *A, const float *B, int m, int n, int k, long long a_b, long long b_b) {
   ugb_pdl_trigger();
   ugb_pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -98,7 +101,7 @@ f32_skinny_kernel(float *__restrict__ C, const float *__restrict__ A, const floa
 #pragma unroll
     for (int r = 0; r < MR; ++r) {
       if (r < m) {
-        const float4 x = __ldg(reinterpret_cast<const float4 *>(a + (long long)r * k) + c);
+        const float4 x = reinterpret_cast<const float4 *>(a + (long long)r * k)[c];
         acc[r] = fmaf(x.x, wv.x, fmaf(x.y, wv.y, fmaf(x.z, wv.z, fmaf(x.w, wv.w, acc[r]))));
       }
     }
@@ -118,8 +121,7 @@ f32_skinny_kernel(float *__restrict__ C, const float *__restrict__ A, const floa
 // for 32 heads x [1, 1024] x [1024, 64].)
 template <int MR>
 __global__ void __launch_bounds__(MR <= 2 ? 1024 : (MR <= 4 ? 512 : 256))
-f32_skinny_n_kernel(float *__restrict__ C, const float *__restrict__ A, const float *__restrict__ B, int m, int n, int k,
-                    long long a_rs, long long a_b, long long b_rs, long long b_b) {
+f32_skinny_n_kernel(float *C, const float *A, const float *B, int m, int n, int k, long long a_rs, long long a_b, long long b_rs, long long b_b) {
   constexpr int WARPS = MR <= 2 ? 32 : (MR <= 4 ? 16 : 8);       // 32 KiB of partial sums at most
   __shared__ __align__(16) float red[WARPS][MR][128];
   ugb_pdl_trigger();
@@ -138,7 +140,7 @@ f32_skinny_n_kernel(float *__restrict__ C, const float *__restrict__ A, const fl
 #pragma unroll
       for (int r = 0; r < MR; ++r) {
         if (r < m) {
-          const float x = __ldg(a + (long long)r * a_rs + kk);
+          const float x = a[(long long)r * a_rs + kk];
           acc[r][0] = fmaf(x, bv.x, acc[r][0]); acc[r][1] = fmaf(x, bv.y, acc[r][1]);
           acc[r][2] = fmaf(x, bv.z, acc[r][2]); acc[r][3] = fmaf(x, bv.w, acc[r][3]);
         }
@@ -232,13 +234,13 @@ f32_tile_kernel(const F32Params p) {
       const E *at = src + r * rs + k * ks;
       if constexpr (VEC) {                             // a piece is all in or all out
         if (r < rows && k < k_hi) {
-          const float4 w = __ldg(reinterpret_cast<const float4 *>(at));
+          const float4 w = *reinterpret_cast<const float4 *>(at);
           v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
         }
       } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (kc ? r < rows && k + e < k_hi : r + e < rows && k < k_hi) v[e] = to_f32<E>(__ldg(at + e * (kc ? ks : rs)));
+          if (kc ? r < rows && k + e < k_hi : r + e < rows && k < k_hi) v[e] = to_f32<E>(at[e * (kc ? ks : rs)]);
       }
       reg[i] = make_float4(v[0], v[1], v[2], v[3]);
     }

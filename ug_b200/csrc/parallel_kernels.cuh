@@ -257,7 +257,7 @@ route_kernel(const float *__restrict__ logits, int n_part, int ld, int rows, int
 // One CTA per token row.
 template <typename T>
 __global__ void __launch_bounds__(256)
-expert_rows_kernel(const T *__restrict__ h, const float4 *__restrict__ choice, const int *__restrict__ count, int experts, int top,
+expert_rows_kernel(const T *h, const float4 *choice, const int *count, int experts, int top,
                    int tile, int tiles, T *__restrict__ x, int *__restrict__ slot, int *__restrict__ map, int ld) {
   __shared__ int first[32 * ROUTER_PER_LANE + 1];          // first tile of every expert
   const int r = blockIdx.x, lane = threadIdx.x & 31;
@@ -315,7 +315,7 @@ static __global__ void silu_mul_kernel(const float *__restrict__ gu, float *__re
 // out = sum of n_part f32 partials, rounded to T; n4 groups of four values
 template <typename T>
 __global__ void __launch_bounds__(256)
-sum_partials_kernel(const float *__restrict__ part, int n_part, size_t part_stride, size_t n4, T *__restrict__ out) {
+sum_partials_kernel(const float *part, int n_part, size_t part_stride, size_t n4, T *__restrict__ out) {
   ugb_pdl_wait();
   ugb_pdl_trigger();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -335,7 +335,7 @@ sum_partials_kernel(const float *__restrict__ part, int n_part, size_t part_stri
 // A thread takes 4 columns of a row; n4 = rows * ld / 4.
 template <typename T>
 __global__ void __launch_bounds__(256)
-token_gate_kernel(const float *__restrict__ part, int n_part, size_t part_stride, size_t n4, int ld, int n, const int *__restrict__ tok, int t,
+token_gate_kernel(const float *part, int n_part, size_t part_stride, size_t n4, int ld, int n, const int *tok, int t,
                   int tok_stride, int tok_off, const T *__restrict__ table, size_t table_ld, int off, int vocab, T *__restrict__ out) {
   ugb_pdl_wait();
   ugb_pdl_trigger();

@@ -15,7 +15,8 @@
 //
 // Every kernel is a dependent launch: its CTAs come to the SMs while the last wave of the kernel before still runs and wait
 // there, so that a chain of small operators does not pay a launch between two of them ([1024, 4096] softmax 8.80 -> 7.23 us,
-// [107, 40] 5.5 -> 3.6, [28239, 104] rms_silu 8.7 -> 6.7).
+// [107, 40] 5.5 -> 3.6, [28239, 104] rms_silu 8.7 -> 6.7).  Every input, alpha too, may have been written by a kernel that runs
+// while this one is already resident: ordinary loads behind the wait, not the non-coherent ones of __ldg.
 #include <cfloat>
 
 #include "ugb_internal.h"
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(THREADS) row_reg_kernel(RowArgs a) {
       for (int i = 0; i < VPT; ++i) {
         const int c = lane + i * LANES;
         if (c < nvec) {
-          const float4 w = __ldg(al + c);
+          const float4 w = al[c];
           float4 o;
           if constexpr (OP == OP_RMS_SILU) {
             // x / m * w * g / (1 + exp(-g)) with one division per element: (x w g) / (m (1 + exp(-g))).

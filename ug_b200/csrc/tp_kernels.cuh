@@ -175,7 +175,7 @@ tp_reduce_rmsnorm_kernel(float *__restrict__ x, TpPeers tp, int n_part, size_t p
 // Vocab-parallel greedy choice.  Stage 1 (per rank): best (value, global id) of the rank's logit
 // slice for every row -> pairs[b] in the rank's own exchange block.  One CTA of 1024 threads per row.
 static __global__ void __launch_bounds__(1024)
-tp_argmax_local_kernel(const float *__restrict__ logits, int vocab_local, int vocab_offset, float2 *__restrict__ pairs) {
+tp_argmax_local_kernel(const float *logits, int vocab_local, int vocab_offset, float2 *__restrict__ pairs) {
   __shared__ float sv[32];
   __shared__ int si[32];
   ugb_pdl_trigger();

@@ -129,6 +129,9 @@ static inline int32_t ugb_check_slice(ugb_device *dev, const ugb_slice *s, int32
 // kernel writes) overlaps the predecessor's tail.  ugb_pdl_trigger() lets the
 // NEXT kernel on the stream begin its own preamble.  Both are no-ops in a
 // kernel launched the ordinary way.
+// Such a kernel lives while its inputs may still be written, so only weights
+// and tables may go through the non-coherent path (__ldg, ld.global.nc, or a
+// const __restrict__ parameter, which the compiler loads the same way).
 #ifdef __CUDACC__
 __device__ __forceinline__ void ugb_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void ugb_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
