@@ -73,6 +73,13 @@ template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return
 // The kernels below are dependent launches: they are resident while the kernels that write their operands may still run.  So
 // no operand is read through the non-coherent path (__ldg, or const __restrict__), which wants memory that nothing writes as
 // long as the kernel lives; ordinary loads behind the wait see what was written before it.
+// The 16-byte ones are written out: the compiler's own sink to their uses, one behind the other ([12, 8192] x [64, 8192]^T
+// 122 us so, 54 with all in flight).  Single values of a guarded piece are left to it (written out, twice the time).
+__device__ __forceinline__ float4 ld_global(const float4 *p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
 
 // ---- fp32 on the FP32 pipe (the reference's default for f32 is CUBLAS_COMPUTE_32F, gemm.rs:87-128: no reduced
 // precision), two shapes -------------------------------------------------------------------------------------
@@ -101,7 +108,7 @@ f32_skinny_kernel(float *C, const float *A, const float *B, int m, int n, int k,
 #pragma unroll
     for (int r = 0; r < MR; ++r) {
       if (r < m) {
-        const float4 x = reinterpret_cast<const float4 *>(a + (long long)r * k)[c];
+        const float4 x = ld_global(reinterpret_cast<const float4 *>(a + (long long)r * k) + c);
         acc[r] = fmaf(x.x, wv.x, fmaf(x.y, wv.y, fmaf(x.z, wv.z, fmaf(x.w, wv.w, acc[r]))));
       }
     }
@@ -234,7 +241,7 @@ f32_tile_kernel(const F32Params p) {
       const E *at = src + r * rs + k * ks;
       if constexpr (VEC) {                             // a piece is all in or all out
         if (r < rows && k < k_hi) {
-          const float4 w = *reinterpret_cast<const float4 *>(at);
+          const float4 w = ld_global(reinterpret_cast<const float4 *>(at));
           v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
         }
       } else {
