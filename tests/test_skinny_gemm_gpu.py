@@ -18,7 +18,9 @@ def _wide(b, f16):
 
 @pytest.mark.parametrize("f16", [False, True])
 @pytest.mark.parametrize("m", [1, 2, 7, 8, 9])
-@pytest.mark.parametrize("n,k", [(1, 8), (15, 64), (16, 72), (17, 520), (33, 2048), (200, 2056), (3000, 512), (48, 5632), (40, 8200)])
+@pytest.mark.parametrize("n,k", [(1, 8), (15, 64), (16, 72), (17, 520), (33, 2048), (200, 2056), (3000, 512), (48, 5632), (40, 8200),
+                                 # more than a piece for every CTA of a 148-SM device: by k and alignment on three kernels
+                                 (3152, 64), (3168, 64), (3168, 1016), (3168, 1024), (3161, 72), (3161, 136), (8191, 8)])
 def test_rows_against_nk(dev, m, n, k, f16):
     a, w = synth.normal(11 + m, (m, k), 0.5), synth.normal(12 + n, (n, k), 0.5)
     ab, wb = _bits(a, f16), _bits(w, f16)
@@ -37,8 +39,8 @@ def test_rows_against_nk(dev, m, n, k, f16):
 
 
 @pytest.mark.parametrize("b,m,shared", [(3, 4, False), (2, 8, False), (2, 4, True), (3, 3, True)])
-def test_batches(dev, b, m, shared):
-    n, k = 72, 328
+@pytest.mark.parametrize("n,k", [(72, 328), (1600, 64), (1601, 136)])
+def test_batches(dev, b, m, shared, n, k):
     a, w = synth.to_bf16_bits(synth.normal(3, (b, m, k), 0.5)), synth.to_bf16_bits(synth.normal(4, (1 if shared else b, n, k), 0.5))
     from ug_b200 import DType
     out = dev.allocate_uninit(DType.BF16, b * m * n)

@@ -228,6 +228,10 @@ skinny_gemm_kernel(const Params p) {
   }
 }
 
+// One CTA per SM leaves the registers for the next kernel's first weights; up to a third more CTAs than SMs, so that every
+// CTA has the same number of units (their loads share the bandwidth, not an SM).  Live groups are known on the device only.
+long long most_ctas(int sm_count, bool groups) { return groups ? (long long)sm_count * 2 : (long long)sm_count * 4 / 3; }
+
 int chunks_of(size_t k) { return (int)((k + CHUNK - 1) / CHUNK); }
 
 }  // namespace
@@ -238,6 +242,8 @@ int ugb_skinny_effective_splits(size_t k, int splits) {
   const int per = (chunks + splits - 1) / splits;
   return (chunks + per - 1) / per;
 }
+
+bool ugb_skinny_one_round(int sm_count, size_t n, size_t batch) { return (n + TILE_N - 1) / TILE_N * batch <= (size_t)most_ctas(sm_count, false); }
 
 int ugb_skinny_splits(int sm_count, size_t n, size_t k) {
   const int chunks = chunks_of(k), tiles = (int)((n + TILE_N - 1) / TILE_N);
@@ -292,9 +298,7 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
   const long long units = (long long)p.tiles * (g.groups ? p.n_groups_tiles : (long long)p.splits * (long long)g.batch);
   if (units > (1ll << 30)) return UGB_ERR_UNSUPPORTED;
   p.units = (int)units;
-  // One CTA per SM leaves the registers for the next kernel's first weights; up to a third more CTAs than SMs, so that every
-  // CTA has the same number of units (their loads share the bandwidth, not an SM).  Live groups are known on the device only.
-  const long long most = g.groups ? (long long)dev->sm_count * 2 : (long long)dev->sm_count * 4 / 3;
+  const long long most = most_ctas(dev->sm_count, g.groups != nullptr);
   const long long rounds = (units + most - 1) / most;
   const unsigned grid = (unsigned)((units + rounds - 1) / rounds);
   if (g.query_grid || g.query_ctas_per_sm) {

@@ -10,6 +10,9 @@ constexpr int UGB_SKINNY_SPLITS = 8;     // most partials it writes
 // the registers beside the weights in flight (with half of those in flight 16 rows took 1.22 ms a step against 1.16).
 inline bool ugb_skinny_rows(size_t rows) { return rows >= 1 && rows <= (size_t)UGB_SKINNY_ROWS; }
 
+// Whether every CTA has one piece (16 rows of W) of an unsplit product at most.
+bool ugb_skinny_one_round(int sm_count, size_t n, size_t batch);
+
 // k splits of a product with a f32 result that the consumer sums: 2048 inputs or fewer each, more where the columns alone do
 // not fill the SMs.
 int ugb_skinny_splits(int sm_count, size_t n, size_t k);

@@ -74,7 +74,8 @@ template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return
 // no operand is read through the non-coherent path (__ldg, or const __restrict__), which wants memory that nothing writes as
 // long as the kernel lives; ordinary loads behind the wait see what was written before it.
 // The 16-byte ones are written out: the compiler's own sink to their uses, one behind the other ([12, 8192] x [64, 8192]^T
-// 122 us so, 54 with all in flight).  Single values of a guarded piece are left to it (written out, twice the time).
+// 122 us so, 58 with all in flight).  Single values of a guarded piece are left to it (64 times [1339, 597] x [597, 19] in bf16
+// 506 us so, 931 written out).
 __device__ __forceinline__ float4 ld_global(const float4 *p) {
   float4 v;
   asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
@@ -557,14 +558,24 @@ int32_t ugb_matmul(ugb_device *dev, ugb_slice *dst, const ugb_slice *lhs, const 
   const char *rp = (const char *)rhs->ptr + rhs_off * es;
 
   // Few rows against [n, k] rows: the kernel that streams the matrix through registers, whatever n (it reads every step of a
-  // batch that shares its matrix again, so those go on as one tall product).
-  if ((dt == UGB_BF16 || dt == UGB_F16) && !L.transposed && R.transposed && ugb_skinny_rows(R.batch == 0 ? b * m : m)) {
+  // batch that shares its matrix again, so those go on as one tall product).  Its CTAs take about 1.5 us for each 16 columns
+  // however short k is.  Where they have one piece each it is ahead of the tensor-core tiles for every k ([4, 64] x [2048, 64]^T 3.4
+  // us against 3.7, k = 2048 4.7 against 9.6), with more of them from about k = 1024 on ([4, k] x [65536, k]^T for k = 64, 512, 1024,
+  // 2048: 31, 31, 32, 47 us against 9.5, 20, 36, 70; 8 times [4, k] x [2048, k]^T 11, 11, 11, 16 against 5, 8, 11, 18).  Columns or
+  // bases that those tiles do not take are still better off here than on the FFMA kernel from about k = 128 on ([65536, k]: 31
+  // us against 8, 19, 31, 57 for k = 8, 64, 128, 256).
+  const bool few = (dt == UGB_BF16 || dt == UGB_F16) && !L.transposed && R.transposed && ugb_skinny_rows(R.batch == 0 ? b * m : m);
+  auto stream_rows = [&]() {
     ugb_tc_gemm_args g;
     g.out = dst->ptr; g.a = lp; g.b = rp;
     g.batch = b; g.m = m; g.n = n; g.k = k;
     g.a_batch = L.batch; g.b_batch = R.batch; g.b_is_nk = true; g.f16 = dt == UGB_F16;
     g.epi = UGB_EPI_BF16; g.splits = 1; g.bn = 0; g.b_static = false; g.pdl = true;
-    const int32_t src = ugb_skinny_gemm(dev, g);
+    return ugb_skinny_gemm(dev, g);
+  };
+  const bool stream = few && (k >= 1024 || ugb_skinny_one_round(dev->sm_count, n, R.batch == 0 ? 1 : b));
+  if (stream) {
+    const int32_t src = stream_rows();
     if (src != UGB_ERR_UNSUPPORTED) return src;
   }
   // Few results of a short k finish on the FFMA kernel before a tensor-core tile is set up ([1, 3, 1616] x [1616, 328]: 28 us there).
@@ -574,6 +585,10 @@ int32_t ugb_matmul(ugb_device *dev, ugb_slice *dst, const ugb_slice *lhs, const 
     // [n,k] row-major ("TN", matmul_t with a weight) or [k,n] row-major ("NN").
     int32_t trc = ugb_tc_gemm_bf16(dev, dst->ptr, lp, rp, b, m, n, k, L.batch, R.batch, R.transposed, dt == UGB_F16);
     if (trc != UGB_ERR_UNSUPPORTED) return trc;
+  }
+  if (few && !stream && k >= 128) {
+    const int32_t src = stream_rows();
+    if (src != UGB_ERR_UNSUPPORTED) return src;
   }
   switch (dt) {
     case UGB_F32: return launch_f32(dev, (float *)dst->ptr, (const float *)lp, (const float *)rp, b, m, n, k, L, R);
