@@ -578,8 +578,11 @@ int32_t ugb_matmul(ugb_device *dev, ugb_slice *dst, const ugb_slice *lhs, const 
     const int32_t src = stream_rows();
     if (src != UGB_ERR_UNSUPPORTED) return src;
   }
-  // Few results of a short k finish on the FFMA kernel before a tensor-core tile is set up ([1, 3, 1616] x [1616, 328]: 28 us there).
-  if ((dt == UGB_BF16 || dt == UGB_F16) && !L.transposed && (m * n >= 128 * 64 || k >= 256)) {
+  // Whatever has the alignment is faster on the tensor cores, also the smallest: [1, 8] x [8, 8] 3.5 us against 4.2 on the FFMA kernel, [1, 32] x
+  // [32, 8] 3.5 against 5.6, [9, 192] x [64, 192]^T 4.1 against 11.1, [100, 64] x [64, 64]^T 4.2 against 8.1, 64 of [64, 128] x [64, 128]^T
+  // 4.0 against 16.3.  Only long rows of results with next to nothing to sum are not ([8, 8] x [65536, 8]^T 16.6 against 9.1; with k = 32 9.7
+  // against 12.1).
+  if ((dt == UGB_BF16 || dt == UGB_F16) && !L.transposed && !(few && !stream && k <= 16)) {
     // tensor-core path (bf16 and f16 are the same tcgen05.mma.kind::f16 instruction with another format field, as
     // both go to cublasGemmStridedBatchedEx in the reference, gemm.rs:130-232): A [m,k] row-major, B either
     // [n,k] row-major ("TN", matmul_t with a weight) or [k,n] row-major ("NN").
