@@ -215,7 +215,8 @@ __device__ __forceinline__ float2 halves(uint64_t v) {
   return r;
 }
 
-template <typename E, int WM, int WK, bool VEC>
+// TURNED: the product's rows are the tile's columns, C^T = B^T A^T.
+template <typename E, int WM, int WK, bool VEC, bool TURNED>
 __global__ void __launch_bounds__(128, 2)
 f32_tile_kernel(const F32Params p) {
   using T = F32Tile<WM, WK>;
@@ -326,14 +327,14 @@ f32_tile_kernel(const F32Params p) {
   auto store = [&](int row, int col, float4 v) {       // row, col inside the tile
     const int gi = m0 + row, gj = n0 + col;
     if (gi >= p.m) return;
-    E *at = C + gi * p.c_rs + gj;
-    if (VEC && gj + 3 < p.n) {
+    E *at = TURNED ? C + gj * p.c_rs + gi : C + gi * p.c_rs + gj;
+    if (VEC && !TURNED && gj + 3 < p.n) {
       if constexpr (VEC) *reinterpret_cast<float4 *>(at) = v;
     } else {
       const float w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        if (gj + e < p.n) at[e] = from_f32<E>(w[e]);
+        if (gj + e < p.n) at[TURNED ? e * p.c_rs : e] = from_f32<E>(w[e]);
     }
   };
   const bool alone = WK == 1 && p.split == 1;
@@ -376,32 +377,36 @@ inline bool al16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 // Warps over rows and over a slice's k, and CTAs along k, for a product on f32_tile_kernel: the least time of the fullest SM.
 // In SM cycles, fitted to 49 timed combinations of eight products of 40-2048 rows (off by 4 % on average): the share of the FMA
 // pipe that one CTA on an SM or several reach, what the k split inside a CTA costs of it, and what a CTA spends besides.
-struct F32Shape { int wm, wk, split; };
+// Turned: columns that leave most of a 128-wide tile empty are the rows of a 32- or 64-row tile instead; the results are then
+// stored one by one, about SCATTER cycles per 32 rows of a tile (64 times [1339, 597] x [597, 19] in bf16 506 us as it lies, 303 turned).
+struct F32Shape { int wm, wk, split; double cost; bool turned; };
 F32Shape f32_shape(int sm_count, size_t b, size_t m, size_t n, size_t k) {
-  constexpr double ONE = 0.62, SEVERAL = 0.75, SHARE[] = {1.0, 0.85, 0.72}, CTA = 1300, REDUCE = 2600, RANK = 400;
-  F32Shape best{4, 1, 1};
-  double least = 0;
-  for (int i = 0; i < 3; ++i) {
+  constexpr double ONE = 0.62, SEVERAL = 0.75, SHARE[] = {1.0, 0.85, 0.72}, CTA = 1300, REDUCE = 2600, RANK = 400, SCATTER = 4000;
+  F32Shape best{4, 1, 1, 0, false};
+  auto consider = [&](int i, bool turned) {
     const int wm = 4 >> i, wk = 1 << i;
-    const size_t rows = (m + 32 * wm - 1) / (32 * wm), tiles = rows * ((n + 127) / 128) * b;
-    if (rows > 65535) continue;
+    const size_t rows = ((turned ? n : m) + 32 * wm - 1) / (32 * wm), tiles = rows * (((turned ? m : n) + 127) / 128) * b;
+    if (rows > 65535) return;
     for (int split = 1; split == 1 || (split <= 8 && k / split >= 64); split *= 2) {
       const double ctas = (double)((tiles * split + sm_count - 1) / sm_count);
       const double mma = 32.0 * wm * ((k + split - 1) / split) / (SHARE[i] * (ctas < 2 ? ONE : SEVERAL));
-      const double cost = ctas * (mma + CTA + (wk * split > 1 ? REDUCE : 0) + (split > 1 ? RANK * split : 0));
-      if (least == 0 || cost < least) { least = cost; best = {wm, wk, split}; }
+      const double cost = ctas * (mma + CTA + (wk * split > 1 ? REDUCE : 0) + (split > 1 ? RANK * split : 0) + (turned ? SCATTER * wm / split : 0));
+      if (best.cost == 0 || cost < best.cost) best = {wm, wk, split, cost, turned};
     }
-  }
+  };
+  for (int i = 0; i < 3; ++i) consider(i, false);
+  if (n <= 64 && n < m)
+    for (int i = 1; i < 3; ++i) consider(i, true);
   return best;
 }
 
-template <typename E, int WM, int WK, bool VEC>
+template <typename E, int WM, int WK, bool VEC, bool TURNED = false>
 int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b) {
   using T = F32Tile<WM, WK>;
   const dim3 grid((unsigned)((p.n + T::BN - 1) / T::BN * p.split), (unsigned)((p.m + T::BM - 1) / T::BM), (unsigned)b);
   const size_t smem = WK * p.split > 1 ? std::max(T::SMEM, T::SMEM_REDUCE) : T::SMEM;
-  if (smem > 48 * 1024) UGB_CUDA(dev, cudaFuncSetAttribute(f32_tile_kernel<E, WM, WK, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const cudaError_t e = ugb_launch_cluster(f32_tile_kernel<E, WM, WK, VEC>, grid, dim3(T::THREADS), smem, dev->stream, true, p.split, p);
+  if (smem > 48 * 1024) UGB_CUDA(dev, cudaFuncSetAttribute(f32_tile_kernel<E, WM, WK, VEC, TURNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const cudaError_t e = ugb_launch_cluster(f32_tile_kernel<E, WM, WK, VEC, TURNED>, grid, dim3(T::THREADS), smem, dev->stream, true, p.split, p);
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of f32_tile_kernel failed: %s", cudaGetErrorString(e));
   return ugb_after_launch(dev, "f32_tile_kernel");
 }
@@ -412,6 +417,14 @@ int32_t launch_f32_tile(ugb_device *dev, F32Params p, size_t b) {
   UGB_REQUIRE(dev, b <= 65535 && ((size_t)p.m + 127) / 128 <= 65535, UGB_ERR_UNSUPPORTED, "matmul: m or batch too large for the FP32-pipe kernel");
   p.split = s.split;
   p.k_per_split = (int)((((size_t)p.k + s.split - 1) / s.split + 15) / 16 * 16);
+  if (s.turned) {
+    std::swap(p.m, p.n);
+    std::swap(p.a, p.b);
+    std::swap(p.a_b, p.b_b);
+    std::swap(p.a_rs, p.b_cs);
+    std::swap(p.a_cs, p.b_rs);
+    return s.wk == 4 ? launch_f32_shape<E, 1, 4, VEC, true>(dev, p, b) : launch_f32_shape<E, 2, 2, VEC, true>(dev, p, b);
+  }
   if (s.wk == 4) return launch_f32_shape<E, 1, 4, VEC>(dev, p, b);
   if (s.wk == 2) return launch_f32_shape<E, 2, 2, VEC>(dev, p, b);
   return launch_f32_shape<E, 4, 1, VEC>(dev, p, b);
