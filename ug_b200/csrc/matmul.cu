@@ -279,6 +279,14 @@ f32_tile_kernel(const F32Params p) {
   };
 
   const int wk = warp % WK, wm = warp / WK;
+  // Halves of this warp's part of a slice that hold anything.  The guarded reads of !VEC lose more by a bound that varies than
+  // they gain ([65536, 63] x [63, 63]^T 37.4 -> 39.8 us); the others gain where k is short ([3694, 8] x [15392, 8]^T 58.8 -> 51.7,
+  // 64 times [595, 8] x [8, 344] 18.5 -> 15.5).
+  const bool live = m0 + wm * 32 < p.m;
+  auto halves_of = [&](int k0) {
+    constexpr int HALF = BK / WK / 2;
+    return !VEC ? 2 : !live ? 0 : min(2, (k_hi - k0 - wk * 2 * HALF + HALF - 1) / HALF);
+  };
   const int ty = lane >> 3, tx = lane & 7;
   uint64_t acc[8][8];                                  // columns in pairs
 #pragma unroll
@@ -296,7 +304,7 @@ f32_tile_kernel(const F32Params p) {
     if (more) fetch_both(k0 + BK);
     const float *as = smem + buf * T::STAGE, *bs = as + BK * BM;
 #pragma unroll 1
-    for (int h = 0; h < 2; ++h)                        // rolled, or the compiler moves the global reads down to their use
+    for (int h = 0; h < halves_of(k0); ++h)               // rolled, or the compiler moves the global reads down to their use
 #pragma unroll
     for (int j = 0; j < BK / WK / 2; ++j) {
       const int kk = wk * (BK / WK) + h * (BK / WK / 2) + j, x = (kk >> 2) * SW;
