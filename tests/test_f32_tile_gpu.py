@@ -6,6 +6,7 @@ import pytest
 from ug_b200 import DType, synth
 
 pytestmark = pytest.mark.gpu
+TURNED = [(20000, 17, 64), (8193, 8, 512), (3000, 5, 1999), (2600, 36, 1000), (5000, 64, 300), (1301, 33, 597)]   # few columns: the rows of the tile
 
 
 def _check(dev, b, m, n, k, a_km, b_kn, shared=False):
@@ -26,9 +27,7 @@ def _check(dev, b, m, n, k, a_km, b_kn, shared=False):
 @pytest.mark.parametrize("a_km", [False, True])
 @pytest.mark.parametrize("b_kn", [False, True])
 @pytest.mark.parametrize("m,n,k", [(17, 4, 4), (32, 128, 16), (33, 132, 20), (64, 260, 128), (100, 512, 1030), (129, 127, 129), (257, 640, 2048),
-                                   (31, 33, 35), (1, 338, 6045), (600, 1280, 96),
-                                   # few columns: they are the tile's rows
-                                   (20000, 17, 64), (8193, 8, 512), (3000, 5, 1999), (2600, 36, 1000), (5000, 64, 300), (1301, 33, 597)])
+                                   (31, 33, 35), (1, 338, 6045), (600, 1280, 96)] + TURNED)
 def test_layouts(dev, m, n, k, a_km, b_kn):
     _check(dev, 1, m, n, k, a_km, b_kn)
 

@@ -33,7 +33,7 @@ def test_rows_against_nk(dev, m, n, k, f16):
     assert np.all(got[m * n:] == 3.0)
     wa, ww = _wide(ab, f16), _wide(wb, f16)
     want = wa @ ww.T
-    # one rounding of the result (half a unit: 2^-9 bf16, 2^-12 f16) plus f32 sums of k products: k 2^-24 of the sum of magnitudes
+    # one rounding of the result (to nearest: at most 2^-8 of it in bf16, 2^-11 in f16) plus f32 sums of k products: k 2^-24 of the sum of magnitudes
     bound = np.abs(want) * 2.0 ** (-11 if f16 else -8) + (np.abs(wa) @ np.abs(ww).T) * k * 2.0 ** -24 + 1e-6
     assert np.all(np.abs(got[:m * n].reshape(m, n) - want) <= bound)
 

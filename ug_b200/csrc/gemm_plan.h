@@ -1,0 +1,78 @@
+// Which shape a product runs on: host arithmetic only, by predicted time.
+#pragma once
+#include <algorithm>
+#include <cstddef>
+
+// ---- tcgen05 kernel (gemm_tcgen05.cu) -------------------------------------------------------------------------------
+constexpr int UGB_TC_BK = 64;              // k elements of a block: one 128-byte swizzle row of 16-bit values
+
+// Number of partials ugb_tc_gemm writes for a requested split factor.
+inline int ugb_tc_gemm_effective_splits(size_t k, int splits) {
+  const int k_blocks = (int)((k + UGB_TC_BK - 1) / UGB_TC_BK);
+  if (splits < 1) splits = 1;
+  if (splits > k_blocks) splits = k_blocks;
+  const int per = (k_blocks + splits - 1) / splits;
+  return (k_blocks + per - 1) / per;
+}
+
+// Tile shape for more than 64 rows: width, 256-row tiles on pairs of CTAs, and a k split where the caller takes f32 partials
+// (max_splits > 1; the pair shapes do not split).  `pairs`: pairs may be chosen at all.
+struct ugb_tc_plan { int bn = 0, splits = 1; bool pair = false; };
+
+// Time of a product, in us: a launch and its epilogue, and for every round of tiles its k blocks at the pace that a tile of this
+// shape keeps, which falls as more SMs are at work (L2, and the clock under the power limit).  Fitted to 36 timed products of
+// 100-4096 rows, bf16, [n, k] weights; the choice was within 4 % of the best shape on 34 of them.  What it replaced took
+// 256 x 256 pairs above 128 rows and 128 x 64 below: [777, 2048] x [2560, 2048]^T 21.3 -> 16.5 us, x [2048, 2048]^T 19.9 -> 15.0,
+// x [11264, 2048]^T 45.9 -> 39.3, [777, 5632] x [2048, 5632]^T 36.3 -> 27.8, from 2048 rows on mostly as before.
+inline ugb_tc_plan ugb_tc_gemm_plan(int sm_count, size_t batch, size_t m, size_t n, size_t k, bool b_is_nk, bool pairs, int max_splits) {
+  static const struct { int bn; bool pair; float pace, crowd, fixed; } shapes[] = {
+      {256, true, .269f, .097f, 10.4f}, {192, true, .211f, .066f, 9.7f}, {128, true, .210f, .023f, 8.4f}, {256, false, .360f, .071f, 9.0f},
+      {192, false, .255f, .058f, 8.4f}, {128, false, .212f, .032f, 7.7f}, {64, false, .186f, .008f, 7.8f}};
+  const size_t k_blocks = (k + UGB_TC_BK - 1) / UGB_TC_BK;
+  ugb_tc_plan best;
+  float least = 0.f;
+  for (const auto &s : shapes) {
+    if (s.pair && (!pairs || m <= 128 || sm_count < 2)) continue;
+    if (s.pair && s.bn == 192 && !b_is_nk) continue;                   // n-major B is boxed in 64-column pieces
+    const size_t rows = s.pair ? 256 : 128, slots = s.pair ? sm_count / 2 : sm_count;
+    const size_t tiles = (m + rows - 1) / rows * ((n + s.bn - 1) / s.bn) * batch;
+    for (int want = 1; want <= (s.pair ? 1 : max_splits); ++want) {
+      const int splits = ugb_tc_gemm_effective_splits(k, want);
+      if (splits != want) continue;
+      const size_t work = tiles * splits, rounds = (work + slots - 1) / slots;
+      const float busy = work < slots ? (float)work / slots : 1.f;
+      float t = s.fixed + (rounds - 1) + rounds * ((k_blocks + splits - 1) / splits) * (s.pace + s.crowd * busy);
+      t += (splits - 1) * (float)(m * n) * 8e-6f / 3.f;                // each further partial is written and read, about 3 TB/s
+      if (s.bn == 256 && s.pair) t *= 0.95f;                           // the shape that everything large runs on: only for a clear gain
+      if (least == 0.f || t < least) { least = t; best.bn = s.bn; best.splits = splits; best.pair = s.pair; }
+    }
+  }
+  return best;
+}
+
+// ---- FFMA kernel (matmul.cu) ------------------------------------------------------------------------------------------
+// Warps over rows and over a slice's k, and CTAs along k, for a product on f32_tile_kernel: the least time of the fullest SM.
+// In SM cycles, fitted to 49 timed combinations of eight products of 40-2048 rows (off by 4 % on average): the share of the FMA
+// pipe that one CTA on an SM or several reach, what the k split inside a CTA costs of it, and what a CTA spends besides.
+// Turned: columns that leave most of a 128-wide tile empty are the rows of a 32- or 64-row tile instead; the results are then
+// stored one by one, about SCATTER cycles per 32 rows of a tile (64 times [1339, 597] x [597, 19] in bf16 506 us as it lies, 303 turned).
+struct ugb_f32_shape { int wm, wk, split; double cost; bool turned; };
+inline ugb_f32_shape ugb_f32_gemm_shape(int sm_count, size_t b, size_t m, size_t n, size_t k) {
+  constexpr double ONE = 0.62, SEVERAL = 0.75, SHARE[] = {1.0, 0.85, 0.72}, CTA = 1300, REDUCE = 2600, RANK = 400, SCATTER = 4000;
+  ugb_f32_shape best{4, 1, 1, 0, false};
+  auto consider = [&](int i, bool turned) {
+    const int wm = 4 >> i, wk = 1 << i;
+    const size_t rows = ((turned ? n : m) + 32 * wm - 1) / (32 * wm), tiles = rows * (((turned ? m : n) + 127) / 128) * b;
+    if (rows > 65535) return;
+    for (int split = 1; split == 1 || (split <= 8 && k / split >= 64); split *= 2) {
+      const double ctas = (double)((tiles * split + sm_count - 1) / sm_count);
+      const double mma = 32.0 * wm * ((k + split - 1) / split) / (SHARE[i] * (ctas < 2 ? ONE : SEVERAL));
+      const double cost = ctas * (mma + CTA + (wk * split > 1 ? REDUCE : 0) + (split > 1 ? RANK * split : 0) + (turned ? SCATTER * wm / split : 0));
+      if (best.cost == 0 || cost < best.cost) best = {wm, wk, split, cost, turned};
+    }
+  };
+  for (int i = 0; i < 3; ++i) consider(i, false);
+  if (n <= 64 && n < m)
+    for (int i = 1; i < 3; ++i) consider(i, true);
+  return best;
+}

@@ -36,7 +36,7 @@
 
 namespace {
 
-constexpr int BK = 64;
+constexpr int BK = UGB_TC_BK;
 constexpr int ACC_STAGES = 2;
 constexpr int THREADS = 192;
 
@@ -44,8 +44,8 @@ constexpr int THREADS = 192;
 // BM = 64 when m <= 64 (decode: the activation tile is half the size, so the
 // shared-memory ring holds more stages and more weight bytes are in flight per
 // SM; the 64 accumulator rows then sit on 16 lanes of each TMEM lane quadrant).
-// BN = 256 for compute-bound products, 64 / 128 for weight streaming.  The ring
-// takes as many stages as fit in 220 KiB (at most 12).
+// BN by predicted time for tall products (ugb_tc_gemm_plan), 64 to 160 for weight
+// streaming.  The ring takes as many stages as fit in 220 KiB (at most 12).
 // PAIR: two CTAs of a cluster work on one 256 x BN tile (tcgen05 cta_group::2): each stages its own 128
 // rows of A and its own half of B's n range, so a CTA's ring stage is BM x 64 of A plus BN/2 x 64 of B.
 template <int BM, int BN, bool PAIR = false> struct Cfg {
@@ -781,45 +781,6 @@ int32_t ugb_tc_encode_bf16(ugb_device *dev, CUtensorMap *map, const void *base, 
   return UGB_OK;
 }
 
-int ugb_tc_gemm_effective_splits(size_t k, int splits) {
-  const int k_blocks = (int)((k + BK - 1) / BK);
-  if (splits < 1) splits = 1;
-  if (splits > k_blocks) splits = k_blocks;
-  const int per = (k_blocks + splits - 1) / splits;
-  return (k_blocks + per - 1) / per;
-}
-
-// Time of a product, in us: a launch and its epilogue, and for every round of tiles its k blocks at the pace that a tile of this
-// shape keeps, which falls as more SMs are at work (L2, and the clock under the power limit).  Fitted to 36 timed products of
-// 100-4096 rows, bf16, [n, k] weights; the choice was within 4 % of the best shape on 34 of them.  What it replaced took
-// 256 x 256 pairs above 128 rows and 128 x 64 below: [777, 2048] x [2560, 2048]^T 21.3 -> 16.5 us, x [2048, 2048]^T 19.9 -> 15.0,
-// x [11264, 2048]^T 45.9 -> 39.3, [777, 5632] x [2048, 5632]^T 36.3 -> 27.8, from 2048 rows on mostly as before.
-ugb_tc_plan ugb_tc_gemm_plan(int sm_count, size_t batch, size_t m, size_t n, size_t k, bool b_is_nk, bool pairs, int max_splits) {
-  static const struct { int bn; bool pair; float pace, crowd, fixed; } shapes[] = {
-      {256, true, .269f, .097f, 10.4f}, {192, true, .211f, .066f, 9.7f}, {128, true, .210f, .023f, 8.4f}, {256, false, .360f, .071f, 9.0f},
-      {192, false, .255f, .058f, 8.4f}, {128, false, .212f, .032f, 7.7f}, {64, false, .186f, .008f, 7.8f}};
-  const size_t k_blocks = (k + BK - 1) / BK;
-  ugb_tc_plan best;
-  float least = 0.f;
-  for (const auto &s : shapes) {
-    if (s.pair && (!pairs || m <= 128 || sm_count < 2)) continue;
-    if (s.pair && s.bn == 192 && !b_is_nk) continue;                   // n-major B is boxed in 64-column pieces
-    const size_t rows = s.pair ? 256 : 128, slots = s.pair ? sm_count / 2 : sm_count;
-    const size_t tiles = (m + rows - 1) / rows * ((n + s.bn - 1) / s.bn) * batch;
-    for (int want = 1; want <= (s.pair ? 1 : max_splits); ++want) {
-      const int splits = ugb_tc_gemm_effective_splits(k, want);
-      if (splits != want) continue;
-      const size_t work = tiles * splits, rounds = (work + slots - 1) / slots;
-      const float busy = work < slots ? (float)work / slots : 1.f;
-      float t = s.fixed + (rounds - 1) + rounds * ((k_blocks + splits - 1) / splits) * (s.pace + s.crowd * busy);
-      t += (splits - 1) * (float)(m * n) * 8e-6f / 3.f;                // each further partial is written and read, about 3 TB/s
-      if (s.bn == 256 && s.pair) t *= 0.95f;                           // the shape that everything large runs on: only for a clear gain
-      if (least == 0.f || t < least) { least = t; best.bn = s.bn; best.splits = splits; best.pair = s.pair; }
-    }
-  }
-  return best;
-}
-
 int32_t ugb_tc_gemm(ugb_device *dev, const ugb_tc_gemm_args &g) {
   size_t batch = g.batch, m = g.m;
   const size_t n = g.n, k = g.k;
@@ -865,8 +826,8 @@ int32_t ugb_tc_gemm(ugb_device *dev, const ugb_tc_gemm_args &g) {
     if (bn == 160) return launch_tc<64, 160>(dev, st, g, batch, m);
     return launch_tc<64, 256>(dev, st, g, batch, m);
   }
-  if (bn == 80 || bn == 96) bn = 128;                                  // BM = 128 needs n % 16 == 0 tiles: keep the three sizes
-  // CTA pairs: 256 x 256 tiles over two SMs; every SM fetches half as much of B per flop
+  if (bn == 80 || bn == 96) bn = 128;                                  // widths of the 64-row tiles only
+  // CTA pairs: tiles of 256 rows over two SMs; every SM fetches half as much of B per flop
   const bool chosen = plan.bn != 0;
   const bool pair = g.groups ? false : chosen ? plan.pair : g.pair < 0 ? dev->gemm_pair != 0 : g.pair != 0;
   if (pair && m > 128 && g.splits <= 1 && dev->sm_count >= 2) {

@@ -1,5 +1,6 @@
 // Interface of the tcgen05 / TMEM bf16 GEMM translation unit.
 #pragma once
+#include "gemm_plan.h"
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -71,12 +72,6 @@ struct ugb_tc_gemm_args {
 // does not meet the kernel's alignment rules so that the caller can fall back
 // to the FFMA kernel.
 int32_t ugb_tc_gemm(ugb_device *dev, const ugb_tc_gemm_args &args);
-// Tile shape for more than 64 rows: width, 256-row tiles on pairs of CTAs, and a k split where the caller takes f32 partials
-// (max_splits > 1; the pair shapes do not split).  `pairs`: pairs may be chosen at all.
-struct ugb_tc_plan { int bn = 0, splits = 1; bool pair = false; };
-ugb_tc_plan ugb_tc_gemm_plan(int sm_count, size_t batch, size_t m, size_t n, size_t k, bool b_is_nk, bool pairs, int max_splits);
-// Number of partials ugb_tc_gemm writes for a requested split factor.
-int ugb_tc_gemm_effective_splits(size_t k, int splits);
 // C[b, m, n] = A . B with the default epilogue, all three bf16 (f16 = false) or IEEE f16.
 int32_t ugb_tc_gemm_bf16(ugb_device *dev, void *c, const void *a, const void *b_, size_t batch,
                          size_t m, size_t n, size_t k, long long a_batch, long long b_batch,

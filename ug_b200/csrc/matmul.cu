@@ -15,6 +15,7 @@
 
 #include <algorithm>
 
+#include "gemm_plan.h"
 #include "gemm_skinny.cuh"
 #include "gemm_tcgen05.cuh"
 #include "ugb_internal.h"
@@ -382,32 +383,6 @@ f32_tile_kernel(const F32Params p) {
 
 inline bool al16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
-// Warps over rows and over a slice's k, and CTAs along k, for a product on f32_tile_kernel: the least time of the fullest SM.
-// In SM cycles, fitted to 49 timed combinations of eight products of 40-2048 rows (off by 4 % on average): the share of the FMA
-// pipe that one CTA on an SM or several reach, what the k split inside a CTA costs of it, and what a CTA spends besides.
-// Turned: columns that leave most of a 128-wide tile empty are the rows of a 32- or 64-row tile instead; the results are then
-// stored one by one, about SCATTER cycles per 32 rows of a tile (64 times [1339, 597] x [597, 19] in bf16 506 us as it lies, 303 turned).
-struct F32Shape { int wm, wk, split; double cost; bool turned; };
-F32Shape f32_shape(int sm_count, size_t b, size_t m, size_t n, size_t k) {
-  constexpr double ONE = 0.62, SEVERAL = 0.75, SHARE[] = {1.0, 0.85, 0.72}, CTA = 1300, REDUCE = 2600, RANK = 400, SCATTER = 4000;
-  F32Shape best{4, 1, 1, 0, false};
-  auto consider = [&](int i, bool turned) {
-    const int wm = 4 >> i, wk = 1 << i;
-    const size_t rows = ((turned ? n : m) + 32 * wm - 1) / (32 * wm), tiles = rows * (((turned ? m : n) + 127) / 128) * b;
-    if (rows > 65535) return;
-    for (int split = 1; split == 1 || (split <= 8 && k / split >= 64); split *= 2) {
-      const double ctas = (double)((tiles * split + sm_count - 1) / sm_count);
-      const double mma = 32.0 * wm * ((k + split - 1) / split) / (SHARE[i] * (ctas < 2 ? ONE : SEVERAL));
-      const double cost = ctas * (mma + CTA + (wk * split > 1 ? REDUCE : 0) + (split > 1 ? RANK * split : 0) + (turned ? SCATTER * wm / split : 0));
-      if (best.cost == 0 || cost < best.cost) best = {wm, wk, split, cost, turned};
-    }
-  };
-  for (int i = 0; i < 3; ++i) consider(i, false);
-  if (n <= 64 && n < m)
-    for (int i = 1; i < 3; ++i) consider(i, true);
-  return best;
-}
-
 template <typename E, int WM, int WK, bool VEC, bool TURNED = false>
 int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b) {
   using T = F32Tile<WM, WK>;
@@ -421,8 +396,8 @@ int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b) {
 
 template <typename E, bool VEC>
 int32_t launch_f32_tile(ugb_device *dev, F32Params p, size_t b) {
-  const F32Shape s = f32_shape(dev->sm_count, b, p.m, p.n, p.k);
   UGB_REQUIRE(dev, b <= 65535 && ((size_t)p.m + 127) / 128 <= 65535, UGB_ERR_UNSUPPORTED, "matmul: m or batch too large for the FP32-pipe kernel");
+  const ugb_f32_shape s = ugb_f32_gemm_shape(dev->sm_count, b, p.m, p.n, p.k);
   p.split = s.split;
   p.k_per_split = (int)((((size_t)p.k + s.split - 1) / s.split + 15) / 16 * 16);
   if (s.turned) {
