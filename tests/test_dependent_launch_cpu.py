@@ -31,7 +31,7 @@ KERNELS = list(_kernels())
 
 def test_all_kinds_are_seen():
     names = {k[1] for k in KERNELS}
-    assert {"f32_tile_kernel", "f32_skinny_kernel", "f32_skinny_n_kernel", "skinny_gemm_kernel", "tc_gemm_kernel", "row_reg_kernel", "row_general_kernel",
+    assert {"f32_tile_kernel", "f32_skinny_kernel", "f32_skinny_n_kernel", "short_k_kernel", "skinny_gemm_kernel", "tc_gemm_kernel", "row_reg_kernel", "row_general_kernel",
             "row_update_kernel", "reduce_rmsnorm_kernel", "argmax_rows_kernel", "expert_rows_kernel"} <= names
 
 

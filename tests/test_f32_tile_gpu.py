@@ -27,7 +27,9 @@ def _check(dev, b, m, n, k, a_km, b_kn, shared=False):
 @pytest.mark.parametrize("a_km", [False, True])
 @pytest.mark.parametrize("b_kn", [False, True])
 @pytest.mark.parametrize("m,n,k", [(17, 4, 4), (32, 128, 16), (33, 132, 20), (64, 260, 128), (100, 512, 1030), (129, 127, 129), (257, 640, 2048),
-                                   (31, 33, 35), (1, 338, 6045), (600, 1280, 96)] + TURNED)
+                                   (31, 33, 35), (1, 338, 6045), (600, 1280, 96),
+                                   # one slice of k or less: 64 x 64 tiles; and far more results than those are taken for
+                                   (65, 63, 1), (130, 129, 15), (64, 65, 16), (63, 200, 17), (5000, 4000, 6)] + TURNED)
 def test_layouts(dev, m, n, k, a_km, b_kn):
     _check(dev, 1, m, n, k, a_km, b_kn)
 

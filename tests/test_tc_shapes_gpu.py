@@ -40,6 +40,7 @@ def test_shapes(dev, m, n, k, kn):
 @pytest.mark.parametrize("b,m,n,k,kn", [(1, 14, 520, 2048, False), (3, 9, 136, 264, True), (2, 4, 128, 880, True), (1, 1, 9, 7, True), (1, 15, 4096, 520, True),   # few rows
                                         (1, 1, 8, 8, True), (1, 9, 8, 8, False), (2, 24, 64, 192, False), (3, 65, 8, 16, True), (64, 20, 24, 40, False), (1, 8, 8192, 16, False),  # few results
                                         (1, 37, 333, 777, True), (2, 100, 255, 129, False), (1, 130, 129, 1001, False), (1, 3, 8, 2, True),
+                                        (3, 65, 67, 1, True), (1, 200, 129, 15, False), (2, 63, 64, 13, True), (1, 8, 20000, 16, False),   # one slice of k
                                         (1, 20001, 17, 67, True), (2, 1500, 3, 999, False), (1, 2601, 36, 1001, True)])                   # no 16-byte rows
 def test_few_rows_and_odd_sizes(dev, b, m, n, k, kn, f16):
     def bits(x):

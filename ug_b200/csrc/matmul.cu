@@ -381,6 +381,56 @@ f32_tile_kernel(const F32Params p) {
   if (p.split > 1) cluster_barrier();                  // the others have read this CTA's sums
 }
 
+// (3) k of one slice or less: hardly anything to sum, so what counts is how soon the first result leaves.  64 x 64 tiles, 4 x 4 results per
+// thread, everything staged once; eight CTAs to an SM where the kernel above has two.  Its time against that kernel's, k = 1 to 16: bf16 [137, k] x
+// [k, 202] 4.1 us against 7, [1920, k] x [k, 104] 6 against 9, 64 times [24, k] x [k, 4920] 0.66, [3694, k] x [k, 8001] as much; from k = 20 on,
+// with a second slice, it is behind.  f32: 0.6 to 0.95 up to 8 M results, [3694, k] x [k, 8001] 1.4 (as many bytes again to store); where the
+// kernel above moves 16 bytes at a time only [30, 8] x [8, 8] and the like are ahead here (0.65; 64 times [595, 8] x [8, 344] 1.6).
+constexpr int SHORT_K = 16;
+constexpr size_t SHORT_K_F32_RESULTS = 1u << 24, SHORT_K_F32_VEC_RESULTS = 1u << 16;
+
+template <typename E>
+__global__ void __launch_bounds__(256)
+short_k_kernel(const F32Params p) {
+  constexpr int BM = 64, BN = 64;
+  __shared__ float as[SHORT_K][BM + 1], bs[SHORT_K][BN + 1];
+  ugb_pdl_trigger();
+  ugb_pdl_wait();
+  const E *A = (const E *)p.a + (long long)blockIdx.z * p.a_b, *B = (const E *)p.b + (long long)blockIdx.z * p.b_b;
+  E *C = (E *)p.c + (long long)blockIdx.z * p.c_b;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+#pragma unroll
+  for (int e = threadIdx.x; e < BM * SHORT_K; e += 256) {               // along an operand's contiguous direction
+    const int i = p.a_cs == 1 ? e / SHORT_K : e % BM, kk = p.a_cs == 1 ? e % SHORT_K : e / BM;
+    as[kk][i] = m0 + i < p.m && kk < p.k ? to_f32<E>(A[(m0 + i) * p.a_rs + kk * p.a_cs]) : 0.f;
+  }
+#pragma unroll
+  for (int e = threadIdx.x; e < BN * SHORT_K; e += 256) {
+    const int j = p.b_cs == 1 ? e % BN : e / SHORT_K, kk = p.b_cs == 1 ? e / BN : e % SHORT_K;
+    bs[kk][j] = n0 + j < p.n && kk < p.k ? to_f32<E>(B[kk * p.b_rs + (n0 + j) * p.b_cs]) : 0.f;
+  }
+  __syncthreads();
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  float acc[4][4] = {};
+#pragma unroll 4
+  for (int kk = 0; kk < p.k; ++kk) {
+    float a[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) { a[u] = as[kk][ty * 4 + u]; b[u] = bs[kk][tx * 4 + u]; }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int i = m0 + ty * 4 + u, j = n0 + tx * 4 + v;
+      if (i < p.m && j < p.n) C[i * p.c_rs + j] = from_f32<E>(acc[u][v]);
+    }
+}
+
 inline bool al16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
 template <typename E, int WM, int WK, bool VEC, bool TURNED = false>
@@ -397,6 +447,11 @@ int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b) {
 template <typename E, bool VEC>
 int32_t launch_f32_tile(ugb_device *dev, F32Params p, size_t b) {
   UGB_REQUIRE(dev, b <= 65535 && ((size_t)p.m + 127) / 128 <= 65535, UGB_ERR_UNSUPPORTED, "matmul: m or batch too large for the FP32-pipe kernel");
+  if (p.k <= SHORT_K && (p.m + 63) / 64 <= 65535 && (sizeof(E) == 2 || b * (size_t)p.m * (size_t)p.n <= (VEC ? SHORT_K_F32_VEC_RESULTS : SHORT_K_F32_RESULTS))) {
+    const cudaError_t e = ugb_launch(short_k_kernel<E>, dim3((unsigned)((p.n + 63) / 64), (unsigned)((p.m + 63) / 64), (unsigned)b), dim3(256), 0, dev->stream, true, p);
+    if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of short_k_kernel failed: %s", cudaGetErrorString(e));
+    return ugb_after_launch(dev, "short_k_kernel");
+  }
   const ugb_f32_shape s = ugb_f32_gemm_shape(dev->sm_count, b, p.m, p.n, p.k);
   p.split = s.split;
   p.k_per_split = (int)((((size_t)p.k + s.split - 1) / s.split + 15) / 16 * 16);
