@@ -53,3 +53,11 @@ def test_matrix_that_a_kernel_may_write_is_read_coherently():
     for launch in re.findall(r"skinny_gemm_kernel<([^>]*)>", src):
         if launch.split(",")[1].strip() == "true":        # f16: public calls only
             assert launch.split(",")[2].strip() == "false"
+
+
+def test_few_rows_read_ahead_on_late_triggers_only():
+    """A decode step of few rows lets kernels read ahead of their wait whatever its projections run on: no path of gemm_rows may
+    take the late trigger back."""
+    src = open(os.path.join(CSRC, "llama_engine.cu")).read()
+    body = src[src.index("int32_t gemm_rows("):src.index("int32_t gemm(ugb_llama")]
+    assert "late_trigger = true" in body and "late_trigger = false" not in body

@@ -252,15 +252,17 @@ def test_gemm_tile_widths_agree(dev, bn):
     gpu.close()
 
 
-def test_attention_front_end_variants_are_bit_identical(dev):
+@pytest.mark.parametrize("batch", [64, 1, 8])
+def test_attention_front_end_variants_are_bit_identical(dev, batch):
     """Work moved in front of griddepcontrol.wait (the attention kernel's K / V ring, the norm kernel's
     residual row) and the TMA fetch path change when bytes are requested, not what is computed: logits and
     chosen tokens are bit for bit the same.  The early paths switch themselves on only for shapes whose
-    projections cannot be co-resident (the condition under which they are race-free), hence the wide model."""
+    projections cannot be co-resident (the condition under which they are race-free), hence the wide model, and up
+    to eight sequences for all shapes: every projection there lets its successor start only after its own wait."""
     cfg = Config(hidden_size=1536, intermediate_size=4864, max_position_embeddings=256, num_attention_heads=24,
                  num_key_value_heads=4, num_hidden_layers=2, vocab_size=1024)
-    gpu = Model.new(cfg, synth.llama_weights(cfg, 31), dev, 64, 128)
-    prompts = synth.tokens(23, (64, 50), cfg.vocab_size)
+    gpu = Model.new(cfg, synth.llama_weights(cfg, 31), dev, batch, 128)
+    prompts = synth.tokens(23, (batch, 50), cfg.vocab_size)
     results = []
     for early, tma in ((1, 0), (0, 0), (1, 1), (0, 1)):
         gpu.set_option("att_early", early)

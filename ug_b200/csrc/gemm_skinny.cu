@@ -260,7 +260,7 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
     g.batch = 1;
   }
   const size_t rows = g.groups ? (size_t)rows_per_tile : g.m;
-  if (!ugb_skinny_rows(rows) || !g.b_is_nk || g.pair_k || g.n == 0 || g.k == 0 || g.k % 8 != 0) return UGB_ERR_UNSUPPORTED;
+  if (!ugb_skinny_rows(rows) || !g.b_is_nk || g.pair_k || g.query_grid || g.query_ctas_per_sm || g.n == 0 || g.k == 0 || g.k % 8 != 0) return UGB_ERR_UNSUPPORTED;
   if (((uintptr_t)g.a | (uintptr_t)g.b) & 15) return UGB_ERR_UNSUPPORTED;                 // 16-byte loads of both operands
   if (g.a_ld < 0 || g.c_ld < 0 || g.a_ld % 8 != 0 || g.a_batch % 8 != 0 || g.b_batch % 8 != 0 || g.a_batch < 0 || g.b_batch < 0) return UGB_ERR_UNSUPPORTED;
   if (g.epi != UGB_EPI_F32 && g.epi != UGB_EPI_BF16 && g.epi != UGB_EPI_SILU_MUL_BF16 && g.epi != UGB_EPI_RELU2_BF16) return UGB_ERR_UNSUPPORTED;
@@ -301,11 +301,6 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
   const long long most = most_ctas(dev->sm_count, g.groups != nullptr);
   const long long rounds = (units + most - 1) / most;
   const unsigned grid = (unsigned)((units + rounds - 1) / rounds);
-  if (g.query_grid || g.query_ctas_per_sm) {
-    if (g.query_grid) *g.query_grid = (int)grid;
-    if (g.query_ctas_per_sm) *g.query_ctas_per_sm = 2;
-    return UGB_OK;
-  }
   cudaError_t e = cudaErrorInvalidValue;
 #define UGB_SKINNY(KC) \
   e = g.f16          ? ugb_launch(skinny_gemm_kernel<KC, true, false>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p) \

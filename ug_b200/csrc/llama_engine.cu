@@ -147,10 +147,9 @@ int32_t gemm_rows(ugb_llama *m, size_t rows, void *out, const __nv_bfloat16 *a, 
   g.epi = epi; g.splits = splits; g.bn = bn; g.b_static = true; g.pdl = m->pdl != 0;
   g.smem_kib = rows <= 64 ? m->gemm_smem_kib : 0;
   if (skinny(m, rows)) {
-    g.late_trigger = true;              // see early_ok in llama_step
+    g.late_trigger = true;              // whichever kernel takes it: early_ok in llama_step rests on this
     const int32_t rc = ugb_skinny_gemm(m->dev, g);
     if (rc != UGB_ERR_UNSUPPORTED) return rc;
-    g.late_trigger = false;
   }
   if (m->gemm_prof && rows <= 64) {     // qkv, o, gate|up, down, lm_head
     const int kind = epi == UGB_EPI_SILU_MUL_BF16 ? 2 : n == (size_t)m->qkv_dim ? 0 : n == (size_t)m->vl ? 4 : k == (size_t)m->lc.ffn ? 3 : 1;
@@ -431,8 +430,8 @@ int32_t llama_step(ugb_llama *m, const int *tok) {
   // everything before it -- the writer included -- has completed.  Both facts are taken from the launches
   // themselves (the grid each projection gets, the residency the occupancy calculator gives its kernel with
   // its shared memory), not from the tuning options, so a retune that breaks the argument switches this off.
-  // Up to 8 rows the projections let their successor start only after their own wait has returned, and one of them
-  // comes right before every kernel that reads ahead: everything before that projection has completed.
+  // Up to 8 rows the projections let their successor start only after their own wait has returned (gemm_rows asks every kernel
+  // for that), and one of them comes right before every kernel that reads ahead: everything before that projection has completed.
   const int sms = dev->sm_count;
   int c_qkv = 0, c_o = 0, c_gu = 0, c_down = 0, o_qkv = 0, o_o = 0, o_gu = 0, o_down = 0;
   bool early = m->att_early && m->pdl && m->skip == 0;
