@@ -78,10 +78,11 @@ UGB_API void *ugb_device_stream(const ugb_device *dev);
 /* Number of kernels this library has launched on `dev` since creation. */
 UGB_API uint64_t ugb_launch_count(const ugb_device *dev);
 /* Tuning switches of a device handle (no counterpart in the reference).
- *   "gemm_cta_pairs"  1 (default) / 0: bf16 GEMMs with more than 128 rows run
- *                     256 x 256 tiles on pairs of CTAs (tcgen05 cta_group::2, a
- *                     cluster of two SMs sharing the B operand) instead of
- *                     128 x 256 tiles on single CTAs.  Same results bit for bit.
+ *   "gemm_cta_pairs"  1 (default) / 0: bf16 / f16 GEMMs with more than 128 rows
+ *                     may run tiles of 256 rows (and 128 to 256 columns) on pairs
+ *                     of CTAs (tcgen05 cta_group::2, a cluster of two SMs sharing
+ *                     the B operand) where the predicted time is best; 0 leaves
+ *                     128-row tiles on single CTAs.  Same results bit for bit.
  *   "wait_limit_us"   100 .. 60000000 (default 2000000): how long a device-side
  *                     wait on something another agent completes (an mbarrier fed
  *                     by TMA / MMA, a peer GPU's flag, a grid-wide barrier) may

@@ -6,6 +6,7 @@ import pytest
 
 from conftest import ROOT
 from test_f32_tile_gpu import TURNED
+from test_llama_prefill_gpu import SPLIT_PROMPT
 from test_tc_shapes_gpu import SHAPES
 
 SMS = 148
@@ -47,6 +48,15 @@ def test_tensor_core_shapes(ask, case):
 
 def test_every_shape_is_reached():
     assert set(SHAPES.values()) == {(64, False), (128, False), (192, False), (256, False), (128, True), (192, True), (256, True)}
+
+
+def test_prompt_that_splits_k(ask):
+    cfg, rows, splits = SPLIT_PROMPT
+    h, f = cfg["hidden_size"], cfg["intermediate_size"]
+    for cap, (o, down) in splits.items():
+        assert (ask("tc", rows, h, h, 0, 1, cap)[2], ask("tc", rows, h, f, 0, 1, cap)[2]) == (o, down)
+    # with or without pairs decides over a split only where the planner is asked without them
+    assert ask("tc", 2310, 2048, 5632, 0, 1, 3)[2] == 1 and ask("tc", 2310, 2048, 5632, 0, 0, 3)[2] == 2
 
 
 @pytest.mark.parametrize("m,n,k", TURNED)

@@ -180,3 +180,41 @@ def test_long_prefill_many_key_tiles(dev, tc):
     assert logit_err(got[1], want[300:]) < TOL
     assert gpu.position == 1100
     gpu.close()
+
+
+# shape and rows of a prompt, and by the partials that the workspace takes how many its o and down products are split into (148 SMs)
+SPLIT_PROMPT = (dict(hidden_size=512, intermediate_size=1408, num_attention_heads=8, num_key_value_heads=2), 300, {1: (1, 1), 2: (2, 2), 4: (2, 3)})
+
+
+def test_prompt_whose_o_and_down_products_split_k(dev):
+    """Short prompts split k of the products that leave SMs idle, as far as a chunk's workspace takes the partials."""
+    over, t, splits = SPLIT_PROMPT
+    cfg = Config(**{**TINY, **over})
+    prompt, got = synth.tokens(29, (1, t), cfg.vocab_size), {}
+    for cap, rows in ((1, 320), (2, 640), (4, 8192)):
+        gpu, ref = make(cfg, dev, 1, 320)
+        gpu.set_option("prefill_rows", rows)
+        gpu.prefill(prompt, all_logits=True)
+        got[cap] = gpu.prefill_logits()[0]
+        assert logit_err(got[cap], ref.fwd(prompt, 0, ref.new_cache())[0]) < TOL
+        gpu.close()
+    assert not np.array_equal(got[1], got[2]) and not np.array_equal(got[2], got[4])      # other sums, so other roundings
+
+
+def test_cta_pairs_do_not_change_a_prompts_bits(dev):
+    """gemm_cta_pairs chooses tile shapes.  Without pairs a split of k would pay for the down product of these 2310 rows, with them it
+    does not: the option must not decide over it."""
+    cfg = Config(hidden_size=2048, intermediate_size=5632, num_attention_heads=32, num_key_value_heads=4, num_hidden_layers=1, vocab_size=512,
+                 max_position_embeddings=2400)
+    gpu = Model.new(cfg, synth.llama_weights(cfg, 5), dev, 1, 2400)
+    prompt, got = synth.tokens(3, (1, 2310), cfg.vocab_size), []
+    try:
+        for pairs in (1, 0):
+            dev.set_option("gemm_cta_pairs", pairs)
+            gpu.reset(0)
+            gpu.prefill(prompt, all_logits=True)
+            got.append(gpu.prefill_logits())
+    finally:
+        dev.set_option("gemm_cta_pairs", 1)
+    assert np.array_equal(got[0], got[1])
+    gpu.close()

@@ -503,10 +503,11 @@ int32_t llama_prefill_chunk(ugb_llama *m, const int *tok, int t, int c0, int tc,
   float *po = o_out(m, m->pf_f32), *pd = down_out(m, m->pf_f32);
   // The reduce kernel adds partials, so the two products before it may split k where their tiles leave SMs idle, as far as the
   // buffer (and the exchange block, which holds no fewer rows) takes the partials.  Several ranks read one partial of each other.
+  // Planned as with CTA pairs whatever option gemm_cta_pairs says: a split changes the order of the sums, a tile shape does not.
   const size_t pf_cap = m->tp_size > 1 ? 1 : (size_t)m->pf_rows / (size_t)rows;
   auto split_plan = [&](size_t k) {
     const int most = (int)std::min<size_t>(4, pf_cap);
-    return rows > 64 && most > 1 ? ugb_tc_gemm_plan(dev->sm_count, 1, rows, H, k, true, dev->gemm_pair != 0, most) : ugb_tc_plan{};
+    return rows > 64 && most > 1 ? ugb_tc_gemm_plan(dev->sm_count, 1, rows, H, k, true, true, most) : ugb_tc_plan{};
   };
   const ugb_tc_plan plan_o = split_plan(AW), plan_down = split_plan(c.ffn);
   auto bn_of = [](const ugb_tc_plan &x) { return x.splits > 1 ? x.bn : 0; };
