@@ -484,7 +484,11 @@ UGB_API int32_t ugb_llama_load_weight(ugb_llama *m, const char *name, const ugb_
  * epilogue is done, at its end (values 0..5 of a projection) and at every k
  * block of its main loop (values 8..); UGB_LLAMA_GEMM_PROFILE reads 5 x 64
  * floats (qkv, o, gate|up, down, lm_head of the last launches), microseconds
- * after the projection's own wait returned, 0 = not recorded. */
+ * after the projection's own wait returned, 0 = not recorded.
+ * Steps of up to 8 sequences run their projections on a kernel that streams the
+ * weights through registers: the tile widths, "gemm_smem_kib" and "gate_up_pair"
+ * mean nothing there, the split factors follow from the shapes until one is set,
+ * and "gemm_profile" moves the step to the kernel whose timeline it records. */
 UGB_API int32_t ugb_llama_set_option(ugb_llama *m, const char *key, int32_t value);
 /* Sets the number of cached positions (0 = empty cache); cache contents at
  * positions >= pos are ignored by later steps. */

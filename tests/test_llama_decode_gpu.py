@@ -252,6 +252,27 @@ def test_gemm_tile_widths_agree(dev, bn):
     gpu.close()
 
 
+@pytest.mark.parametrize("batch", [1, 8, 9])
+def test_split_factors_that_a_caller_sets_hold_at_every_batch(dev, batch):
+    """The split factors say how many f32 partials a projection is summed from, whichever kernel runs it: other factors round
+    differently, setting one again gives its bits again."""
+    cfg = Config(**{**TINY, "hidden_size": 512, "num_attention_heads": 8, "num_key_value_heads": 2, "intermediate_size": 2048})
+    gpu, ref = make(cfg, dev, batch, 32)
+    prompts, seen = synth.tokens(41, (batch, 6), cfg.vocab_size), {}
+    for key, values in (("splits_down", (1, 8)), ("splits_o", (1, 8)), ("splits_qkv", (1, 8))):
+        for v in values + values[:1]:
+            gpu.set_option(key, v)
+            worst, _ = run_teacher_forced(gpu, ref, prompts, check_seqs=[batch - 1])
+            assert worst < TOL
+            h = gpu.hidden()
+            if (key, v) in seen:
+                assert np.array_equal(h, seen[key, v])
+            seen[key, v] = h
+        if key != "splits_qkv":                       # those sums are rounded to bf16 before anything else, and often to the same values
+            assert not np.array_equal(seen[key, 1], seen[key, 8])
+    gpu.close()
+
+
 @pytest.mark.parametrize("batch", [64, 1, 8])
 def test_attention_front_end_variants_are_bit_identical(dev, batch):
     """Work moved in front of griddepcontrol.wait (the attention kernel's K / V ring, the norm kernel's

@@ -70,6 +70,7 @@ struct ugb_llama : ugb_engine {   // t_max is padded to a multiple of 16
   int *tok = nullptr;
   // tuning
   int splits_qkv = 5, splits_o = 8, splits_down = 8, att_splits = 1, att_stages = 5;
+  bool set_qkv = false, set_o = false, set_down = false;   // the caller set that split factor: it holds for few rows too
   int gemm_smem_kib = 144;        // shared-memory cap of the decode GEMM CTAs (0 = deepest ring); measured best
   int skip = 0;                   // measurement aid: bit mask of kernel types left out of the step
   int bn_qkv = 128, bn_o = 128, bn_gate_up = 128, bn_down = 128, bn_lm_head = 256;   // GEMM tile widths
@@ -171,9 +172,16 @@ int32_t gemm_rows(ugb_llama *m, size_t rows, void *out, const __nv_bfloat16 *a, 
   return rc;
 }
 
-// Partials that a step's projection writes for the split factor `option`.
-int step_splits(const ugb_llama *m, size_t n, size_t k, int option) {
-  return skinny(m, m->batch) ? ugb_skinny_splits(m->dev->sm_count, n, k) : ugb_tc_gemm_effective_splits(k, option);
+// Partials that the projections of a step write.
+struct StepSplits { int qkv, o, down; };
+StepSplits step_splits(const ugb_llama *m) {
+  const size_t H = m->lc.hidden, AW = (size_t)m->lc.n_heads * m->lc.head_dim;
+  const bool few = skinny(m, m->batch);
+  auto of = [&](size_t n, size_t k, int option, bool set) {
+    if (!few) return ugb_tc_gemm_effective_splits(k, option);
+    return set ? ugb_skinny_effective_splits(k, option) : ugb_skinny_splits(m->dev->sm_count, n, k);
+  };
+  return {of(m->qkv_dim, H, m->splits_qkv, m->set_qkv), of(H, AW, m->splits_o, m->set_o), of(H, m->lc.ffn, m->splits_down, m->set_down)};
 }
 
 int32_t gemm(ugb_llama *m, void *out, const __nv_bfloat16 *a, const __nv_bfloat16 *w, size_t n, size_t k,
@@ -417,8 +425,7 @@ int32_t llama_step(ugb_llama *m, const int *tok) {
   cudaError_t e = ugb_launch(embed_gather_kernel, dim3(B), dim3(256), 0, st, pdl, m->embed, tok, m->x, H, c.vocab, dev->status_dev, 1, 1, 0);
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of embed_gather_kernel failed: %s", cudaGetErrorString(e));
   if ((rc = ugb_after_launch(dev, "embed_gather_kernel"))) return rc;
-  const int s_qkv = step_splits(m, m->qkv_dim, H, m->splits_qkv), s_o = step_splits(m, H, AW, m->splits_o);
-  const int s_down = step_splits(m, H, c.ffn, m->splits_down);
+  const auto [s_qkv, s_o, s_down] = step_splits(m);
   const float scale = powf((float)c.head_dim, -0.5f);   // model.rs:236
   float *po = o_out(m, m->part), *pd = down_out(m, m->part);
   // Work done before griddepcontrol.wait (the attention kernel's K/V ring, the norm kernel's residual row)
@@ -924,9 +931,9 @@ int32_t ugb_llama_set_option(ugb_llama *m, const char *key, int32_t value) {
     return UGB_OK;
   }
   UGB_REQUIRE(dev, value >= 1 && value <= 8, UGB_ERR_INVALID, "option %s: value %d outside 1..8", key, value);
-  if (k == "splits_qkv") m->splits_qkv = value;
-  else if (k == "splits_o") m->splits_o = value;
-  else if (k == "splits_down") m->splits_down = value;
+  if (k == "splits_qkv") m->splits_qkv = value, m->set_qkv = true;
+  else if (k == "splits_o") m->splits_o = value, m->set_o = true;
+  else if (k == "splits_down") m->splits_down = value, m->set_down = true;
   else if (k == "att_splits") m->att_splits = value;
   else if (k == "att_stages") m->att_stages = value < 2 ? 2 : (value > 6 ? 6 : value);
   else return ugb_fail(dev, UGB_ERR_INVALID, "unknown option %s", key);
@@ -1013,8 +1020,7 @@ int32_t ugb_llama_time_kernel(ugb_llama *m, int32_t which, int32_t iters, float 
   const ugb_llama_config &c = m->lc;
   const int H = c.hidden, AW = c.n_heads * c.head_dim;
   const float scale = powf((float)c.head_dim, -0.5f);
-  const int s_qkv = step_splits(m, m->qkv_dim, H, m->splits_qkv), s_o = step_splits(m, H, AW, m->splits_o);
-  const int s_down = step_splits(m, H, c.ffn, m->splits_down);
+  const auto [s_qkv, s_o, s_down] = step_splits(m);
   int32_t rc = UGB_OK;
   // the kernels read the device-side position; during timing it must name the last cached position
   const int last = m->host_pos - 1;
