@@ -888,6 +888,7 @@ int32_t ugb_llama_set_option(ugb_llama *m, const char *key, int32_t value) {
     }
     if (!value) m->gemm_prof = nullptr;
     engine_drop_graph(m);
+    m->warmed = false;            // few rows change kernels with it
     return UGB_OK;
   }
   if (k == "gate_up_pair") {
