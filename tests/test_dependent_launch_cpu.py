@@ -61,3 +61,14 @@ def test_few_rows_read_ahead_on_late_triggers_only():
     src = open(os.path.join(CSRC, "llama_engine.cu")).read()
     body = src[src.index("int32_t gemm_rows("):src.index("int32_t gemm(ugb_llama")]
     assert "late_trigger = true" in body and "late_trigger = false" not in body
+
+
+def test_f32_products_of_an_engine_follow_its_option():
+    """pdl = 0 means ordinary launches for the f32 products of a layer-list model too."""
+    engine, products = (open(os.path.join(CSRC, f)).read() for f in ("hybrid_engine.cu", "matmul.cu"))
+    call = engine[engine.index("ugb_f32_gemm("):]
+    assert "m->pdl != 0" in call[:call.index(";")]
+    gemm = products[products.index("int32_t ugb_f32_gemm("):products.index('extern "C" {')]
+    assert gemm.count("pdl") >= 3 and "true)" not in re.sub(r"R\{[^}]*\}", "", gemm)
+    launches = re.findall(r"ugb_launch(?:_cluster)?\(([^;]*?)\)[;\n]", products)
+    assert len(launches) >= 4 and all("dev->stream, pdl," in l for l in launches)

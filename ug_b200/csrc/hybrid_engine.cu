@@ -61,7 +61,7 @@ int32_t ugb_hybrid_matmul(ugb_hybrid *m, const Mat &x) {
       return ugb_f32_grouped_gemm(dev, (float *)x.out, (const float *)x.a, (const float *)x.w, x.groups, x.m, x.tile, (int)x.n, (int)x.k);
     int32_t rc = ugb_f32_gemm(dev, (float *)x.out, (const float *)x.a, (const float *)x.w, x.batch, x.m, x.n, x.k,
                               x.a_ld ? x.a_ld : x.k, x.a_batch, x.nk, x.w_batch, x.c_ld ? x.c_ld : x.n,
-                              x.c_batch ? x.c_batch : x.m * (x.c_ld ? x.c_ld : x.n));
+                              x.c_batch ? x.c_batch : x.m * (x.c_ld ? x.c_ld : x.n), m->pdl != 0);
     if (rc || !(x.relu2 || x.silu_mul)) return rc;
     if (x.silu_mul) return ugb_fail(dev, UGB_ERR_UNSUPPORTED, "f32 product with a fused gate");
     relu2_kernel<<<dev->sm_count * 4, 256, 0, dev->stream>>>((float *)x.out, x.m * x.n / 4);

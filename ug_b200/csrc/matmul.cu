@@ -434,21 +434,21 @@ short_k_kernel(const F32Params p) {
 inline bool al16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
 template <typename E, int WM, int WK, bool VEC, bool TURNED = false>
-int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b) {
+int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b, bool pdl) {
   using T = F32Tile<WM, WK>;
   const dim3 grid((unsigned)((p.n + T::BN - 1) / T::BN * p.split), (unsigned)((p.m + T::BM - 1) / T::BM), (unsigned)b);
   const size_t smem = WK * p.split > 1 ? std::max(T::SMEM, T::SMEM_REDUCE) : T::SMEM;
   if (smem > 48 * 1024) UGB_CUDA(dev, cudaFuncSetAttribute(f32_tile_kernel<E, WM, WK, VEC, TURNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const cudaError_t e = ugb_launch_cluster(f32_tile_kernel<E, WM, WK, VEC, TURNED>, grid, dim3(T::THREADS), smem, dev->stream, true, p.split, p);
+  const cudaError_t e = ugb_launch_cluster(f32_tile_kernel<E, WM, WK, VEC, TURNED>, grid, dim3(T::THREADS), smem, dev->stream, pdl, p.split, p);
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of f32_tile_kernel failed: %s", cudaGetErrorString(e));
   return ugb_after_launch(dev, "f32_tile_kernel");
 }
 
 template <typename E, bool VEC>
-int32_t launch_f32_tile(ugb_device *dev, F32Params p, size_t b) {
+int32_t launch_f32_tile(ugb_device *dev, F32Params p, size_t b, bool pdl) {
   UGB_REQUIRE(dev, b <= 65535 && ((size_t)p.m + 127) / 128 <= 65535, UGB_ERR_UNSUPPORTED, "matmul: m or batch too large for the FP32-pipe kernel");
   if (p.k <= SHORT_K && (p.m + 63) / 64 <= 65535 && (sizeof(E) == 2 || b * (size_t)p.m * (size_t)p.n <= (VEC ? SHORT_K_F32_VEC_RESULTS : SHORT_K_F32_RESULTS))) {
-    const cudaError_t e = ugb_launch(short_k_kernel<E>, dim3((unsigned)((p.n + 63) / 64), (unsigned)((p.m + 63) / 64), (unsigned)b), dim3(256), 0, dev->stream, true, p);
+    const cudaError_t e = ugb_launch(short_k_kernel<E>, dim3((unsigned)((p.n + 63) / 64), (unsigned)((p.m + 63) / 64), (unsigned)b), dim3(256), 0, dev->stream, pdl, p);
     if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of short_k_kernel failed: %s", cudaGetErrorString(e));
     return ugb_after_launch(dev, "short_k_kernel");
   }
@@ -461,15 +461,15 @@ int32_t launch_f32_tile(ugb_device *dev, F32Params p, size_t b) {
     std::swap(p.a_b, p.b_b);
     std::swap(p.a_rs, p.b_cs);
     std::swap(p.a_cs, p.b_rs);
-    return s.wk == 4 ? launch_f32_shape<E, 1, 4, VEC, true>(dev, p, b) : launch_f32_shape<E, 2, 2, VEC, true>(dev, p, b);
+    return s.wk == 4 ? launch_f32_shape<E, 1, 4, VEC, true>(dev, p, b, pdl) : launch_f32_shape<E, 2, 2, VEC, true>(dev, p, b, pdl);
   }
-  if (s.wk == 4) return launch_f32_shape<E, 1, 4, VEC>(dev, p, b);
-  if (s.wk == 2) return launch_f32_shape<E, 2, 2, VEC>(dev, p, b);
-  return launch_f32_shape<E, 4, 1, VEC>(dev, p, b);
+  if (s.wk == 4) return launch_f32_shape<E, 1, 4, VEC>(dev, p, b, pdl);
+  if (s.wk == 2) return launch_f32_shape<E, 2, 2, VEC>(dev, p, b, pdl);
+  return launch_f32_shape<E, 4, 1, VEC>(dev, p, b, pdl);
 }
 
 int32_t launch_f32(ugb_device *dev, float *dst, const float *lhs, const float *rhs, size_t b, size_t m, size_t n, size_t k,
-                   const MatLayout &L, const MatLayout &R) {
+                   const MatLayout &L, const MatLayout &R, bool pdl) {
   if (k == 0) {
     UGB_CUDA(dev, cudaMemsetAsync(dst, 0, b * m * n * sizeof(float), dev->stream));
     return UGB_OK;
@@ -478,7 +478,7 @@ int32_t launch_f32(ugb_device *dev, float *dst, const float *lhs, const float *r
   const bool bases = al16(dst) && al16(lhs) && al16(rhs) && L.batch % 4 == 0 && R.batch % 4 == 0;
   if (m <= 16 && !L.transposed && R.transposed && k % 4 == 0 && bases) {
     const dim3 grid((unsigned)((n + 7) / 8), (unsigned)b);
-#define UGB_SKINNY(MR) ugb_launch(f32_skinny_kernel<MR>, grid, dim3(256), 0, dev->stream, true, dst, lhs, rhs, (int)m, (int)n, (int)k, L.batch, R.batch)
+#define UGB_SKINNY(MR) ugb_launch(f32_skinny_kernel<MR>, grid, dim3(256), 0, dev->stream, pdl, dst, lhs, rhs, (int)m, (int)n, (int)k, L.batch, R.batch)
     if (m <= 1) UGB_SKINNY(1); else if (m <= 2) UGB_SKINNY(2); else if (m <= 4) UGB_SKINNY(4); else if (m <= 8) UGB_SKINNY(8); else UGB_SKINNY(16);
 #undef UGB_SKINNY
     return ugb_after_launch(dev, "f32_skinny_kernel");
@@ -487,7 +487,7 @@ int32_t launch_f32(ugb_device *dev, float *dst, const float *lhs, const float *r
   if (m <= 8 && !L.transposed && !R.transposed && (L.cs == 1 || k == 1) && (R.cs == 1 || n == 1) && n % 4 == 0 &&
       R.rs % 4 == 0 && R.batch % 4 == 0 && al16(rhs)) {
     const dim3 grid((unsigned)((n + 127) / 128), (unsigned)b);
-#define UGB_SKINNY_N(MR) ugb_launch(f32_skinny_n_kernel<MR>, grid, dim3((MR) <= 2 ? 1024 : ((MR) <= 4 ? 512 : 256)), 0, dev->stream, true, dst, lhs, rhs, (int)m, (int)n, (int)k, L.rs, L.batch, R.rs, R.batch)
+#define UGB_SKINNY_N(MR) ugb_launch(f32_skinny_n_kernel<MR>, grid, dim3((MR) <= 2 ? 1024 : ((MR) <= 4 ? 512 : 256)), 0, dev->stream, pdl, dst, lhs, rhs, (int)m, (int)n, (int)k, L.rs, L.batch, R.rs, R.batch)
     if (m <= 1) UGB_SKINNY_N(1); else if (m <= 2) UGB_SKINNY_N(2); else if (m <= 4) UGB_SKINNY_N(4); else UGB_SKINNY_N(8);
 #undef UGB_SKINNY_N
     return ugb_after_launch(dev, "f32_skinny_n_kernel");
@@ -498,7 +498,7 @@ int32_t launch_f32(ugb_device *dev, float *dst, const float *lhs, const float *r
   const bool vec = bases && a_c % 4 == 0 && a_ld % 4 == 0 && b_c % 4 == 0 && b_ld % 4 == 0 && n % 4 == 0;
   {
     const F32Params p{dst, lhs, rhs, (int)m, (int)n, (int)k, L.rs, L.cs, L.batch, R.rs, R.cs, R.batch, (long long)n, (long long)(m * n), 1, 0};
-    return vec ? launch_f32_tile<float, true>(dev, p, b) : launch_f32_tile<float, false>(dev, p, b);
+    return vec ? launch_f32_tile<float, true>(dev, p, b, pdl) : launch_f32_tile<float, false>(dev, p, b, pdl);
   }
 }
 
@@ -550,11 +550,11 @@ int32_t ugb_f32_grouped_gemm(ugb_device *dev, float *c, const float *a, const fl
 }
 
 int32_t ugb_f32_gemm(ugb_device *dev, float *c, const float *a, const float *b, size_t batch, size_t m, size_t n, size_t k,
-                     size_t a_ld, size_t a_batch, bool b_is_nk, size_t b_batch, size_t c_ld, size_t c_batch) {
+                     size_t a_ld, size_t a_batch, bool b_is_nk, size_t b_batch, size_t c_ld, size_t c_batch, bool pdl) {
   if (batch == 0 || m == 0 || n == 0) return UGB_OK;
   if (batch == 1 && a_ld == k && c_ld == n && b_is_nk && k > 0) {   // a Linear: the skinny kernel takes few rows
     const MatLayout L{(long long)k, 1, (long long)a_batch, false}, R{1, (long long)k, (long long)b_batch, true};
-    return launch_f32(dev, c, a, b, batch, m, n, k, L, R);
+    return launch_f32(dev, c, a, b, batch, m, n, k, L, R, pdl);
   }
   UGB_REQUIRE(dev, batch <= 65535 && (m + 127) / 128 <= 65535 && m < (1u << 31) && n < (1u << 31) && k < (1u << 31), UGB_ERR_UNSUPPORTED,
               "f32 product: extent too large");
@@ -563,7 +563,7 @@ int32_t ugb_f32_gemm(ugb_device *dev, float *c, const float *a, const float *b, 
   const long long b_rs = b_is_nk ? 1 : (long long)n, b_cs = b_is_nk ? (long long)k : 1;
   {
     const F32Params p{c, a, b, (int)m, (int)n, (int)k, (long long)a_ld, 1, (long long)a_batch, b_rs, b_cs, (long long)b_batch, (long long)c_ld, (long long)c_batch, 1, 0};
-    return vec ? launch_f32_tile<float, true>(dev, p, batch) : launch_f32_tile<float, false>(dev, p, batch);
+    return vec ? launch_f32_tile<float, true>(dev, p, batch, pdl) : launch_f32_tile<float, false>(dev, p, batch, pdl);
   }
 }
 
@@ -645,14 +645,14 @@ int32_t ugb_matmul(ugb_device *dev, ugb_slice *dst, const ugb_slice *lhs, const 
     if (src != UGB_ERR_UNSUPPORTED) return src;
   }
   switch (dt) {
-    case UGB_F32: return launch_f32(dev, (float *)dst->ptr, (const float *)lp, (const float *)rp, b, m, n, k, L, R);
+    case UGB_F32: return launch_f32(dev, (float *)dst->ptr, (const float *)lp, (const float *)rp, b, m, n, k, L, R, true);
     default: {
       if (k == 0) {
         UGB_CUDA(dev, cudaMemsetAsync(dst->ptr, 0, b * m * n * es, dev->stream));
         return UGB_OK;
       }
       const F32Params p{dst->ptr, lp, rp, (int)m, (int)n, (int)k, L.rs, L.cs, L.batch, R.rs, R.cs, R.batch, (long long)n, (long long)(m * n), 1, 0};
-      return dt == UGB_BF16 ? launch_f32_tile<__nv_bfloat16, false>(dev, p, b) : launch_f32_tile<__half, false>(dev, p, b);
+      return dt == UGB_BF16 ? launch_f32_tile<__nv_bfloat16, false>(dev, p, b, true) : launch_f32_tile<__half, false>(dev, p, b, true);
     }
   }
 }

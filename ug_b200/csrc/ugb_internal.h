@@ -75,9 +75,9 @@ static inline cudaError_t ugb_malloc_async(ugb_device *dev, void **p, size_t byt
 }
 
 // c[b, m, n] = a[b, m, k] . w on the FP32 pipe, a row-major with row stride a_ld, w [n, k] (b_is_nk) or [k, n] row-major,
-// c with row stride c_ld; *_batch: elements between batch steps (0 = shared operand).
+// c with row stride c_ld; *_batch: elements between batch steps (0 = shared operand); pdl: as a dependent launch.
 int32_t ugb_f32_gemm(ugb_device *dev, float *c, const float *a, const float *b, size_t batch, size_t m, size_t n, size_t k,
-                     size_t a_ld, size_t a_batch, bool b_is_nk, size_t b_batch, size_t c_ld, size_t c_batch);
+                     size_t a_ld, size_t a_batch, bool b_is_nk, size_t b_batch, size_t c_ld, size_t c_batch, bool pdl);
 
 // c[m, n] = a[m, k] . w with rows grouped by the weights they multiply: rows of tile i (tile_m of them, a multiple of 64) take
 // the n rows of w [.., k] from groups[i] * n on; groups (device memory) < 0: rows without work.
