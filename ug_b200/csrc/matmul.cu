@@ -14,6 +14,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "gemm_plan.h"
 #include "gemm_skinny.cuh"
@@ -438,7 +439,11 @@ int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b, bool pdl
   using T = F32Tile<WM, WK>;
   const dim3 grid((unsigned)((p.n + T::BN - 1) / T::BN * p.split), (unsigned)((p.m + T::BM - 1) / T::BM), (unsigned)b);
   const size_t smem = WK * p.split > 1 ? std::max(T::SMEM, T::SMEM_REDUCE) : T::SMEM;
-  if (smem > 48 * 1024) UGB_CUDA(dev, cudaFuncSetAttribute(f32_tile_kernel<E, WM, WK, VEC, TURNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  constexpr unsigned bit = 1u << ((sizeof(E) == 4 ? VEC : std::is_same<E, __half>::value ? 2 : 3) * 6 + (TURNED ? 3 : 0) + (WM == 4 ? 0 : WM == 2 ? 1 : 2));
+  if (smem > 48 * 1024 && !(dev->f32_smem_set & bit)) {      // once: a step that is captured has run eagerly before
+    UGB_CUDA(dev, cudaFuncSetAttribute(f32_tile_kernel<E, WM, WK, VEC, TURNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(T::SMEM, T::SMEM_REDUCE)));
+    dev->f32_smem_set |= bit;
+  }
   const cudaError_t e = ugb_launch_cluster(f32_tile_kernel<E, WM, WK, VEC, TURNED>, grid, dim3(T::THREADS), smem, dev->stream, pdl, p.split, p);
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of f32_tile_kernel failed: %s", cudaGetErrorString(e));
   return ugb_after_launch(dev, "f32_tile_kernel");
