@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 from conftest import ROOT
-from kabidra_cases import CONFIGS, agree, oracle, oracle_logits, tokens, weights, write_model
+from kabidra_cases import CONFIGS, K, agree, oracle, oracle_logits, tokens, weights, write_model
 from ug_b200 import DType, UgError, synth
 from ug_b200.generate import generate
 from ug_b200.kabidra import Config, Layer, Model
@@ -115,7 +115,7 @@ def test_prompt_in_engine_chunks(make, dtype):
 
 
 @pytest.mark.parametrize("dtype", BOTH)
-@pytest.mark.parametrize("batch", [3, 70])
+@pytest.mark.parametrize("batch", [3, 8, 9, 33, 70])      # steps: streamed weights up to 8 rows, 64-row tiles, 128-row ones
 def test_batch_rows_are_independent(make, dtype, batch):
     """Different sequences in one batch, in a prompt, a continued prompt and steps; the same as each alone."""
     rows = tokens("mixed", 45, 60, batch)
@@ -134,6 +134,24 @@ def test_batch_rows_are_independent(make, dtype, batch):
     alone = make("mixed", dtype, 1, 96)
     alone.prefill(rows[1:2, :57])
     assert agree(b[1, -1:], alone.logits().astype(np.float64), dtype == DType.F32, 2.0)
+
+
+@pytest.mark.parametrize("batch", [1, 8, 9])
+def test_wide_steps(dev, batch):
+    """Steps at widths where the products of few rows leave several f32 partials."""
+    cfg = Config(vocab=64, width=1024, eps=1e-5, taps=4,
+                 layers=[Layer("mingru", dict(width=1152), 2816), Layer("latent_attention", dict(heads=16, dim=64, vdim=64, q_rank=256, kv_rank=256, scale=0.2), 1408)])
+    w = synth.kabidra_weights(cfg, 301)
+    ref = K.Model(cfg.to_dict(), synth.llama_weights_f32(w))
+    rows = synth.tokens(78, (batch, 12), cfg.vocab)
+    m = Model.new(cfg, w, dev, batch, 32, DType.BF16)
+    got = []
+    for i in range(12):
+        m.fwd(rows[:, i])
+        got.append(m.logits())
+    for k in {0, batch - 1}:
+        assert agree(np.stack([g[k] for g in got]), ref.fwd([int(x) for x in rows[k]], ref.new_state()), False)
+    m.close()
 
 
 @pytest.mark.parametrize("dtype", BOTH)

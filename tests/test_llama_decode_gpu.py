@@ -131,13 +131,23 @@ def test_full_width_two_layers_greedy(dev):
     gpu.close()
 
 
+@pytest.mark.parametrize("batch", [1, 8])
+def test_wide_steps_of_few_rows(dev, batch):
+    """Widths at which the products of few rows leave several f32 partials."""
+    cfg = Config(**{**TINY, "hidden_size": 1024, "intermediate_size": 2816, "num_attention_heads": 16, "num_key_value_heads": 4, "max_position_embeddings": 128})
+    gpu, ref = make(cfg, dev, batch, 32)
+    worst, _ = run_teacher_forced(gpu, ref, synth.tokens(13, (batch, 8), cfg.vocab_size), check_seqs=sorted({0, batch - 1}))
+    assert worst < TOL
+    gpu.close()
+
+
 def test_gate_up_on_cta_pairs_or_single_ctas(dev):
     """The gate|up projection of a decode step runs its k halves on a pair of CTAs (a cluster) that exchange their
     sums through shared memory, or on one CTA per tile: two summation orders of the same products, both within
     tolerance of the oracle, at a width whose last tile is partly outside (ffn 5632: 11264 = 70 x 160 + 64) and at
     a small one."""
     for over, batch in (({"hidden_size": 2048, "intermediate_size": 5632, "num_attention_heads": 32, "num_key_value_heads": 4,
-                          "num_hidden_layers": 1, "vocab_size": 512, "max_position_embeddings": 128}, 64), ({}, 5)):
+                          "num_hidden_layers": 1, "vocab_size": 512, "max_position_embeddings": 128}, 64), ({}, 9)):
         cfg = Config(**{**TINY, **over})
         gpu, ref = make(cfg, dev, batch, 32)
         prompts = synth.tokens(12, (batch, 6), cfg.vocab_size)

@@ -15,7 +15,8 @@ from conftest import ROOT
 from ug_b200 import DType, UgError, synth
 from ug_b200.generate import generate
 from ug_b200.zidevik import Config, Model
-from zidevik_cases import CONFIGS, agree, layer, oracle, oracle_logits, position_err, reference, tokens, weights, write_model
+from ug_b200.zidevik_config import Experts, Loop
+from zidevik_cases import CONFIGS, agree, layer, oracle, oracle_logits, position_err, reference, separate_experts, tokens, weights, write_model
 
 pytestmark = pytest.mark.gpu
 BOTH = [DType.F32, DType.BF16]
@@ -131,7 +132,7 @@ def test_prompt_in_engine_chunks(make, dtype):
 
 
 @pytest.mark.parametrize("dtype", BOTH)
-@pytest.mark.parametrize("batch", [3, 70])
+@pytest.mark.parametrize("batch", [3, 8, 9, 33, 70])      # steps: streamed weights up to 8 rows, 64-row tiles, 128-row ones
 def test_batch_rows_are_independent(make, dtype, batch):
     """Different sequences in one batch, in a prompt, a continued prompt and steps; the same as each alone."""
     rows = tokens("mixed", 45, 60, batch)
@@ -150,6 +151,24 @@ def test_batch_rows_are_independent(make, dtype, batch):
     alone = make("mixed", dtype, 1, 96)
     alone.prefill(rows[1:2, :57])
     assert agree(b[1, -1:], alone.logits().astype(np.float64), dtype == DType.F32, 2.0)
+
+
+@pytest.mark.parametrize("batch", [1, 8, 9])
+def test_wide_steps(dev, batch):
+    """Steps at widths where the products of few rows leave several f32 partials, the token's gate is formed inside a product over
+    more than one chunk of k, and eight tokens choose more than 32 experts between them."""
+    cfg = Config(vocab=64, width=1024, eps=1e-5, loop=Loop(0, 1, 2), side_dim=256, logit_softcap=3.0, layers=[
+        layer((4, 2, 64, 64, 64, 5000.0, 0.3), (256, 16, 4, 32), Experts(64, 8, 40, 64)), layer((8, 2, 64, 64, 32, 900.0, 0.3), (128, 8, 3, 16), 1408)])
+    w = separate_experts(cfg, synth.zidevik_weights(cfg, 501))
+    rows, ref = synth.tokens(77, (batch, 12), cfg.vocab), reference(cfg, w)
+    m = Model.new(cfg, w, dev, batch, 32, DType.BF16)
+    got = []
+    for i in range(12):
+        m.fwd(rows[:, i])
+        got.append(m.logits())
+    for k in {0, batch - 1}:
+        assert agree(np.stack([g[k] for g in got]), ref.fwd([int(x) for x in rows[k]], ref.new_state()), False)
+    m.close()
 
 
 @pytest.mark.parametrize("dtype", BOTH)
