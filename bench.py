@@ -586,7 +586,7 @@ class GraphDecodeWorkload:
 
 class F32MatmulWorkload:
     """f32 matmul_t on the FP32 pipe (the dtype ug-llama casts every weight to, model.rs:118,140,313): the
-    128 x 128 register-blocked kernel on 4096^3 ("gemm_f32", FP32-pipe bound) or the warp-per-column kernel on one
+    register-blocked tile kernel on 4096^3 ("gemm_f32", FP32-pipe bound) or the warp-per-column kernel on one
     activation row against the [32000, 2048] embedding ("gemv_f32", HBM bound on the weight)."""
     dtype = "f32"
     kernel_only = True

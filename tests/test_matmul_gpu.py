@@ -148,7 +148,7 @@ def test_f16_tensor_core_matmul(dev, bs, m, n, k, t):
     assert np.abs(got - ref.astype(np.float16).astype(np.float32)).mean() < 3e-4 * np.abs(ref).mean()
 
 
-# ---- f32 on the FP32 pipe: the skinny (decode) kernel and the 128 x 128 register-blocked kernel ----------------
+# ---- f32 on the FP32 pipe: the skinny (decode) kernel and the register-blocked tile kernel ----------------
 @pytest.mark.parametrize("bs,m,n,k,t", [
     (1, 1, 2048, 2048, True), (1, 3, 5632, 2048, True), (2, 16, 264, 512, True), (1, 8, 32000, 256, True),   # skinny
     (1, 130, 200, 72, True), (1, 130, 200, 72, False), (2, 256, 384, 128, True), (1, 512, 2048, 2048, True),  # tiles

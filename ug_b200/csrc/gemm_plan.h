@@ -20,10 +20,11 @@ inline int ugb_tc_gemm_effective_splits(size_t k, int splits) {
 struct ugb_tc_plan { int bn = 0, splits = 1; bool pair = false; };
 
 // Time of a product, in us: a launch and its epilogue, and for every round of tiles its k blocks at the pace that a tile of this
-// shape keeps, which falls as more SMs are at work (L2, and the clock under the power limit).  Fitted to 36 timed products of
-// 100-4096 rows, bf16, [n, k] weights; the choice was within 4 % of the best shape on 34 of them.  What it replaced took
-// 256 x 256 pairs above 128 rows and 128 x 64 below: [777, 2048] x [2560, 2048]^T 21.3 -> 16.5 us, x [2048, 2048]^T 19.9 -> 15.0,
-// x [11264, 2048]^T 45.9 -> 39.3, [777, 5632] x [2048, 5632]^T 36.3 -> 27.8, from 2048 rows on mostly as before.
+// shape keeps, which falls as more SMs are at work (L2, and the clock under the power limit).  Fitted to timed products of 100-4096
+// rows, bf16, [n, k] weights.  Against every shape on 32 of them (100 to 4096 rows, n of 2048 to 11264, k of 2048 and 5632) the choice is within
+// 2 % of the best on 29 and 7 % off at most.  256 x 256 pairs above 128 rows and 128 x 64 below, the rule before, take 17.7 us for
+// [777, 2048] x [2560, 2048]^T where the choice takes 12.0, 16.3 and 11.6 for x [2048, 2048]^T, 37.6 and 35.4 for x [11264, 2048]^T, 32.6 and 23.5
+// for [777, 5632] x [2048, 5632]^T; from 2048 rows on mostly the same shape.
 inline ugb_tc_plan ugb_tc_gemm_plan(int sm_count, size_t batch, size_t m, size_t n, size_t k, bool b_is_nk, bool pairs, int max_splits) {
   static const struct { int bn; bool pair; float pace, crowd, fixed; } shapes[] = {
       {256, true, .269f, .097f, 10.4f}, {192, true, .211f, .066f, 9.7f}, {128, true, .210f, .023f, 8.4f}, {256, false, .360f, .071f, 9.0f},

@@ -127,8 +127,8 @@ f32_skinny_kernel(float *C, const float *A, const float *B, int m, int n, int k,
 // (1b) Skinny products against a [k, n] operand with n contiguous (Attention::fwd's probabilities x values for the
 // one new token, model.rs:243: [1, T] x [T, 64] per head): one CTA per (128-column chunk, batch step); its warps (32 for
 // m <= 2, fewer for more rows) split k, a lane keeps 4 adjacent columns, so every k row of the chunk is one coalesced 512-byte read per warp and
-// is used for all m rows; the partial sums meet in shared memory.  (The 128 x 128 tile kernel below needs 199 us
-// for 32 heads x [1, 1024] x [1024, 64].)
+// is used for all m rows; the partial sums meet in shared memory.  (32 heads x [1, 1024] x [1024, 64] took 199 us
+// on 128 x 128 tiles.)
 template <int MR>
 __global__ void __launch_bounds__(MR <= 2 ? 1024 : (MR <= 4 ? 512 : 256))
 f32_skinny_n_kernel(float *C, const float *A, const float *B, int m, int n, int k, long long a_rs, long long a_b, long long b_rs, long long b_b) {
@@ -184,12 +184,12 @@ f32_skinny_n_kernel(float *C, const float *A, const float *B, int m, int n, int 
 // the edges; the columns of slice k are permuted by 8 (k / 4 mod 4), so that four lanes along k and eight along the rows write
 // without conflicts.
 //
-// [2048, 2048] x [4096, 2048]^T runs at 50 TFLOP/s, FMA pipe 75 % busy while its CTAs run (two CTAs of 256 threads with 8 x 8
-// outputs on 128 x 128 tiles: 41 and 64 %).  Against those: [257, 2048] x [5632, 2048]^T 310 -> 179 us, [1619, 1768] x
-// [984, 1768]^T 243 -> 140, [120, 7144] x [1352, 7144]^T 957 -> 114, [2, 6045] x [338, 6045]^T 951 -> 83.  Slices of 8 were
+// [2048, 2048] x [4096, 2048]^T runs at 45 TFLOP/s with k unsplit, FMA pipe 75 % busy while its CTAs run, and at 50 with k split in two, as it is
+// (two CTAs of 256 threads with 8 x 8 outputs on 128 x 128 tiles: 41, 64 %).  Against those: [257, 2048] x [5632, 2048]^T 288 -> 180 us,
+// [1619, 1768] x [984, 1768]^T 246 -> 136, [120, 7144] x [1352, 7144]^T 978 -> 112, [2, 6045] x [338, 6045]^T 977 -> 44.  Slices of 8 were
 // slower (683 -> 770 us on the first), and CTAs whose warps lie over columns no faster than these.
-// 16-bit operands (E) that no tensor-core kernel takes, odd rows above all: [500, 999] x [1001, 999]^T 169 -> 46 us, [11, 2001] x
-// [200, 2001]^T 267 -> 38 on 64 x 64 tiles of one 16-deep buffer before.
+// 16-bit operands (E) that no tensor-core kernel takes, odd rows above all: [500, 999] x [1001, 999]^T 168 -> 44 us, [11, 2001] x
+// [200, 2001]^T 271 -> 36 on 64 x 64 tiles of one 16-deep buffer before.
 template <int WM, int WK> struct F32Tile {
   static constexpr int BM = 32 * WM, BN = 128, BK = 16, THREADS = 32 * WM * WK;
   static constexpr int STAGE = BK * (BM + BN);                                     // floats
