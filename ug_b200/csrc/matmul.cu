@@ -188,6 +188,9 @@ f32_skinny_n_kernel(float *C, const float *A, const float *B, int m, int n, int 
 // (two CTAs of 256 threads with 8 x 8 outputs on 128 x 128 tiles: 41, 64 %).  Against those: [257, 2048] x [5632, 2048]^T 288 -> 180 us,
 // [1619, 1768] x [984, 1768]^T 246 -> 136, [120, 7144] x [1352, 7144]^T 978 -> 112, [2, 6045] x [338, 6045]^T 977 -> 44.  Slices of 8 were
 // slower (683 -> 770 us on the first), and CTAs whose warps lie over columns no faster than these.
+// The next kernel is let in by this one's end, not by a trigger: let in earlier, the CTAs of a product of 75 to 148 tiles come to SMs that are
+// still taken, two on one and none on another, and that product takes nearly twice as long (2 of [526, 216] x [1080, 216]^T one behind the other
+// 43 us with a trigger at the start, 34 with one behind the last slice, 26 without; 64 of [128, 64] x [128, 64]^T 12.4, 9.0, 8.8).
 // 16-bit operands (E) that no tensor-core kernel takes, odd rows above all: [500, 999] x [1001, 999]^T 168 -> 44 us, [11, 2001] x
 // [200, 2001]^T 271 -> 36 on 64 x 64 tiles of one 16-deep buffer before.
 template <int WM, int WK> struct F32Tile {
@@ -225,7 +228,6 @@ f32_tile_kernel(const F32Params p) {
   constexpr int BM = T::BM, BN = T::BN, BK = T::BK, QK = BK / 4, SW = 32 / QK;
   static_assert(T::THREADS == 128, "four warps");
   extern __shared__ __align__(16) float smem[];
-  ugb_pdl_trigger();
   ugb_pdl_wait();
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int rank = p.split > 1 ? (int)(blockIdx.x % p.split) : 0, n0 = (int)(p.split > 1 ? blockIdx.x / p.split : blockIdx.x) * BN;
