@@ -168,6 +168,7 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
         heads(a);
         a.pre = w.pre; a.n_part = in_t.splits; a.part_stride = pre_part;
         a.conv_w = L.conv_w; a.conv_b = L.conv_b; a.taps = d.conv; a.ci = L.ci; a.tail = tail; a.u = (T *)w.hc;
+        a.early = early ? 1 : 0;
         if (experts && whole) { a.experts = d.experts; a.top = d.top; a.choice = w.choice; a.count = w.count; }
         if ((rc = launch_mixer_inputs<float, T, true>(dev, a, rows, pdl))) return rc;
       }

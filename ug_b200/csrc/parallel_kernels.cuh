@@ -36,6 +36,7 @@ template <typename TI, typename T> struct MixerIn {
   int experts = 0, top = 0;
   float4 *choice = nullptr;                                // [rows][top]
   int *count = nullptr;                                    // [experts]
+  int early = 0;                                           // 1: position and tail may be read before the wait for the preceding kernel
   ugb_status_word *status = nullptr;
 };
 
@@ -88,9 +89,41 @@ mixer_inputs_kernel(MixerIn<TI, T> a, int rows) {
   const int n_head = a.heads + a.kv_heads;
   const MixerUnits n = mixer_units<STEP>(n_head, a.dp, a.kv_heads * a.vp, a.ci, a.experts);
   const int id = blockIdx.x * 8 + (threadIdx.x >> 5), r = id / n.all, unit = id - r * n.all, lane = threadIdx.x & 31;
+  // What the kernels before the predecessor wrote, and tables, are read ahead of the wait (see row_update_kernel): the position and
+  // then its angles, the convolution's tail and taps.  Behind it each was a round trip of its own, the taps one after the other:
+  // 8 rows of 10752 columns, 4 taps: 5.3 -> 2.9 us in the chain of a step.
+  constexpr int TAPS = STEP ? ROW_TAPS : 1;
+  const bool conv_unit = STEP && unit >= n.heads + n.v && unit < n.heads + n.v + n.x, short_conv = conv_unit && a.taps <= TAPS;
+  const int xc = (unit - n.heads - n.v) * 128 + 4 * lane;
+  int pos = 0;
+  float4 angle[2], tap[TAPS], tail[TAPS], conv_b = make_float4(0.f, 0.f, 0.f, 0.f);
+  bool angles = false;
+  auto ahead = [&]() {
+    if (r >= rows) return;
+    if (unit < n.heads + n.v) pos = *a.pos_p + a.pos_off + r % a.t;
+    if (unit < n.heads && a.interleaved && (a.rot_dims & 7) == 0 && pos >= 0 && pos < a.t_max) {
+      const int i0 = 8 * (lane % head_lanes(a.dp)), half = a.rot_dims >> 1;
+      angles = i0 < a.rot_dims;                            // four angles at once: all inside, the table's rows aligned
+      if (angles) {
+        angle[0] = __ldg(reinterpret_cast<const float4 *>(a.cos_ + (size_t)pos * half + (i0 >> 1)));
+        angle[1] = __ldg(reinterpret_cast<const float4 *>(a.sin_ + (size_t)pos * half + (i0 >> 1)));
+      }
+    }
+    if (short_conv && xc < a.ci) {
+      conv_b = __ldg(reinterpret_cast<const float4 *>(a.conv_b + xc));
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j)
+        if (j < a.taps) {
+          tap[j] = __ldg(reinterpret_cast<const float4 *>(a.conv_w + (size_t)j * a.ci + xc));
+          if (j + 1 < a.taps) tail[j] = Act<T>::ld4(a.tail + ((size_t)r * (a.taps - 1) + j) * a.ci + xc);
+        }
+    }
+  };
+  if (a.early) ahead();
   ugb_pdl_wait();
   ugb_pdl_trigger();
   if (r >= rows) return;
+  if (!a.early) ahead();
   const int b = r / a.t;
   const TI *row = a.pre + (size_t)r * a.ld;
   auto sum4 = [&](int c) {                                 // the partials are added in order
@@ -112,7 +145,6 @@ mixer_inputs_kernel(MixerIn<TI, T> a, int rows) {
     return s;
   };
   if (unit < n.heads + n.v) {
-    const int pos = *a.pos_p + a.pos_off + r % a.t;
     if (pos < 0 || pos >= a.t_max) {
       if (lane == 0 && atomicCAS(&a.status->code, 0u, (unsigned)UGB_ERR_INVALID) == 0u) a.status->detail = (unsigned)pos;
       return;
@@ -127,9 +159,9 @@ mixer_inputs_kernel(MixerIn<TI, T> a, int rows) {
         if (a.interleaved) {
           const int p0 = i0 >> 1;
           float c[4], s[4];
-          if ((half & 3) == 0) {                           // four angles at once: all inside, the table's rows aligned
-            *reinterpret_cast<float4 *>(c) = __ldg(reinterpret_cast<const float4 *>(cs + p0));
-            *reinterpret_cast<float4 *>(s) = __ldg(reinterpret_cast<const float4 *>(sn + p0));
+          if (angles) {
+            *reinterpret_cast<float4 *>(c) = angle[0];
+            *reinterpret_cast<float4 *>(s) = angle[1];
           } else {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -187,17 +219,23 @@ mixer_inputs_kernel(MixerIn<TI, T> a, int rows) {
   if constexpr (STEP) {
     const int x0 = n_head * a.dp + a.kv_heads * a.vp;
     if (unit < n.heads + n.v + n.x) {
-      const int c = (unit - n.heads - n.v) * 128 + 4 * lane;
+      const int c = xc;
       if (c >= a.ci) return;
-      float4 x = sum4(x0 + c), s = __ldg(reinterpret_cast<const float4 *>(a.conv_b + c));
+      float4 x = sum4(x0 + c), s = short_conv ? conv_b : __ldg(reinterpret_cast<const float4 *>(a.conv_b + c));
       // what the convolution sees, now and later, is the rounded input
       x = make_float4(Act<T>::round(x.x), Act<T>::round(x.y), Act<T>::round(x.z), Act<T>::round(x.w));
       T *tp = a.tail + (size_t)r * (a.taps - 1) * a.ci + c;
-      for (int j = 0; j < a.taps; ++j) {
-        const float4 w = __ldg(reinterpret_cast<const float4 *>(a.conv_w + (size_t)j * a.ci + c));
-        const float4 q = j + 1 < a.taps ? Act<T>::ld4(tp + (size_t)j * a.ci) : x;
+      auto add = [&](int j, float4 w, float4 q) {
         if (j > 0) Act<T>::st4(tp + (size_t)(j - 1) * a.ci, q);
         s.x = fmaf(w.x, q.x, s.x); s.y = fmaf(w.y, q.y, s.y); s.z = fmaf(w.z, q.z, s.z); s.w = fmaf(w.w, q.w, s.w);
+      };
+      if (short_conv) {
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j)
+          if (j < a.taps) add(j, tap[j], j + 1 < a.taps ? tail[j] : x);
+      } else {
+        for (int j = 0; j < a.taps; ++j)
+          add(j, __ldg(reinterpret_cast<const float4 *>(a.conv_w + (size_t)j * a.ci + c)), j + 1 < a.taps ? Act<T>::ld4(tp + (size_t)j * a.ci) : x);
       }
       constexpr bool EXACT = sizeof(T) == 4;
       Act<T>::st4(a.u + (size_t)r * a.ci + c, make_float4(s.x * sigmoid_t<EXACT>(s.x), s.y * sigmoid_t<EXACT>(s.y),
