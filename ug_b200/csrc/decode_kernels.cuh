@@ -271,8 +271,8 @@ constexpr int ATT_RING_BYTES = att_ring_bytes(ATT_STAGES);
 // separately, as ug-llama/src/cpu_ops.rs:73-78), rounds to bf16 (q once per CTA, 64 threads with 8 independent
 // loads each, handed to the warps' fragments through shared memory: 2.4 us against 4.8 when every warp
 // fetched and rotated all of q for itself), and -- the CTA whose slice holds the
-// new position, when `rope.append` -- writes the K / V rows of position pos into the cache before it
-// reads them back with the rest of its slice.  Same arithmetic as rope_append_kernel.
+// new position, when `rope.append` -- writes the K / V rows of position pos into the cache, and into its ring over
+// what it fetched in their place.  Same arithmetic as rope_append_kernel.
 struct AttRope {
   const float *part;
   int n_part;
@@ -327,8 +327,8 @@ decode_attention_kernel_t(const __nv_bfloat16 *q, __nv_bfloat16 *__restrict__ kc
   // written a step ago.  The caller sets it only where the position counter, too, is certainly up to date
   // (not for the first layer of a step, which follows the previous step's argmax closely).
   ugb_pdl_trigger();
-  bool dep_ready = false;
-  if (rope.part == nullptr || !rope.early) { ugb_pdl_wait(); dep_ready = true; }
+  const bool dep_ready = rope.part == nullptr || !rope.early;
+  if (dep_ready) ugb_pdl_wait();
   const int sp = blockIdx.x, n_split = gridDim.x, kvh = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -377,48 +377,14 @@ decode_attention_kernel_t(const __nv_bfloat16 *q, __nv_bfloat16 *__restrict__ kc
       if (s < rope.n_part) { a.x += p[s].x; a.y += p[s].y; a.z += p[s].z; a.w += p[s].w; }
     return a;
   };
-  // K / V rows of the new position: written by the warp that will fetch the sub-tile holding them, so
-  // that no CTA barrier is needed -- before the ring is filled when that sub-tile is part of the fill,
-  // otherwise after, with the fill's loads in flight.
-  auto append_kv = [&]() {
-    const int pos = T - 1;
-    const int kcol = (n_heads + kvh) * ATT_HD, vcol = (n_heads + n_kv + kvh) * ATT_HD;
-    __nv_bfloat16 *kd = kcache + (((size_t)b * n_kv + kvh) * t_max + pos) * ATT_HD;
-    __nv_bfloat16 *vd = vcache + (((size_t)b * n_kv + kvh) * t_max + pos) * ATT_HD;
-    if (lane < 8) {                                      // 4 rotation pairs per lane
-      const int i = lane * 4;
-      const float4 c = *reinterpret_cast<const float4 *>(rope.cos_ + (size_t)pos * half + i);
-      const float4 sn = *reinterpret_cast<const float4 *>(rope.sin_ + (size_t)pos * half + i);
-      if (rope.interleaved) {
-        const float4 u = sum4(kcol + 2 * i), w = sum4(kcol + 2 * i + 4);
-        uint4 o;
-        o.x = pack_bf16(__fsub_rn(__fmul_rn(u.x, c.x), __fmul_rn(u.y, sn.x)), __fadd_rn(__fmul_rn(u.x, sn.x), __fmul_rn(u.y, c.x)));
-        o.y = pack_bf16(__fsub_rn(__fmul_rn(u.z, c.y), __fmul_rn(u.w, sn.y)), __fadd_rn(__fmul_rn(u.z, sn.y), __fmul_rn(u.w, c.y)));
-        o.z = pack_bf16(__fsub_rn(__fmul_rn(w.x, c.z), __fmul_rn(w.y, sn.z)), __fadd_rn(__fmul_rn(w.x, sn.z), __fmul_rn(w.y, c.z)));
-        o.w = pack_bf16(__fsub_rn(__fmul_rn(w.z, c.w), __fmul_rn(w.w, sn.w)), __fadd_rn(__fmul_rn(w.z, sn.w), __fmul_rn(w.w, c.w)));
-        *reinterpret_cast<uint4 *>(kd + 2 * i) = o;
-      } else {
-        const float4 x1 = sum4(kcol + i), x2 = sum4(kcol + i + half);
-        uint2 lo, hi;
-        lo.x = pack_bf16(__fsub_rn(__fmul_rn(x1.x, c.x), __fmul_rn(x2.x, sn.x)), __fsub_rn(__fmul_rn(x1.y, c.y), __fmul_rn(x2.y, sn.y)));
-        lo.y = pack_bf16(__fsub_rn(__fmul_rn(x1.z, c.z), __fmul_rn(x2.z, sn.z)), __fsub_rn(__fmul_rn(x1.w, c.w), __fmul_rn(x2.w, sn.w)));
-        hi.x = pack_bf16(__fadd_rn(__fmul_rn(x1.x, sn.x), __fmul_rn(x2.x, c.x)), __fadd_rn(__fmul_rn(x1.y, sn.y), __fmul_rn(x2.y, c.y)));
-        hi.y = pack_bf16(__fadd_rn(__fmul_rn(x1.z, sn.z), __fmul_rn(x2.z, c.z)), __fadd_rn(__fmul_rn(x1.w, sn.w), __fmul_rn(x2.w, c.w)));
-        *reinterpret_cast<uint2 *>(kd + i) = lo;
-        *reinterpret_cast<uint2 *>(kd + i + half) = hi;
-      }
-    } else if (lane < 24) {                              // 4 v values per lane
-      const int i = (lane - 8) * 4;
-      const float4 x = sum4(vcol + i);
-      *reinterpret_cast<uint2 *>(vd + i) = make_uint2(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w));
-    }
-    __threadfence();                                     // in L2 before this warp's cp.async fetches the row
-    if (TMA) asm volatile("fence.proxy.async;" ::: "memory");   // ... or before the TMA engine reads it
-    __syncwarp();
-  };
-  const int sub_pos = (T - 1) / ATT_SUB;                 // sub-tile of the new position
-  const bool appender = rope.part != nullptr && rope.append && sub_pos >= sub_lo && sub_pos < sub_hi &&
-                        ((sub_pos - sub_lo) & (ATT_WARPS - 1)) == warp;
+  // Angles of this thread's part of q (threads 0 .. 63), of k (64 .. 71): tables, so they may be read ahead of the wait.
+  float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), sn = cs;
+  if (rope.part != nullptr && threadIdx.x < 72) {
+    const size_t at = (size_t)(T - 1) * half + 4 * (threadIdx.x & 7);
+    cs = __ldg(reinterpret_cast<const float4 *>(rope.cos_ + at));
+    sn = __ldg(reinterpret_cast<const float4 *>(rope.sin_ + at));
+  }
+  const int sub_pos = rope.part != nullptr && rope.append ? (T - 1) / ATT_SUB : -1;   // sub-tile of the new position
 
   auto issue = [&](int sub, int stage) {
     // 16 keys x 128 B for K and for V: 4 + 4 chunks of 16 B per lane, XOR-swizzled rows
@@ -451,9 +417,6 @@ decode_attention_kernel_t(const __nv_bfloat16 *q, __nv_bfloat16 *__restrict__ kc
 
   // prologue: fill the ring
   const int first = sub_lo + warp;
-  const bool append_first = appender && sub_pos < first + (NSTAGE - 1) * ATT_WARPS;
-  if (!dep_ready && append_first) { ugb_pdl_wait(); dep_ready = true; }   // the new row comes first
-  if (append_first) append_kv();
 #pragma unroll
   for (int s = 0; s < NSTAGE - 1; ++s) {
     const int sub = first + s * ATT_WARPS;
@@ -461,41 +424,42 @@ decode_attention_kernel_t(const __nv_bfloat16 *q, __nv_bfloat16 *__restrict__ kc
     cp_async_commit();
   }
   if (!dep_ready) ugb_pdl_wait();
-  if (appender && !append_first) append_kv();
+  __shared__ __align__(16) uint32_t kv_sh[2][ATT_HD / 2];    // K and V row of the new position
   if (rope.part != nullptr) {
-    // ---- q of the 8 heads, rotated: computed once per CTA (threads 0..63: one head and 8 of its dims each, all
-    // of a thread's loads requested before the first is used), rounded to bf16 and handed to the four warps
-    // through shared memory, each lane picking up the 16 dims of its fragment --------------------------------
+    // ---- q of the 8 heads and k, rotated, and v: computed once per CTA (threads 0..63: one head and 8 of its dims each, 64..71
+    // 8 dims of k, 72..87 4 of v; all of a thread's loads requested before the first is used), rounded to bf16 and handed to the
+    // four warps through shared memory, each lane picking up the 16 dims of its fragment -----------------------------------
     __shared__ __align__(16) uint32_t q_sh[ATT_GROUP][ATT_HD / 2];
-    if (threadIdx.x < 64) {
+    if (threadIdx.x < 72) {
       const int h = threadIdx.x >> 3, c = threadIdx.x & 7;
-      uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
-      if (h < group) {
-        const int pos = T - 1, qcol = (kvh * group + h) * ATT_HD;
-        const float4 cs = *reinterpret_cast<const float4 *>(rope.cos_ + (size_t)pos * half + 4 * c);
-        const float4 sn = *reinterpret_cast<const float4 *>(rope.sin_ + (size_t)pos * half + 4 * c);
+      uint32_t *dst = threadIdx.x < 64 ? q_sh[h] : kv_sh[0];
+      uint4 o = make_uint4(0, 0, 0, 0);
+      if (h < group || threadIdx.x >= 64) {
+        const int col = (threadIdx.x < 64 ? kvh * group + h : n_heads + kvh) * ATT_HD;
         if (rope.interleaved) {                              // pairs (2i, 2i + 1), i = 4c .. 4c + 3: dims 8c .. 8c + 7
-          const float4 u = sum4(qcol + 8 * c), w = sum4(qcol + 8 * c + 4);
-          lo.x = pack_bf16(__fsub_rn(__fmul_rn(u.x, cs.x), __fmul_rn(u.y, sn.x)), __fadd_rn(__fmul_rn(u.x, sn.x), __fmul_rn(u.y, cs.x)));
-          lo.y = pack_bf16(__fsub_rn(__fmul_rn(u.z, cs.y), __fmul_rn(u.w, sn.y)), __fadd_rn(__fmul_rn(u.z, sn.y), __fmul_rn(u.w, cs.y)));
-          lo.z = pack_bf16(__fsub_rn(__fmul_rn(w.x, cs.z), __fmul_rn(w.y, sn.z)), __fadd_rn(__fmul_rn(w.x, sn.z), __fmul_rn(w.y, cs.z)));
-          lo.w = pack_bf16(__fsub_rn(__fmul_rn(w.z, cs.w), __fmul_rn(w.w, sn.w)), __fadd_rn(__fmul_rn(w.z, sn.w), __fmul_rn(w.w, cs.w)));
-          *reinterpret_cast<uint4 *>(&q_sh[h][4 * c]) = lo;
+          const float4 u = sum4(col + 8 * c), w = sum4(col + 8 * c + 4);
+          o.x = pack_bf16(__fsub_rn(__fmul_rn(u.x, cs.x), __fmul_rn(u.y, sn.x)), __fadd_rn(__fmul_rn(u.x, sn.x), __fmul_rn(u.y, cs.x)));
+          o.y = pack_bf16(__fsub_rn(__fmul_rn(u.z, cs.y), __fmul_rn(u.w, sn.y)), __fadd_rn(__fmul_rn(u.z, sn.y), __fmul_rn(u.w, cs.y)));
+          o.z = pack_bf16(__fsub_rn(__fmul_rn(w.x, cs.z), __fmul_rn(w.y, sn.z)), __fadd_rn(__fmul_rn(w.x, sn.z), __fmul_rn(w.y, cs.z)));
+          o.w = pack_bf16(__fsub_rn(__fmul_rn(w.z, cs.w), __fmul_rn(w.w, sn.w)), __fadd_rn(__fmul_rn(w.z, sn.w), __fmul_rn(w.w, cs.w)));
         } else {                                             // pairs (i, i + 32), i = 4c .. 4c + 3
-          const float4 x1 = sum4(qcol + 4 * c), x2 = sum4(qcol + half + 4 * c);
-          lo.x = pack_bf16(__fsub_rn(__fmul_rn(x1.x, cs.x), __fmul_rn(x2.x, sn.x)), __fsub_rn(__fmul_rn(x1.y, cs.y), __fmul_rn(x2.y, sn.y)));
-          lo.y = pack_bf16(__fsub_rn(__fmul_rn(x1.z, cs.z), __fmul_rn(x2.z, sn.z)), __fsub_rn(__fmul_rn(x1.w, cs.w), __fmul_rn(x2.w, sn.w)));
-          hi.x = pack_bf16(__fadd_rn(__fmul_rn(x1.x, sn.x), __fmul_rn(x2.x, cs.x)), __fadd_rn(__fmul_rn(x1.y, sn.y), __fmul_rn(x2.y, cs.y)));
-          hi.y = pack_bf16(__fadd_rn(__fmul_rn(x1.z, sn.z), __fmul_rn(x2.z, cs.z)), __fadd_rn(__fmul_rn(x1.w, sn.w), __fmul_rn(x2.w, cs.w)));
-          *reinterpret_cast<uint2 *>(&q_sh[h][2 * c]) = make_uint2(lo.x, lo.y);
-          *reinterpret_cast<uint2 *>(&q_sh[h][16 + 2 * c]) = make_uint2(hi.x, hi.y);
+          const float4 x1 = sum4(col + 4 * c), x2 = sum4(col + half + 4 * c);
+          o.x = pack_bf16(__fsub_rn(__fmul_rn(x1.x, cs.x), __fmul_rn(x2.x, sn.x)), __fsub_rn(__fmul_rn(x1.y, cs.y), __fmul_rn(x2.y, sn.y)));
+          o.y = pack_bf16(__fsub_rn(__fmul_rn(x1.z, cs.z), __fmul_rn(x2.z, sn.z)), __fsub_rn(__fmul_rn(x1.w, cs.w), __fmul_rn(x2.w, sn.w)));
+          o.z = pack_bf16(__fadd_rn(__fmul_rn(x1.x, sn.x), __fmul_rn(x2.x, cs.x)), __fadd_rn(__fmul_rn(x1.y, sn.y), __fmul_rn(x2.y, cs.y)));
+          o.w = pack_bf16(__fadd_rn(__fmul_rn(x1.z, sn.z), __fmul_rn(x2.z, cs.z)), __fadd_rn(__fmul_rn(x1.w, sn.w), __fmul_rn(x2.w, cs.w)));
         }
-      } else if (rope.interleaved) {
-        *reinterpret_cast<uint4 *>(&q_sh[h][4 * c]) = lo;    // zero padding rows
-      } else {
-        *reinterpret_cast<uint2 *>(&q_sh[h][2 * c]) = make_uint2(0u, 0u);
-        *reinterpret_cast<uint2 *>(&q_sh[h][16 + 2 * c]) = make_uint2(0u, 0u);
       }
+      if (rope.interleaved) {                                // rows behind the group are zero
+        *reinterpret_cast<uint4 *>(dst + 4 * c) = o;
+      } else {
+        *reinterpret_cast<uint2 *>(dst + 2 * c) = make_uint2(o.x, o.y);
+        *reinterpret_cast<uint2 *>(dst + 16 + 2 * c) = make_uint2(o.z, o.w);
+      }
+    } else if (threadIdx.x < 88) {
+      const int i = threadIdx.x - 72;
+      const float4 x = sum4((n_heads + n_kv + kvh) * ATT_HD + 4 * i);
+      *reinterpret_cast<uint2 *>(&kv_sh[1][2 * i]) = make_uint2(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w));
     }
     __syncthreads();
     {
@@ -529,6 +493,19 @@ decode_attention_kernel_t(const __nv_bfloat16 *q, __nv_bfloat16 *__restrict__ kc
       cp_async_wait<NSTAGE - 1>();
     }
     __syncwarp();
+    if (sub == sub_pos) {
+      // The row of the new position goes over what was fetched in its place, and to the cache: through the cache alone it would
+      // be a store, a fence and a read from L2, and k and v would be formed behind q and not beside it (a step of one sequence at 300
+      // keys 845 -> 820 us, of 64 at 2048 1.52 -> 1.49 ms).
+      const int key = (T - 1) & (ATT_SUB - 1), c = lane & 7;
+      if (lane < 16) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(&kv_sh[lane >> 3][4 * c]);
+        *reinterpret_cast<uint4 *>(&ring[warp][stage][lane >> 3][key * 128 + ((c ^ (key & 7)) << 4)]) = v;
+        __nv_bfloat16 *row = (lane < 8 ? kcache : vcache) + (((size_t)b * n_kv + kvh) * t_max + T - 1) * ATT_HD;
+        *reinterpret_cast<uint4 *>(row + 8 * c) = v;
+      }
+      __syncwarp();
+    }
     const uint8_t *ks = &ring[warp][stage][0][0];
     const uint32_t vs = (uint32_t)__cvta_generic_to_shared(&ring[warp][stage][1][0]);
 
