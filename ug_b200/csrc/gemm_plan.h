@@ -77,3 +77,28 @@ inline ugb_f32_shape ugb_f32_gemm_shape(int sm_count, size_t b, size_t m, size_t
     for (int i = 1; i < 3; ++i) consider(i, true);
   return best;
 }
+
+// ---- f32 products on the tensor cores (gemm_f32_split.cu) -------------------------------------------------------------------
+// Tile width and split of k by predicted time, and whether that is less than the FFMA kernel's.  In us, fitted to 206 timed combinations of 24
+// products of 2-2048 rows (off by 11 % on average; the choice is within 7 % of the best on all): a launch, per round of tiles a fixed part and 32-k
+// stages that widen with the tile and slow down a little as more SMs are at work, and the exchange of sums.  Clusters of 4 and 8 find fewer
+// SMs: those of a cluster have to be neighbours.  Short k stays with the FFMA kernel: from k = 64 on the error is below its error
+// (6.8e-8 of the result against 8.5e-8 at 64, 1.3e-7 against 4.1e-7 at 2048), and there is nothing to gain below.
+constexpr size_t UGB_F32_SPLIT_K = 64;
+struct ugb_f32_split_plan { int bn = 0, split = 1; };          // bn 0: not on the tensor cores
+inline ugb_f32_split_plan ugb_f32_gemm_split_plan(int sm_count, size_t b, size_t m, size_t n, size_t k, bool rows_contiguous) {
+  ugb_f32_split_plan best;
+  if (k < UGB_F32_SPLIT_K || m == 0 || n == 0 || b == 0) return best;
+  if (n <= 32 && n < m) return best;       // a quarter of the 128 lanes: the FFMA kernel's turned tiles (5 of [3922, 88] x [88, 8] 14.9 us here, 11.2 there)
+  double least = ugb_f32_gemm_shape(sm_count, b, m, n, k).cost / 1900 + 2.5;
+  for (int split = 1; split <= 8 && (split == 1 || k / split >= 64); split *= 2)
+    for (int bn : {32, 64, 96, 128}) {
+      if (rows_contiguous && bn % 64 != 0) continue;
+      const size_t tiles = (n + 127) / 128 * ((m + bn - 1) / bn) * b * split, slots = std::max<size_t>(split, split <= 2 ? sm_count : sm_count * (split == 4 ? 92 : 75) / 100);
+      if (split > 1 && tiles > slots) continue;                        // several rounds are better spent on whole sums (2048 x 4096 x 2048: 282 against 270)
+      const double stages = split == 1 ? (double)((k + 31) / 32) : 2.0 * (double)(((k + split - 1) / split + 63) / 64), busy = std::min(1.0, (double)tiles / sm_count);
+      const double us = -0.2 + (double)((tiles + slots - 1) / slots) * (4.45 + stages * (0.476 + 0.004 * bn) * (0.894 + 0.106 * busy)) + (split > 1 ? 1.5 + 0.02 * bn : 0);
+      if (us < least) { least = us; best = {bn, split}; }
+    }
+  return best;
+}

@@ -6,9 +6,9 @@
 // layout rules pick between
 //   * the tcgen05 / TMEM tensor-core kernel (bf16 operands, fp32 accumulate),
 //     declared in gemm_tcgen05.cuh, and
-//   * for f32 (the dtype ug-llama casts every weight to, model.rs:118,140,313) two FP32-pipe kernels: a
+//   * for f32 (the dtype ug-llama casts every weight to, model.rs:118,140,313) two FP32-pipe kernels, a
 //     warp-per-column streaming kernel for the skinny products of a decode step and a register-blocked FFMA kernel
-//     for the rest, and
+//     for short k, and for the rest the tensor cores on three bf16 parts of every value (gemm_f32_split.cu), and
 //   * the same FFMA kernel on 16-bit operands for the shapes and layouts the tensor-core kernels do not take.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "gemm_f32_split.cuh"
 #include "gemm_plan.h"
 #include "gemm_skinny.cuh"
 #include "gemm_tcgen05.cuh"
@@ -453,6 +454,14 @@ int32_t launch_f32_shape(ugb_device *dev, const F32Params &p, size_t b, bool pdl
 
 template <typename E, bool VEC>
 int32_t launch_f32_tile(ugb_device *dev, F32Params p, size_t b, bool pdl) {
+  if constexpr (sizeof(E) == 4) {
+    const ugb_f32_split_plan s = ugb_f32_gemm_split_plan(dev->sm_count, b, p.m, p.n, p.k, p.a_cs != 1);
+    if (s.bn) {
+      const ugb_f32_split_args g{(float *)p.c, (const float *)p.b, (const float *)p.a, b, (size_t)p.n, (size_t)p.m, (size_t)p.k, p.b_cs, p.b_rs, p.b_b, p.a_rs, p.a_cs, p.a_b, p.c_rs, p.c_b, pdl};
+      const int32_t rc = ugb_f32_split(dev, g, s.bn, s.split);
+      if (rc != UGB_ERR_UNSUPPORTED) return rc;
+    }
+  }
   UGB_REQUIRE(dev, b <= 65535 && ((size_t)p.m + 127) / 128 <= 65535, UGB_ERR_UNSUPPORTED, "matmul: m or batch too large for the FP32-pipe kernel");
   if (p.k <= SHORT_K && (p.m + 63) / 64 <= 65535 && (sizeof(E) == 2 || b * (size_t)p.m * (size_t)p.n <= (VEC ? SHORT_K_F32_VEC_RESULTS : SHORT_K_F32_RESULTS))) {
     const cudaError_t e = ugb_launch(short_k_kernel<E>, dim3((unsigned)((p.n + 63) / 64), (unsigned)((p.m + 63) / 64), (unsigned)b), dim3(256), 0, dev->stream, pdl, p);

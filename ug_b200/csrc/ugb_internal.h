@@ -31,6 +31,7 @@ struct ugb_device {
   std::string last_error;
   void *gemm_state = nullptr;  // owned by the GEMM translation unit
   unsigned f32_smem_set = 0;   // instances of f32_tile_kernel whose shared memory has been asked for (matmul.cu)
+  unsigned long long f32_split_smem_set = 0;   // the same of f32_split_kernel (gemm_f32_split.cu)
   int gemm_pair = 1;           // option gemm_cta_pairs: tall bf16 GEMMs on pairs of CTAs (tcgen05 cta_group::2)
   cudaMemPool_t pool = nullptr;  // this handle's own stream-ordered pool (the process-wide default pool is left alone)
   unsigned wait_timeouts = 0;  // device-side waits that gave up, as seen by ugb_sync (tensor-parallel models refuse
