@@ -171,6 +171,28 @@ def test_wide_steps(dev, batch):
     m.close()
 
 
+@pytest.mark.parametrize("width,ffn,batch", [(264, 72, 1), (1024, 136, 8), (1544, 72, 8), (2112, 264, 3), (1024, None, 2)])
+def test_steps_that_run_ahead(dev, width, ffn, batch):
+    """Products, attention and experts' rows that run beside the kernels before them (up to two chunks of k with a warp that waits for
+    them, more chunks, k in several pieces, no shared feed-forward) give what they give one behind the other, bit by bit: where a
+    kernel waits changes no operand and no order of a sum."""
+    cfg = Config(vocab=64, width=width, eps=1e-5, layers=[
+        layer((4, 2, 64, 64, 64, 5000.0, 0.3), (256, 16, 4, 32), Experts(16, 2, 40, ffn)), layer((8, 2, 64, 64, 32, 900.0, 0.3), (1032, 8, 3, 16), 200)])
+    w = separate_experts(cfg, synth.zidevik_weights(cfg, 502))
+    rows, got = synth.tokens(78, (batch, 40), cfg.vocab), []
+    for pdl in (0, 1):
+        m = Model.new(cfg, w, dev, batch, 64, DType.BF16)
+        m.set_option("pdl", pdl)
+        m.set_option("att_splits", 2)
+        m.prefill(rows[:, :30])
+        got.append([])
+        for i in range(30, 40):
+            m.fwd(rows[:, i])
+            got[-1].append(m.logits())
+        m.close()
+    assert np.isfinite(got[0]).all() and np.array_equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("dtype", BOTH)
 @pytest.mark.parametrize("name", ["mixed", "odd"])
 def test_sequences_follow_one_another(make, name, dtype):

@@ -23,7 +23,7 @@
 // what the stages leave of 256 KB: 32 k a stage, not 64.  The fence between the planes and the tensor core is that of shared memory
 // alone: the general one also waits for the loads ahead (86 -> 59 us on the first of these).  8 warps with twice the work each 68 us there
 // against 56, three stages ahead 61, lines asked into the L2 six stages ahead 59.
-// Against the FFMA kernel: [257, 2048] x [5632, 2048]^T 184 -> 56 us (70 with the matrix from HBM), [2048, 2048] x [4096, 2048]^T 680 -> 270, [777, 5632] x
+// Against the FFMA kernel: [257, 2048] x [5632, 2048]^T 182 -> 56 us (70 with the matrix from HBM), [2048, 2048] x [4096, 2048]^T 680 -> 298, [777, 5632] x
 // [2048, 5632]^T 481 -> 165, [128, 2048] x [2048, 2048]^T 56 -> 18, [500, 999] x [1001, 999]^T 34 -> 19.  Values that send a tile to FFMA: up to
 // four times the FFMA kernel's time.
 #include "gemm_f32_split.cuh"

@@ -70,11 +70,13 @@ template <bool F16> static __device__ __forceinline__ void store16(void *out, lo
 // Activations k .. k + 7 of row r, formed from the product before: gelu_tanh(sum of its partials) * the row's token in the table,
 // rounded to bf16.  Every CTA does it again for all of its k (2048 values of 1024 bytes of partials and table each); what it
 // saves is a kernel between two products of 1 MB (Zidevik, 8 sequences: 28 of them a step, request of 32 steps 96.4 -> 95.0 ms).
-static __device__ __forceinline__ uint4 gated_act(const ugb_skinny_gate &q, int r, int k) {
-  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+static __device__ __forceinline__ uint4 gate_entry(const ugb_skinny_gate &q, int r, int k) {
   const int id = q.tok[r];
-  uint4 e = make_uint4(0, 0, 0, 0);
-  if (id >= 0 && id < q.vocab) e = __ldg(reinterpret_cast<const uint4 *>(q.table + (size_t)id * q.table_ld + q.off + k));
+  return id >= 0 && id < q.vocab ? __ldg(reinterpret_cast<const uint4 *>(q.table + (size_t)id * q.table_ld + q.off + k)) : make_uint4(0, 0, 0, 0);
+}
+// `e`: the table's values, asked for ahead of the wait: the token is the step's own, and its row comes from HBM.
+static __device__ __forceinline__ uint4 gated_act(const ugb_skinny_gate &q, int r, int k, uint4 e) {
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const float *row = q.part + (size_t)r * q.ld + k;
   for (int p = 0; p < q.n_part; p += 4) {  // the partials are added in order
     float4 v[4][2];
@@ -100,8 +102,10 @@ static __device__ __forceinline__ uint4 gated_act(const ugb_skinny_gate &q, int 
 }
 
 // KC: chunks of a warp per piece; a unit whose split is longer runs in p.spans pieces.  FIXED: no kernel of the stream writes W.
-template <int KC, bool F16, bool FIXED, bool GATE = false>
-__global__ void __launch_bounds__(THREADS, 2)
+// AHEAD: see ugb_tc_gemm_args::a_ahead.  Up to two chunks leave registers for a ninth warp, which waits and then lets the next kernel in;
+// with more chunks the CTA does so behind its first unit.
+template <int KC, bool F16, bool FIXED, bool GATE = false, bool AHEAD = false>
+__global__ void __launch_bounds__(AHEAD && KC <= 2 ? THREADS + 32 : THREADS, 2)
 skinny_gemm_kernel(const Params p) {
   __shared__ float red[2][WARPS][8 * RED_LD];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -119,6 +123,11 @@ skinny_gemm_kernel(const Params p) {
   }
   if (!p.late_trigger) ugb_pdl_trigger();
   if (p.wait_first) ugb_pdl_wait();
+  if (AHEAD && KC <= 2 && warp == WARPS) {
+    ugb_pdl_wait();
+    ugb_pdl_trigger();
+    return;
+  }
   const int u1 = (int)((long long)(blockIdx.x + 1) * units / gridDim.x);
   int u = (int)((long long)blockIdx.x * units / gridDim.x), s = 0;
 
@@ -156,7 +165,15 @@ skinny_gemm_kernel(const Params p) {
 #pragma unroll
     for (int i = 0; i < KC; ++i) load(i);
   }
-  if (!p.groups) {
+  uint4 entry[2] = {};
+  if constexpr (GATE) {                    // all of k is one piece
+    if (u < u1 && g < p.rows)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (warp * CHUNK + 32 * h + 8 * t < p.k) entry[h] = gate_entry(p.gate, g, warp * CHUNK + 32 * h + 8 * t);
+  }
+  bool waits = AHEAD && KC > 2 && u < u1;
+  if (!p.groups && !(AHEAD && KC <= 2) && !waits) {
     ugb_pdl_wait();
     if (p.late_trigger) ugb_pdl_trigger();
   }
@@ -176,8 +193,8 @@ skinny_gemm_kernel(const Params p) {
         const int c = lc + i * WARPS, k = c * CHUNK + 8 * t;
         const bool on = g < p.rows && c < lc1;
         if constexpr (GATE) {
-          act[i][0] = on && k < p.k ? gated_act(p.gate, g, k) : make_uint4(0, 0, 0, 0);
-          act[i][1] = on && k + 32 < p.k ? gated_act(p.gate, g, k + 32) : make_uint4(0, 0, 0, 0);
+          act[i][0] = on && k < p.k ? gated_act(p.gate, g, k, entry[0]) : make_uint4(0, 0, 0, 0);
+          act[i][1] = on && k + 32 < p.k ? gated_act(p.gate, g, k + 32, entry[1]) : make_uint4(0, 0, 0, 0);
           continue;
         }
         act[i][0] = on && k < p.k ? __ldcg(reinterpret_cast<const uint4 *>(row + 2 * (size_t)k)) : make_uint4(0, 0, 0, 0);
@@ -202,7 +219,7 @@ skinny_gemm_kernel(const Params p) {
       c0[0] = acc[0]; c1[0] = acc[1]; c0[8] = acc[2]; c1[8] = acc[3];
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[e] = 0.f;
-      __syncthreads();                     // one per unit: the other buffer's readers have passed it before it is written again
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // one per unit: the other buffer's readers have passed it before it is written again
       if (threadIdx.x < 128) {
         const int r = threadIdx.x >> 4, e = threadIdx.x & 15;
         float v = 0.f;
@@ -222,6 +239,11 @@ skinny_gemm_kernel(const Params p) {
         }
       }
       buf ^= 1;
+      if (waits) {
+        ugb_pdl_wait();
+        ugb_pdl_trigger();
+        waits = false;
+      }
     }
     if (!more) return;
     u = nu; s = ns;
@@ -293,6 +315,7 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
   p.epi = g.epi;
   p.late_trigger = g.late_trigger ? 1 : 0;
   p.wait_first = !g.b_static && !g.groups ? 1 : 0;
+  const bool ahead = g.a_ahead && g.b_static && !g.groups && !gate && g.late_trigger && g.pdl && !g.f16;
   p.groups = g.groups; p.tile_m = g.tile_m;
   p.n_groups_tiles = g.groups ? (int)(g.m / g.tile_m) : 0;
   const long long units = (long long)p.tiles * (g.groups ? p.n_groups_tiles : (long long)p.splits * (long long)g.batch);
@@ -303,7 +326,8 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
   const unsigned grid = (unsigned)((units + rounds - 1) / rounds);
   cudaError_t e = cudaErrorInvalidValue;
 #define UGB_SKINNY(KC) \
-  e = g.f16          ? ugb_launch(skinny_gemm_kernel<KC, true, false>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p) \
+  e = ahead          ? ugb_launch(skinny_gemm_kernel<KC, false, true, false, true>, dim3(grid), dim3(KC <= 2 ? THREADS + 32 : THREADS), 0, dev->stream, g.pdl, p) \
+      : g.f16        ? ugb_launch(skinny_gemm_kernel<KC, true, false>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p) \
       : p.wait_first ? ugb_launch(skinny_gemm_kernel<KC, false, false>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p) \
                      : ugb_launch(skinny_gemm_kernel<KC, false, true>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p)
   if (gate) e = ugb_launch(skinny_gemm_kernel<1, false, true, true>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p);

@@ -51,6 +51,9 @@ struct ugb_tc_gemm_args {
                                // of a stream whose kernels all do so may read what the kernels before its predecessor wrote
                                // ahead of its own wait
   int smem_kib = 0;     // cap on the shared memory of a CTA (ring depth follows); 0 = as deep as fits in 220 KiB
+  // Few rows, with b_static and late_trigger: A was written by kernels before the predecessor, and the predecessor neither reads nor
+  // writes `out`.  In a stream whose kernels all trigger late the product may then run beside its predecessor: only its end waits.
+  bool a_ahead = false;
   bool f16 = false;     // operands (and the UGB_EPI_BF16 output) are IEEE f16 instead of bf16: same instruction, other format field
   bool pair_k = false;  // m <= 64, an epilogue that writes bf16 columns: two CTAs (a thread-block cluster) per tile, each over half of k; the
                         // second hands its sums to the first through distributed shared memory.  UGB_ERR_UNSUPPORTED when

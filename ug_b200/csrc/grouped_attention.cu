@@ -64,15 +64,18 @@ grouped_attention_mma_kernel(Params p) {
   extern __shared__ __align__(128) uint8_t ring[];
   __shared__ float2 wml[WARPS][16];                        // (max, sum) of a warp per head
   __shared__ float2 ml[16];                                // of this slice
-  __shared__ float fac[16][UGB_GROUPED_MAX_SPLITS];        // weight of a slice's sums, 1 / sum included
-  if (!p.early) { ugb_pdl_wait(); ugb_pdl_trigger(); }
+  // early: queries and cache were written by kernels before the predecessor, so the whole of it runs beside that kernel and only the
+  // results wait.  The next kernel is let in at once: when this one runs, everything up to the predecessor's predecessor is complete,
+  // which is all that a product may read ahead of its own wait, and that wait covers this kernel's, the predecessor included.
+  if (!p.early) ugb_pdl_wait();
+  ugb_pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
   const int share = p.heads / p.kv_heads, per_kv = (share + 15) / 16;
   const int sp = blockIdx.x, kvh = blockIdx.y / per_kv, hg = blockIdx.y % per_kv, r = blockIdx.z, b = r / p.t;
   const int head0 = kvh * share + hg * 16, n_heads = min(16, share - hg * 16);
   const int T = keys_of(p, r);
   if (T == 0) {                                            // the whole cluster leaves
-    if (p.early) { ugb_pdl_wait(); ugb_pdl_trigger(); }
+    if (p.early) ugb_pdl_wait();
     return;
   }
   const int n_sub = (T + KT - 1) / KT, per = (n_sub + p.splits - 1) / p.splits;
@@ -113,8 +116,6 @@ grouped_attention_mma_kernel(Params p) {
       qa[k][3] = ld2(g + 8, 16 * k + 8 + 2 * tq);
     }
   }
-  if (p.early) { ugb_pdl_wait(); ugb_pdl_trigger(); }
-
   const float scl = p.scale * 1.4426950408889634f;
   const int mi = lane >> 3, ri = lane & 7;
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};  // of heads g and g + 8; l: this lane's keys
@@ -197,6 +198,7 @@ grouped_attention_mma_kernel(Params p) {
       *reinterpret_cast<float2 *>(wo + (warp * 16 + g + 8 * h) * DV + 8 * d + 2 * tq) = make_float2(o[d][2 * h], o[d][2 * h + 1]);
   __syncthreads();
   __nv_bfloat16 *out = (__nv_bfloat16 *)p.out + (size_t)r * p.out_ld + (size_t)head0 * DV;
+  if (p.early && p.splits == 1) ugb_pdl_wait();
   for (int idx = threadIdx.x; idx < n_heads * (DV / 4); idx += WARPS * 32) {
     const int h = idx / (DV / 4), c = 4 * (idx % (DV / 4));
     float mm = -INFINITY, ll = 0.f;
@@ -223,42 +225,34 @@ grouped_attention_mma_kernel(Params p) {
   // The slices of a row are the CTAs of one cluster: after one barrier each combines its share of the elements, in slice
   // order, reading the peers' shared memory.
   cluster_sync_all();
-  if (threadIdx.x < n_heads) {
-    const int h = threadIdx.x;
-    const uint32_t addr = smem_u32(&ml[h]);
-    float2 v[UGB_GROUPED_MAX_SPLITS];
+  if (p.early) ugb_pdl_wait();
+  for (int idx = sp * (WARPS * 32) + threadIdx.x; idx < n_heads * (DV / 4); idx += p.splits * (WARPS * 32)) {
+    const int h = idx / (DV / 4), c = 4 * (idx % (DV / 4));
+    const uint32_t at = smem_u32(co + h * DV + c), at_ml = smem_u32(&ml[h]);
+    float4 v[UGB_GROUPED_MAX_SPLITS], acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float2 w[UGB_GROUPED_MAX_SPLITS];                      // (max, sum) of a slice; all that is remote is asked for at once
     float mm = -INFINITY, ll = 0.f;
 #pragma unroll
     for (int s = 0; s < UGB_GROUPED_MAX_SPLITS; ++s) {
-      v[s] = make_float2(-INFINITY, 0.f);
-      if (s < p.splits)
-        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v[s].x), "=f"(v[s].y) : "r"(mapa_u32(addr, (uint32_t)s)) : "memory");
-    }
-#pragma unroll
-    for (int s = 0; s < UGB_GROUPED_MAX_SPLITS; ++s) mm = fmaxf(mm, v[s].x);
-#pragma unroll
-    for (int s = 0; s < UGB_GROUPED_MAX_SPLITS; ++s) {
-      v[s].x = v[s].x == -INFINITY ? 0.f : ex2(v[s].x - mm);
-      ll = fmaf(v[s].x, v[s].y, ll);
-    }
-#pragma unroll
-    for (int s = 0; s < UGB_GROUPED_MAX_SPLITS; ++s) fac[h][s] = v[s].x * (p.out_scale / ll);
-  }
-  __syncthreads();
-  for (int idx = sp * (WARPS * 32) + threadIdx.x; idx < n_heads * (DV / 4); idx += p.splits * (WARPS * 32)) {
-    const int h = idx / (DV / 4), c = 4 * (idx % (DV / 4));
-    const uint32_t addr = smem_u32(co + h * DV + c);
-    float4 v[UGB_GROUPED_MAX_SPLITS], acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int s = 0; s < UGB_GROUPED_MAX_SPLITS; ++s) {
       v[s] = acc;
-      if (s < p.splits)
+      w[s] = make_float2(-INFINITY, 0.f);
+      if (s < p.splits) {
+        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(w[s].x), "=f"(w[s].y) : "r"(mapa_u32(at_ml, (uint32_t)s)) : "memory");
         asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(v[s].x), "=f"(v[s].y), "=f"(v[s].z), "=f"(v[s].w) : "r"(mapa_u32(addr, (uint32_t)s)) : "memory");
+                     : "=f"(v[s].x), "=f"(v[s].y), "=f"(v[s].z), "=f"(v[s].w) : "r"(mapa_u32(at, (uint32_t)s)) : "memory");
+      }
     }
 #pragma unroll
+    for (int s = 0; s < UGB_GROUPED_MAX_SPLITS; ++s) mm = fmaxf(mm, w[s].x);
+#pragma unroll
     for (int s = 0; s < UGB_GROUPED_MAX_SPLITS; ++s) {
-      const float f = s < p.splits ? fac[h][s] : 0.f;
+      w[s].x = w[s].x == -INFINITY ? 0.f : ex2(w[s].x - mm);
+      ll = fmaf(w[s].x, w[s].y, ll);
+    }
+    const float scale = p.out_scale / ll;
+#pragma unroll
+    for (int s = 0; s < UGB_GROUPED_MAX_SPLITS; ++s) {
+      const float f = w[s].x * scale;
       acc.x = fmaf(f, v[s].x, acc.x); acc.y = fmaf(f, v[s].y, acc.y); acc.z = fmaf(f, v[s].z, acc.z); acc.w = fmaf(f, v[s].w, acc.w);
     }
     *reinterpret_cast<uint2 *>(out + (size_t)h * DV + c) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));

@@ -76,6 +76,7 @@ int32_t ugb_hybrid_matmul(ugb_hybrid *m, const Mat &x) {
   g.epi = x.relu2 ? UGB_EPI_RELU2_BF16 : x.silu_mul ? UGB_EPI_SILU_MUL_BF16 : (x.f32_out ? UGB_EPI_F32 : UGB_EPI_BF16);
   if (x.silu_mul) g.c_ld = x.c_ld == x.n / 2 ? 0 : (long long)x.c_ld;
   g.splits = x.splits; g.bn = x.bn; g.b_static = x.groups == nullptr; g.pdl = m->pdl != 0; g.late_trigger = true;
+  g.a_ahead = x.ahead;
   g.groups = x.groups; g.n_groups = x.n_groups; g.tile_m = x.tile;
   if (ugb_skinny_rows(x.groups ? (size_t)x.tile_rows : x.m)) {
     const int32_t rc = ugb_skinny_gemm(dev, g, x.tile_rows, x.gate);

@@ -81,6 +81,7 @@ struct ugb_hybrid_mat {            // out[b, m, n] = a . w
   int tile = 0, n_groups = 0;
   int tile_rows = 0;               // rows of a tile that may hold something (0: all)
   int splits = 1, bn = 0;
+  bool ahead = false;              // see ugb_tc_gemm_args::a_ahead
   const ugb_skinny_gate *gate = nullptr;   // up to 8 rows: activations formed inside the product (see gemm_skinny.cuh)
 };
 

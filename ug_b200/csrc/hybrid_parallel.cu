@@ -13,7 +13,7 @@
 //   [experts]  blocks: GEMM router, route;  expert_rows (rows by expert, times their weight);  grouped GEMMs up and down
 //   GEMM cat -> f32                                     output projections of mixer and feed-forward as one product
 //   row_update      stream += product + experts' rows;  copy -> T (token input or loop) or norm -> h
-//   (a step runs feed-forward and experts ahead of the scan, see run())
+//   (a step runs feed-forward, experts and attention ahead of the scan, see run())
 //   [token input]  GEMM gate;  token_gate (a step of few rows: inside proj);  GEMM proj -> f32;  row_update  stream += norm(product);  copy or norm
 // The factors of attention and scan are applied where their f32 results are rounded to T.  Products with a f32 result are
 // split over k in a step; the consumer sums the partials.
@@ -100,6 +100,9 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
   // In a bf16 decode step every kernel lets its successor start only after its own wait: when a kernel starts, everything up
   // to its predecessor's predecessor is complete (see row_update_kernel).
   const bool early = decode && pdl && !m->f32;
+  // What does not depend on its predecessor runs beside it, and only its end waits: the gate | up product beside mixer_inputs
+  // and the scan's input product beside attention or the experts' last product (a_ahead, up to 8 rows), attention beside the gate | up
+  // product, the experts' rows beside both (request 8x512+32: 94.3 -> 88.0 ms).
   const int B = m->batch, rows = B * t, wl = m->wl, n_runs = (int)m->runs.size();
   const bool whole = m->only == UGB_HYBRID_K_ALL;            // kernels timed alone leave the counts of the last whole pass as they are
   const bool looped = m->cfg.loop_times > 0, side = m->cfg.side_dim > 0;
@@ -186,13 +189,35 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
     }
 
     const size_t n_cat = L.n_cat(), cat_s = (size_t)d.heads * L.vp, cat_f = cat_s + L.ci;
+    // ---- attention
+    const bool beside = early && whole && L.fl > 0;        // a product lies between mixer_inputs and what follows it
+    auto attention = [&]() -> int32_t {
+      if (!m->on(UGB_HYBRID_K_ATTENTION)) return UGB_OK;
+      if (!decode && L.expand && t > m->absorb_max) {
+        ugb_prefill_attention_args a;
+        a.q = (const __nv_bfloat16 *)w.q; a.k = (const __nv_bfloat16 *)R.cache; a.v = (const __nv_bfloat16 *)R.vcache;
+        a.out = (__nv_bfloat16 *)w.cat; a.out_ld = (long long)n_cat; a.out_scale = d.attention_scale;
+        a.batch = B; a.t = t; a.pos0 = m->host_pos + off; a.n_heads = d.heads; a.n_kv = d.kv_heads; a.kv_rows = m->t_max;
+        a.dq = L.dp; a.dv = L.vp; a.scale = d.scale;
+        return ugb_prefill_attention_tc(dev, a);
+      } else {
+        ugb_grouped_attention_args a{};
+        a.f32 = m->f32; a.q = w.q; a.k = R.cache; a.v = R.vcache; a.out = w.cat; a.out_ld = n_cat; a.out_scale = d.attention_scale;
+        a.rows = rows; a.t = t; a.pos_p = m->pos; a.pos_off = off; a.heads = d.heads; a.kv_heads = d.kv_heads; a.dq = L.dp; a.dv = L.vp;
+        a.t_max = m->t_max; a.scale = d.scale; a.pdl = pdl; a.early = beside;
+        a.splits = m->att_splits_opt > 0 ? std::min(m->att_splits_opt, UGB_GROUPED_MAX_SPLITS) : ugb_grouped_attention_splits(a, dev->sm_count);
+        return ugb_grouped_attention(dev, a);
+      }
+    };
     // ---- feed-forward
     auto feed_forward = [&]() -> int32_t {
       if (L.fl && m->on(UGB_HYBRID_K_UP)) {
         Mat g{(T *)w.cat + cat_f, w.h, L.w_up, (size_t)rows, 2 * (size_t)L.fl, (size_t)wl};
         g.c_ld = n_cat;
+        g.ahead = early && whole;
         if ((rc = gated_product(m, w, g))) return rc;
       }
+      if (decode && (rc = attention())) return rc;
       if (experts) {
         const int tile = w.tile, tiles = group_tiles((size_t)rows * d.top, d.experts, tile);
         const size_t xrows = (size_t)tiles * tile;
@@ -206,7 +231,7 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
             route_kernel<<<(rows + ROUTE_ROWS - 1) / ROUTE_ROWS, 256, 0, dev->stream>>>(w.part, g.splits, L.ep, rows, d.experts, d.top, w.choice, w.count);
             if ((rc = ugb_after_launch(dev, "route_kernel"))) return rc;
           }
-          e = ugb_launch(expert_rows_kernel<T>, dim3(rows), dim3(256), 0, dev->stream, pdl, (const T *)w.h, w.choice, w.count, d.experts, d.top, tile, tiles,
+          e = ugb_launch(expert_rows_kernel<T>, dim3(rows), dim3(beside ? 288 : 256), 0, dev->stream, pdl, (const T *)w.h, w.choice, w.count, d.experts, d.top, tile, tiles,
                          (T *)w.xin, w.slot, w.map, wl);
           if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of expert_rows_kernel failed: %s", cudaGetErrorString(e));
           if ((rc = ugb_after_launch(dev, "expert_rows_kernel"))) return rc;
@@ -221,8 +246,8 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
       }
       return UGB_OK;
     };
-    // A step does it here: its first product requests weights while the mixer's inputs are formed, and the output product while
-    // attention runs; products one behind the other have no such time to use (request 8x512+32: 99.5 -> 96.4 ms).
+    // A step does it here: its first product runs while the mixer's inputs are formed and attention behind it; products one behind the
+    // other have no such time to use (request 8x512+32: 99.5 -> 96.4 ms before anything ran ahead).
     if (decode && (rc = feed_forward())) return rc;
 
     // ---- scan
@@ -232,6 +257,7 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
       const bool sum = !decode && x_t.splits > 1;            // a block's split product is summed and rounded to T
       Mat g{sum ? (void *)w.part : w.xdb, w.hc, L.w_x, (size_t)rows, (size_t)xr, (size_t)L.ci};
       g.splits = x_t.splits; g.bn = sum ? 256 : x_t.bn; g.f32_out = decode || m->f32 || sum;
+      g.ahead = beside;
       if ((rc = ugb_hybrid_matmul(m, g))) return rc;
       if (sum) {
         const size_t n4 = (size_t)rows * xr / 4;
@@ -256,25 +282,7 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
       if (rc) return rc;
     }
 
-    // ---- attention
-    if (m->on(UGB_HYBRID_K_ATTENTION)) {
-      if (!decode && L.expand && t > m->absorb_max) {
-        ugb_prefill_attention_args a;
-        a.q = (const __nv_bfloat16 *)w.q; a.k = (const __nv_bfloat16 *)R.cache; a.v = (const __nv_bfloat16 *)R.vcache;
-        a.out = (__nv_bfloat16 *)w.cat; a.out_ld = (long long)n_cat; a.out_scale = d.attention_scale;
-        a.batch = B; a.t = t; a.pos0 = m->host_pos + off; a.n_heads = d.heads; a.n_kv = d.kv_heads; a.kv_rows = m->t_max;
-        a.dq = L.dp; a.dv = L.vp; a.scale = d.scale;
-        if ((rc = ugb_prefill_attention_tc(dev, a))) return rc;
-      } else {
-        ugb_grouped_attention_args a{};
-        a.f32 = m->f32; a.q = w.q; a.k = R.cache; a.v = R.vcache; a.out = w.cat; a.out_ld = n_cat; a.out_scale = d.attention_scale;
-        a.rows = rows; a.t = t; a.pos_p = m->pos; a.pos_off = off; a.heads = d.heads; a.kv_heads = d.kv_heads; a.dq = L.dp; a.dv = L.vp;
-        a.t_max = m->t_max; a.scale = d.scale; a.pdl = pdl; a.early = early;
-        a.splits = m->att_splits_opt > 0 ? std::min(m->att_splits_opt, UGB_GROUPED_MAX_SPLITS) : ugb_grouped_attention_splits(a, dev->sm_count);
-        if ((rc = ugb_grouped_attention(dev, a))) return rc;
-      }
-    }
-
+    if (!decode && (rc = attention())) return rc;
     if (!decode && (rc = feed_forward())) return rc;
 
     // ---- output projections, residual

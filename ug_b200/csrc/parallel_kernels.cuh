@@ -249,9 +249,18 @@ mixer_inputs_kernel(MixerIn<TI, T> a, int rows) {
         if (e < a.experts)
           for (int p = 0; p < a.n_part; ++p) z[j] += (float)row[(size_t)p * a.part_stride + x0 + 2 * a.ci + e];
       }
+      // lane k mod 32 keeps the choice, so that the counters' answers are waited for together
+      int own = 0, own_e = -1;
+      float own_z = 0.f;
+      auto put = [&]() {
+        if (own_e >= 0) a.choice[(size_t)r * a.top + own] = make_float4(__int_as_float(own_e), __int_as_float(atomicAdd(a.count + own_e, 1)), sigmoid_f(own_z), 0.f);
+        own_e = -1;
+      };
       top_experts(z, a.experts, a.top, [&](int k, int e, float zk) {
-        if (lane == 0) a.choice[(size_t)r * a.top + k] = make_float4(__int_as_float(e), __int_as_float(atomicAdd(a.count + e, 1)), sigmoid_f(zk), 0.f);
+        if ((k & 31) == lane) { own = k; own_e = e; own_z = zk; }
+        if ((k & 31) == 31) put();
       });
+      put();
     }
   }
 }
@@ -292,15 +301,19 @@ route_kernel(const float *__restrict__ logits, int n_part, int ld, int rows, int
 
 // Lays the chosen rows out by expert: expert e has ceil(count[e] / tile) tiles of `tile` rows, one after the other.
 //   x[row of (r, k)] = weight h[r]    slot[r][k] = that row    map[i] = expert of tile i, -1 behind the last
-// One CTA per token row.
+// One CTA of 256 threads per token row.  With 32 more it runs beside its predecessor, which then neither writes what this kernel reads nor
+// touches what it writes: the ninth warp waits, so that the end of the kernel does.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(288)
 expert_rows_kernel(const T *h, const float4 *choice, const int *count, int experts, int top,
                    int tile, int tiles, T *__restrict__ x, int *__restrict__ slot, int *__restrict__ map, int ld) {
   __shared__ int first[32 * ROUTER_PER_LANE + 1];          // first tile of every expert
   const int r = blockIdx.x, lane = threadIdx.x & 31;
-  ugb_pdl_wait();
-  ugb_pdl_trigger();
+  if (blockDim.x == 256 || threadIdx.x >= 256) {
+    ugb_pdl_wait();
+    ugb_pdl_trigger();
+    if (threadIdx.x >= 256) return;
+  }
   if (threadIdx.x < 32) {
     int carry = 0;
     for (int e0 = 0; e0 < experts; e0 += 32) {
@@ -315,7 +328,7 @@ expert_rows_kernel(const T *h, const float4 *choice, const int *count, int exper
     }
     if (lane == 0) first[experts] = carry;
   }
-  __syncthreads();
+  asm volatile("bar.sync 1, 256;" ::: "memory");
   if (r == 0) {
     for (int i = threadIdx.x; i < tiles; i += 256) {
       int e = -1;
