@@ -250,9 +250,17 @@ skinny_gemm_kernel(const Params p) {
   }
 }
 
-// One CTA per SM leaves the registers for the next kernel's first weights; up to a third more CTAs than SMs, so that every
-// CTA has the same number of units (their loads share the bandwidth, not an SM).  Live groups are known on the device only.
-long long most_ctas(int sm_count, bool groups) { return groups ? (long long)sm_count * 2 : (long long)sm_count * 4 / 3; }
+// Two CTAs per SM at most, all with the same number of units where that comes out: what bounds the stream is how much of it is in flight
+// (a step of Llama, one sequence, with up to 1.33, 1.5 and 2 CTAs per SM: 822, 822, 792 us; with one 901).
+//
+// Loads into registers wait for their data in the L1, which is what a launch leaves of an SM's 256 KB as shared memory.  A chain whose
+// kernels want different splits pays for it twice: with much shared memory the L1 holds less than two CTAs have in flight, and an SM
+// changes the split only when it is empty, so that a kernel that needs more than there is cannot start beside this one.  64 KB hold this
+// kernel's sums and a CTA of attention beside them (the same step without a preference 792 us, with 32, 64 and 100 KB 726, 724 and 723, with
+// next to none 943).
+constexpr size_t CARVEOUT_BYTES = 64 * 1024;
+// CTAs that a product may have so that it still counts as one round (ugb_skinny_one_round).
+long long round_ctas(int sm_count) { return (long long)sm_count * 4 / 3; }
 
 int chunks_of(size_t k) { return (int)((k + CHUNK - 1) / CHUNK); }
 
@@ -265,7 +273,7 @@ int ugb_skinny_effective_splits(size_t k, int splits) {
   return (chunks + per - 1) / per;
 }
 
-bool ugb_skinny_one_round(int sm_count, size_t n, size_t batch) { return (n + TILE_N - 1) / TILE_N * batch <= (size_t)most_ctas(sm_count, false); }
+bool ugb_skinny_one_round(int sm_count, size_t n, size_t batch) { return (n + TILE_N - 1) / TILE_N * batch <= (size_t)round_ctas(sm_count); }
 
 int ugb_skinny_splits(int sm_count, size_t n, size_t k) {
   const int chunks = chunks_of(k), tiles = (int)((n + TILE_N - 1) / TILE_N);
@@ -321,16 +329,17 @@ int32_t ugb_skinny_gemm(ugb_device *dev, const ugb_tc_gemm_args &args, int rows_
   const long long units = (long long)p.tiles * (g.groups ? p.n_groups_tiles : (long long)p.splits * (long long)g.batch);
   if (units > (1ll << 30)) return UGB_ERR_UNSUPPORTED;
   p.units = (int)units;
-  const long long most = most_ctas(dev->sm_count, g.groups != nullptr);
+  const ugb_launch_form form{g.pdl, 1, ugb_carveout(CARVEOUT_BYTES)};
+  const long long most = 2ll * dev->sm_count;
   const long long rounds = (units + most - 1) / most;
   const unsigned grid = (unsigned)((units + rounds - 1) / rounds);
   cudaError_t e = cudaErrorInvalidValue;
 #define UGB_SKINNY(KC) \
-  e = ahead          ? ugb_launch(skinny_gemm_kernel<KC, false, true, false, true>, dim3(grid), dim3(KC <= 2 ? THREADS + 32 : THREADS), 0, dev->stream, g.pdl, p) \
-      : g.f16        ? ugb_launch(skinny_gemm_kernel<KC, true, false>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p) \
-      : p.wait_first ? ugb_launch(skinny_gemm_kernel<KC, false, false>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p) \
-                     : ugb_launch(skinny_gemm_kernel<KC, false, true>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p)
-  if (gate) e = ugb_launch(skinny_gemm_kernel<1, false, true, true>, dim3(grid), dim3(THREADS), 0, dev->stream, g.pdl, p);
+  e = ahead          ? ugb_launch_as(skinny_gemm_kernel<KC, false, true, false, true>, dim3(grid), dim3(KC <= 2 ? THREADS + 32 : THREADS), 0, dev->stream, form, p) \
+      : g.f16        ? ugb_launch_as(skinny_gemm_kernel<KC, true, false>, dim3(grid), dim3(THREADS), 0, dev->stream, form, p) \
+      : p.wait_first ? ugb_launch_as(skinny_gemm_kernel<KC, false, false>, dim3(grid), dim3(THREADS), 0, dev->stream, form, p) \
+                     : ugb_launch_as(skinny_gemm_kernel<KC, false, true>, dim3(grid), dim3(THREADS), 0, dev->stream, form, p)
+  if (gate) e = ugb_launch_as(skinny_gemm_kernel<1, false, true, true>, dim3(grid), dim3(THREADS), 0, dev->stream, form, p);
   else switch (kc) { case 1: UGB_SKINNY(1); break; case 2: UGB_SKINNY(2); break; case 3: UGB_SKINNY(3); break; default: UGB_SKINNY(4); }
 #undef UGB_SKINNY
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of skinny_gemm_kernel failed: %s", cudaGetErrorString(e));

@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "decode_kernels.cuh"
+#include "gemm_skinny.cuh"
 
 namespace {
 
@@ -336,15 +337,20 @@ template <int DQ, int DV> int32_t prepare_one(ugb_device *dev) {
   UGB_CUDA(dev, cudaFuncSetAttribute(grouped_attention_mma_kernel<DQ, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<DQ, DV>::BYTES));
   return UGB_OK;
 }
-template <int DQ, int DV> cudaError_t launch_one(dim3 grid, cudaStream_t st, bool pdl, const Params &p) {
-  return ugb_launch_cluster(grouped_attention_mma_kernel<DQ, DV>, grid, dim3(WARPS * 32), Ring<DQ, DV>::BYTES, st, pdl, p.splits, p);
+template <int DQ, int DV> cudaError_t launch_one(dim3 grid, int sms, cudaStream_t st, bool pdl, const Params &p) {
+  // an SM's share of the CTAs, and room for the sums of two product CTAs beside them (see gemm_skinny.cu)
+  const size_t ctas = ((size_t)grid.x * grid.y * grid.z + sms - 1) / sms;
+  const ugb_launch_form form{pdl, p.splits, ugb_carveout((Ring<DQ, DV>::BYTES + 2048) * ctas + 22 * 1024)};
+  return ugb_launch_as(grouped_attention_mma_kernel<DQ, DV>, grid, dim3(WARPS * 32), Ring<DQ, DV>::BYTES, st, form, p);
 }
 
 }  // namespace
 
 int ugb_grouped_attention_splits(const ugb_grouped_attention_args &a, int sms) {
   const int pairs = a.rows * a.kv_heads * ((a.heads / a.kv_heads + 15) / 16);
-  const int slots = a.dq + a.dv <= 128 ? 4 * sms : 2 * sms;    // CTAs that are resident together
+  // CTAs that are resident together; beside a product of few rows (early) one per SM, which is what finds room there (8 sequences of 544
+  // keys in 8 slices each 87.9 ms for a request of 32 steps, in 4 86.2, in 2 87.4)
+  const int slots = a.early && ugb_skinny_rows((size_t)a.rows) ? sms : a.dq + a.dv <= 128 ? 4 * sms : 2 * sms;
   return std::max(1, std::min(UGB_GROUPED_MAX_SPLITS, slots / std::max(1, pairs)));
 }
 
@@ -370,8 +376,8 @@ int32_t ugb_grouped_attention(ugb_device *dev, const ugb_grouped_attention_args 
     UGB_REQUIRE(dev, a.splits >= 1 && a.splits <= UGB_GROUPED_MAX_SPLITS, UGB_ERR_INVALID, "grouped attention: %d slices", a.splits);
     UGB_REQUIRE(dev, a.rows <= 65535 && a.kv_heads * ((share + 15) / 16) <= 65535, UGB_ERR_UNSUPPORTED, "grouped attention: %d rows in one launch", a.rows);
     const dim3 grid((unsigned)a.splits, (unsigned)(a.kv_heads * ((share + 15) / 16)), (unsigned)a.rows);
-    if (a.dq == 64) e = a.dv == 64 ? launch_one<64, 64>(grid, dev->stream, a.pdl, p) : launch_one<64, 128>(grid, dev->stream, a.pdl, p);
-    else e = a.dv == 64 ? launch_one<128, 64>(grid, dev->stream, a.pdl, p) : launch_one<128, 128>(grid, dev->stream, a.pdl, p);
+    if (a.dq == 64) e = a.dv == 64 ? launch_one<64, 64>(grid, dev->sm_count, dev->stream, a.pdl, p) : launch_one<64, 128>(grid, dev->sm_count, dev->stream, a.pdl, p);
+    else e = a.dv == 64 ? launch_one<128, 64>(grid, dev->sm_count, dev->stream, a.pdl, p) : launch_one<128, 128>(grid, dev->sm_count, dev->stream, a.pdl, p);
     if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of grouped_attention_mma_kernel failed: %s", cudaGetErrorString(e));
     return ugb_after_launch(dev, "grouped_attention_mma_kernel");
   }

@@ -389,8 +389,11 @@ template <int NT> int32_t prepare_one(ugb_device *dev) {
   UGB_CUDA(dev, cudaFuncSetAttribute(latent_attention_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<NT>::BYTES));
   return UGB_OK;
 }
-template <int NT> cudaError_t launch_one(dim3 grid, cudaStream_t st, bool pdl, const Params &p) {
-  return ugb_launch_cluster(latent_attention_mma_kernel<NT>, grid, dim3(WARPS * 32), Ring<NT>::BYTES, st, pdl, p.splits, p);
+template <int NT> cudaError_t launch_one(dim3 grid, int sms, cudaStream_t st, bool pdl, const Params &p) {
+  // an SM's share of the CTAs, and room for the sums of two product CTAs beside them (see gemm_skinny.cu; a request of 32 steps 34.0 -> 33.4 ms)
+  const size_t ctas = ((size_t)grid.x * grid.y * grid.z + sms - 1) / sms;
+  const ugb_launch_form form{pdl, p.splits, ugb_carveout((Ring<NT>::BYTES + 2048) * ctas + 22 * 1024)};
+  return ugb_launch_as(latent_attention_mma_kernel<NT>, grid, dim3(WARPS * 32), Ring<NT>::BYTES, st, form, p);
 }
 
 }  // namespace
@@ -423,11 +426,11 @@ int32_t ugb_latent_attention(ugb_device *dev, const ugb_latent_attention_args &a
     UGB_REQUIRE(dev, a.rows <= 65535, UGB_ERR_UNSUPPORTED, "latent attention: %d rows in one launch", a.rows);
     const dim3 grid((unsigned)a.splits, (unsigned)((a.heads + 15) / 16), (unsigned)a.rows);
     switch (a.ld / 64) {
-      case 1: e = launch_one<1>(grid, dev->stream, a.pdl, p); break;
-      case 2: e = launch_one<2>(grid, dev->stream, a.pdl, p); break;
-      case 4: e = launch_one<4>(grid, dev->stream, a.pdl, p); break;
-      case 6: e = launch_one<6>(grid, dev->stream, a.pdl, p); break;
-      default: e = launch_one<8>(grid, dev->stream, a.pdl, p); break;
+      case 1: e = launch_one<1>(grid, dev->sm_count, dev->stream, a.pdl, p); break;
+      case 2: e = launch_one<2>(grid, dev->sm_count, dev->stream, a.pdl, p); break;
+      case 4: e = launch_one<4>(grid, dev->sm_count, dev->stream, a.pdl, p); break;
+      case 6: e = launch_one<6>(grid, dev->sm_count, dev->stream, a.pdl, p); break;
+      default: e = launch_one<8>(grid, dev->sm_count, dev->stream, a.pdl, p); break;
     }
     if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of latent_attention_mma_kernel failed: %s", cudaGetErrorString(e));
     return ugb_after_launch(dev, "latent_attention_mma_kernel");

@@ -138,46 +138,45 @@ static inline int32_t ugb_check_slice(ugb_device *dev, const ugb_slice *s, int32
 __device__ __forceinline__ void ugb_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void ugb_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// How a kernel is launched: as a dependent launch, in thread-block clusters of consecutive CTAs (grid.x a multiple), and how much of
+// an SM's memory it wants as shared memory, in per cent of the most (-1: no preference).  What is not shared memory is L1, and the L1 is
+// where loads into registers wait for their data; and an SM changes the split only while it is empty.
+struct ugb_launch_form { bool pdl = false; int cluster = 1, carveout = -1; };
+// Per cent for `bytes` of shared memory per SM.
+inline int ugb_carveout(size_t bytes) { return (int)((bytes * 100 + 228 * 1024 - 1) / (228 * 1024)); }
 template <typename... KArgs, typename... Args>
-inline cudaError_t ugb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              bool pdl, Args &&...args) {
+inline cudaError_t ugb_launch_as(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const ugb_launch_form &form, Args &&...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-// The same with thread-block clusters of `cluster` consecutive CTAs (1 = none); grid.x a multiple of it.
-template <typename... KArgs, typename... Args>
-inline cudaError_t ugb_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                                      bool pdl, int cluster, Args &&...args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   int n = 0;
-  if (pdl) {
+  if (form.pdl) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n].val.programmaticStreamSerializationAllowed = 1;
-    ++n;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
   }
-  if (cluster > 1) {
+  if (form.cluster > 1) {
     attr[n].id = cudaLaunchAttributeClusterDimension;
-    attr[n].val.clusterDim.x = (unsigned)cluster;
+    attr[n].val.clusterDim.x = (unsigned)form.cluster;
     attr[n].val.clusterDim.y = 1;
-    attr[n].val.clusterDim.z = 1;
-    ++n;
+    attr[n++].val.clusterDim.z = 1;
+  }
+  if (form.carveout >= 0) {
+    attr[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[n++].val.sharedMemCarveout = (unsigned)(form.carveout > 100 ? 100 : form.carveout);
   }
   cfg.attrs = attr;
   cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t ugb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, Args &&...args) {
+  return ugb_launch_as(kernel, grid, block, smem, st, ugb_launch_form{pdl}, static_cast<Args &&>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t ugb_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, int cluster, Args &&...args) {
+  return ugb_launch_as(kernel, grid, block, smem, st, ugb_launch_form{pdl, cluster}, static_cast<Args &&>(args)...);
 }
 #endif
