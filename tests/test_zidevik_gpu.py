@@ -288,6 +288,23 @@ def test_options_do_not_change_results(make, pdl, splits):
     assert agree(feed(m, row, [70] + [1] * 20), want_of("wide_heads", row), False)
 
 
+@pytest.mark.parametrize("n", [1, 64, 65, 150])
+def test_steps_that_nobody_reads(make, n):
+    """Steps enqueued one after another, their tokens in one array that the caller overwrites at once, end where steps that are read
+    one by one do, bit by bit."""
+    row, fed, got = tokens("mixed", 55, n)[0], np.zeros(1, np.int32), []
+    for read in (True, False):
+        m = make("mixed", DType.BF16)
+        for t in row:
+            fed[0] = t
+            m.fwd(fed)
+            fed[0] = -1
+            if read:
+                m.next_tokens()
+        got.append(m.logits())
+    assert np.isfinite(got[0]).all() and np.array_equal(got[0], got[1])
+
+
 def test_greedy_generation(make):
     """generate() against the oracle's argmax in f32, whole and in portions, and the same tokens for a row in a batch."""
     rows = tokens("mixed", 53, 20, 4)

@@ -8,13 +8,14 @@ import ctypes as C
 import numpy as np
 
 from ._lib import lib
-from .device import UgError
+from .device import DType, UgError
 
 
 class EngineModel:
     """``batch`` independent sequences at one shared position, greedy choice on the device."""
 
     PREFIX = None
+    _fed = []      # tokens of steps whose copies may be on their way
     READ_LOGITS, READ_NEXT, READ_HIDDEN, READ_PREFILL_LOGITS = 0, 1, 2, 3
 
     dev = None
@@ -27,7 +28,8 @@ class EngineModel:
         return getattr(lib, f"{self.PREFIX}_{name}")
 
     def _read(self, what, out):
-        self.dev._check(self._fn("read")(self._h, what, out.ctypes.data, out.size))
+        self.dev._check(self._fn("read")(self._h, what, out.ctypes.data, out.size))   # waits for the stream
+        self._fed = []
         return out
 
     def load_weight(self, name, arr):
@@ -67,7 +69,15 @@ class EngineModel:
         tokens = np.ascontiguousarray(tokens, dtype=np.int32)
         if tokens.ndim == 2 and tokens.shape[1] > 1:
             return self.prefill(tokens, all_logits=True)
-        s = self.dev.slice_from_values(tokens.reshape(-1))
+        # The step is enqueued behind the copy of its tokens instead of after a wait for it (Llama, one sequence: 725 -> 717 us a
+        # step).  The copy's source is an array of the model's own, kept until something has waited for the stream.
+        if len(self._fed) >= 64:
+            self.dev.synchronize()
+            self._fed = []
+        tokens = np.array(tokens.reshape(-1))
+        self._fed = self._fed + [tokens]
+        s = self.dev.allocate_uninit(DType.I32, tokens.size)
+        self.dev._check(lib.ugb_h2d_async(s._h, tokens.ctypes.data, tokens.size, int(DType.I32)))
         self.dev._check(self._fn("decode")(self._h, s._h, 1))
 
     def prefill(self, tokens, all_logits=False):
