@@ -38,6 +38,14 @@ def test_rows_against_nk(dev, m, n, k, f16):
     assert np.all(np.abs(got[:m * n].reshape(m, n) - want) <= bound)
 
 
+@pytest.mark.parametrize("f16", [False, True])
+@pytest.mark.parametrize("m", [1, 8])
+@pytest.mark.parametrize("n,k", [(4720, 1024), (4736, 2056), (4737, 1032), (9489, 1024)])
+def test_pieces_around_two_ctas_per_sm(dev, m, n, k, f16):
+    """295 to 594 pieces: one for every CTA of two per SM (148 SMs), and one and two more than that."""
+    test_rows_against_nk(dev, m, n, k, f16)
+
+
 @pytest.mark.parametrize("b,m,shared", [(3, 4, False), (2, 8, False), (2, 4, True), (3, 3, True)])
 @pytest.mark.parametrize("n,k", [(72, 328), (1600, 64), (1601, 136)])
 def test_batches(dev, b, m, shared, n, k):
