@@ -98,11 +98,13 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
   ugb_device *dev = m->dev;
   const bool pdl = m->pdl != 0;
   // In a bf16 decode step every kernel lets its successor start only after its own wait: when a kernel starts, everything up
-  // to its predecessor's predecessor is complete (see row_update_kernel).
+  // to its predecessor's predecessor is complete (see row_update_kernel).  Attention beside the gate | up product is the one that does not:
+  // when its successor starts, that product may still run, and everything before it is complete.
   const bool early = decode && pdl && !m->f32;
   // What does not depend on its predecessor runs beside it, and only its end waits: the gate | up product beside mixer_inputs
   // and the scan's input product beside attention or the experts' last product (a_ahead, up to 8 rows), attention beside the gate | up
-  // product, the experts' rows beside both (request 8x512+32: 94.3 -> 88.0 ms).
+  // product, the experts' rows beside both (request 8x512+32: 94.3 -> 88.0 ms).  What runs ahead reads mixer_inputs' results and older ones,
+  // and writes what neither that product nor attention touches.
   const int B = m->batch, rows = B * t, wl = m->wl, n_runs = (int)m->runs.size();
   const bool whole = m->only == UGB_HYBRID_K_ALL;            // kernels timed alone leave the counts of the last whole pass as they are
   const bool looped = m->cfg.loop_times > 0, side = m->cfg.side_dim > 0;
