@@ -19,6 +19,7 @@ struct ugb_hybrid_weights {
   float *bz = nullptr, *bu = nullptr;
   float *q_gain = nullptr, *c_gain = nullptr;
   void *w_uq = nullptr, *w_uk = nullptr, *w_uv = nullptr;
+  void *w_ukt = nullptr;                      // w_uk of every head transposed, for the few rows of a step (up to 8, bf16)
   void *w_up = nullptr, *w_down = nullptr;    // parallel form: w_up holds (gate, up) row pairs
   int dp = 0, vp = 0;                         // padded widths of an attention head's queries / keys and values
   // parallel form: w_in rows are q | k | v | x | z | router, w_out columns attention | scan | feed-forward

@@ -728,5 +728,10 @@ static __global__ void taps_kernel(const float *__restrict__ w, float *__restric
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < width * taps) out[(size_t)(i % taps) * ld + i / taps] = w[i];
 }
+// n values [heads][rows][cols] -> [heads][cols][rows]
+static __global__ void transpose_heads_kernel(const __nv_bfloat16 *__restrict__ in, __nv_bfloat16 *__restrict__ out, size_t n, int rows, int cols) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, c = i / rows % cols, h = i / rows / cols;
+  if (i < n) out[i] = in[(h * rows + i % rows) * cols + c];
+}
 
 }  // namespace ugb_hybrid_k
