@@ -305,6 +305,18 @@ def test_steps_that_nobody_reads(make, n):
     assert np.isfinite(got[0]).all() and np.array_equal(got[0], got[1])
 
 
+def test_steps_after_a_bad_token_are_enqueued(make, dev):
+    """What a step reports is left for synchronize(): however many unread steps follow, none of them raises it, and none is lost."""
+    m, n = make("odd", DType.BF16), 140
+    m.fwd(np.array([CONFIGS["odd"].vocab], np.int32))
+    for i in range(n):
+        m.fwd(np.array([i % 7], np.int32))
+    assert m.position == n + 1
+    with pytest.raises(UgError):
+        dev.synchronize()
+    dev.synchronize()
+
+
 def test_greedy_generation(make):
     """generate() against the oracle's argmax in f32, whole and in portions, and the same tokens for a row in a batch."""
     rows = tokens("mixed", 53, 20, 4)

@@ -65,19 +65,21 @@ class EngineModel:
     def fwd(self, tokens):
         """Model::fwd on explicit token ids, asynchronous: int32 [batch] or [batch, 1] is one
         decode step; [batch, t] with t > 1 appends t positions (causal prefill) and keeps the
-        logits of every position for :meth:`prefill_logits`."""
+        logits of every position for :meth:`prefill_logits`.  What a step reports on the device (a token that does not exist, say) is
+        raised by the device's next ``synchronize``, not by a later call of this one."""
         tokens = np.ascontiguousarray(tokens, dtype=np.int32)
         if tokens.ndim == 2 and tokens.shape[1] > 1:
             return self.prefill(tokens, all_logits=True)
         # The step is enqueued behind the copy of its tokens instead of after a wait for it (Llama, one sequence: 725 -> 717 us a
-        # step).  The copy's source is an array of the model's own, kept until something has waited for the stream.
+        # step).  The copy's source is an array of the model's own, kept until something has waited for the stream: a read, or the
+        # copy of every 65th step that nobody reads, which waits and leaves what the steps have reported to the caller's own synchronize.
         if len(self._fed) >= 64:
-            self.dev.synchronize()
-            self._fed = []
-        tokens = np.array(tokens.reshape(-1))
-        self._fed = self._fed + [tokens]
-        s = self.dev.allocate_uninit(DType.I32, tokens.size)
-        self.dev._check(lib.ugb_h2d_async(s._h, tokens.ctypes.data, tokens.size, int(DType.I32)))
+            s, self._fed = self.dev.slice_from_values(tokens.reshape(-1)), []
+        else:
+            tokens = np.array(tokens.reshape(-1))
+            self._fed = self._fed + [tokens]
+            s = self.dev.allocate_uninit(DType.I32, tokens.size)
+            self.dev._check(lib.ugb_h2d_async(s._h, tokens.ctypes.data, tokens.size, int(DType.I32)))
         self.dev._check(self._fn("decode")(self._h, s._h, 1))
 
     def prefill(self, tokens, all_logits=False):
