@@ -192,7 +192,9 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
 
     const size_t n_cat = L.n_cat(), cat_s = (size_t)d.heads * L.vp, cat_f = cat_s + L.ci;
     // ---- attention
-    const bool beside = early && whole && L.fl > 0;        // a product lies between mixer_inputs and what follows it
+    // A step runs it behind the gate | up product where there is one (beside), else behind the scan; either way a kernel lies between
+    // mixer_inputs and attention, which may then start early.
+    const bool beside = early && whole && L.fl > 0;
     auto attention = [&]() -> int32_t {
       if (!m->on(UGB_HYBRID_K_ATTENTION)) return UGB_OK;
       if (!decode && L.expand && t > m->absorb_max) {
@@ -206,7 +208,7 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
         ugb_grouped_attention_args a{};
         a.f32 = m->f32; a.q = w.q; a.k = R.cache; a.v = R.vcache; a.out = w.cat; a.out_ld = n_cat; a.out_scale = d.attention_scale;
         a.rows = rows; a.t = t; a.pos_p = m->pos; a.pos_off = off; a.heads = d.heads; a.kv_heads = d.kv_heads; a.dq = L.dp; a.dv = L.vp;
-        a.t_max = m->t_max; a.scale = d.scale; a.pdl = pdl; a.early = beside;
+        a.t_max = m->t_max; a.scale = d.scale; a.pdl = pdl; a.early = early && whole;
         a.splits = m->att_splits_opt > 0 ? std::min(m->att_splits_opt, UGB_GROUPED_MAX_SPLITS) : ugb_grouped_attention_splits(a, dev->sm_count);
         return ugb_grouped_attention(dev, a);
       }
@@ -219,7 +221,7 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
         g.ahead = early && whole;
         if ((rc = gated_product(m, w, g))) return rc;
       }
-      if (decode && (rc = attention())) return rc;
+      if (decode && L.fl && (rc = attention())) return rc;
       if (experts) {
         const int tile = w.tile, tiles = group_tiles((size_t)rows * d.top, d.experts, tile);
         const size_t xrows = (size_t)tiles * tile;
@@ -284,7 +286,7 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
       if (rc) return rc;
     }
 
-    if (!decode && (rc = attention())) return rc;
+    if (!(decode && L.fl) && (rc = attention())) return rc;
     if (!decode && (rc = feed_forward())) return rc;
 
     // ---- output projections, residual
