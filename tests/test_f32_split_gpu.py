@@ -9,7 +9,9 @@ pytestmark = pytest.mark.gpu
 # (b, m, n, k) -> (rows of a tile, CTAs along k) on 148 SMs; test_f32_split_plan_cpu.py holds the rule to these
 SHAPES = {(1, 257, 5632, 2048): (96, 1), (1, 128, 2048, 2048): (64, 4), (1, 120, 1352, 7144): (128, 8), (2, 526, 1080, 216): (96, 1), (1, 31, 8000, 128): (32, 1),
           (32, 128, 64, 64): (32, 1), (16, 300, 777, 400): (128, 1), (1, 33, 4000, 512): (64, 4), (1, 500, 1001, 999): (128, 4), (1, 19, 1031, 65): (32, 1),
-          (1, 65, 129, 97): (32, 1), (1, 97, 127, 4095): (32, 8), (1, 128, 5000, 500): (64, 1), (1, 60, 5000, 500): (64, 2), (1, 250, 3000, 500): (96, 2)}
+          (1, 65, 129, 97): (32, 1), (1, 97, 127, 4095): (32, 8), (1, 128, 5000, 500): (64, 1), (1, 60, 5000, 500): (64, 2), (1, 250, 3000, 500): (96, 2),
+          # the tests of single values, of long k and of shared matrices
+          (1, 70, 300, 200): (32, 1), (1, 130, 260, 128): (32, 1), (1, 150, 300, 256): (32, 4), (1, 200, 640, 4096): (128, 8), (3, 257, 1024, 512): (96, 2)}
 
 
 def _product(dev, a, w, a_km, b_kn, guard=64):
@@ -26,7 +28,7 @@ def _product(dev, a, w, a_km, b_kn, guard=64):
 
 
 def _bound(a, w):
-    """k products and sums in f32, each rounding at most 2^-24 of the sum of magnitudes; the parts that are left out are 2^-26 of it."""
+    """k products and sums in f32, each rounding at most 2^-24 of the sum of magnitudes; the parts that are left out are 2^-24 of it at most."""
     return np.abs(a).astype(np.float64) @ np.abs(w).astype(np.float64) * (a.shape[2] + 16) * 2.0 ** -24 + 1e-44
 
 
@@ -36,7 +38,31 @@ def _bound(a, w):
 def test_layouts(dev, b, m, n, k, a_km, b_kn):
     a, w = synth.normal(31 + m, (b, m, k), 0.5), synth.normal(32 + n, (b, k, n), 0.5)
     got = _product(dev, a, w, a_km, b_kn)
-    assert np.all(np.abs(got - a.astype(np.float64) @ w.astype(np.float64)) <= _bound(a, w))
+    want = a.astype(np.float64) @ w.astype(np.float64)
+    assert np.all(np.abs(got - want) <= _bound(a, w))
+    # A few times the spacing of f32 at 1 (1.2e-7): sums that are cut off at most four times before they are rounded.  A product of parts that is
+    # missing or taken from the wrong k is 2e-6 and more of such a result, which the bound above does not see.
+    assert np.linalg.norm(got - want) <= 3e-7 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("a_km", [False, True])
+@pytest.mark.parametrize("b_kn", [False, True])
+@pytest.mark.parametrize("b,m,n,k", list(SHAPES))
+def test_every_part_counts(dev, b, m, n, k, a_km, b_kn):
+    """Values whose last seven bits are in the third part alone, times a matrix that picks one of them for every result: each comes out
+    exact, through either operand."""
+    rng = np.random.default_rng(m + n)
+    full = lambda *shape: (1 + 129 * 2.0 ** -16 + rng.integers(-63, 64, shape) * 2.0 ** -23).astype(np.float32)
+    a, pick = full(b, m, k), rng.integers(0, k, n)
+    pick[:min(n, k)] = np.arange(k)[::-1][:min(n, k)]
+    w = np.zeros((b, k, n), np.float32)
+    w[:, pick, np.arange(n)] = 1.0
+    assert np.array_equal(_product(dev, a, w, a_km, b_kn), a[:, :, pick])
+    w, pick = full(b, k, n), rng.integers(0, k, m)
+    pick[:min(m, k)] = np.arange(k)[:min(m, k)]
+    a = np.zeros((b, m, k), np.float32)
+    a[:, np.arange(m), pick] = 1.0
+    assert np.array_equal(_product(dev, a, w, a_km, b_kn), w[:, pick])
 
 
 def test_error_is_that_of_one_rounding_not_of_k(dev):
@@ -68,17 +94,33 @@ def test_one_tiny_value_in_a_tile(dev):
 
 
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 3.4e38])
-def test_what_is_not_finite_stays_in_its_row(dev, value):
-    a, w = synth.normal(7, (1, 70, 300), 0.5), synth.normal(8, (1, 300, 260), 0.5)
-    a[0, 69, 299] = value
-    w[0, :, 100] = 0.0
-    w[0, 299, 100] = 0.25
+@pytest.mark.parametrize("last", [False, True])
+@pytest.mark.parametrize("m,n,k", [(257, 5632, 2048), (128, 2048, 2048), (70, 300, 200), (60, 5000, 500)])
+def test_what_is_not_finite_stays_in_its_row(dev, m, n, k, last, value):
+    """In the last row, at either end of k (with k over a cluster, one CTA sees it), against columns of which the last is zero elsewhere.  The
+    results beside it in its tile are the bits that they are without it."""
+    a, w = synth.normal(7, (1, m, k), 0.5), synth.normal(8, (1, k, n), 0.5)
+    at = k - 1 if last else 3
+    w[0, :, n - 1] = 0.0
+    w[0, at, n - 1] = 0.25
+    plain = _product(dev, a, w, False, False)[0]
+    a[0, m - 1, at] = value
     with np.errstate(all="ignore"):
-        want = (a[0].astype(np.float64) @ w[0].astype(np.float64)).astype(np.float32)
+        want = (a[0, m - 1].astype(np.float64) @ w[0].astype(np.float64)).astype(np.float32)
     got = _product(dev, a, w, False, False)[0]
-    assert np.all(np.isfinite(got[:69]))
-    assert np.array_equal(np.isnan(got[69]), np.isnan(want[69])) and np.array_equal(np.isinf(got[69]), np.isinf(want[69]))
-    assert got[69, 100] == want[69, 100] or np.isnan(value)
+    assert np.array_equal(got[:m - 1], plain[:m - 1]) and np.all(np.isfinite(plain))
+    assert np.array_equal(np.isnan(got[m - 1]), np.isnan(want)) and np.array_equal(np.isinf(got[m - 1]), np.isinf(want))
+    on = np.isfinite(want)
+    assert np.all(np.abs(got[m - 1, on] - want[on]) <= 2.0 ** -20 * np.abs(want[on])) and np.array_equal(got[m - 1][np.isinf(want)], want[np.isinf(want)])
+
+
+@pytest.mark.parametrize("a_km,b_kn", [(False, True), (True, False), (True, True)])
+def test_a_column_that_is_not_finite(dev, a_km, b_kn):
+    a, w = synth.normal(12, (1, 257, 2048), 0.5), synth.normal(13, (1, 2048, 5632), 0.5)
+    plain = _product(dev, a, w, a_km, b_kn)[0]
+    w[0, 2047, 5631] = np.nan
+    got = _product(dev, a, w, a_km, b_kn)[0]
+    assert np.array_equal(got[:, :5631], plain[:, :5631]) and np.all(np.isnan(got[:, 5631]))
 
 
 def test_whole_numbers_are_exact(dev):
@@ -87,11 +129,14 @@ def test_whole_numbers_are_exact(dev):
     assert np.array_equal(_product(dev, a, w, False, False), a @ w)
 
 
-def test_shared_matrix_and_strided_result(dev):
-    """One matrix for every batch step, as a linear layer of the graph has it."""
-    b, m, n, k = 3, 45, 200, 320
-    a, w = synth.normal(10, (b, m, k), 0.5), synth.normal(11, (k, n), 0.5)
+@pytest.mark.parametrize("which", ["left", "right"])
+def test_shared_matrix(dev, which):
+    """One matrix for every batch step, as a linear layer of the graph has it, on either side."""
+    b, m, n, k = 3, 257, 1024, 512
+    a, w = synth.normal(10, (b if which == "right" else 1, m, k), 0.5), synth.normal(11, (b if which == "left" else 1, n, k), 0.5)
     out = dev.allocate_uninit(DType.F32, b * m * n)
-    dev.matmul(out, dev.slice_from_values(a.ravel()), dev.slice_from_values(np.ascontiguousarray(w.T).ravel()), (b, m, n, k), ([b, m, k], [m * k, k, 1], 0), ([b, k, n], [0, 1, k], 0))
-    got = out.to_vec().reshape(b, m, n)
-    assert np.all(np.abs(got - a.astype(np.float64) @ w.astype(np.float64)) <= _bound(a, np.broadcast_to(w, (b, k, n))))
+    dev.matmul(out, dev.slice_from_values(a.ravel()), dev.slice_from_values(w.ravel()), (b, m, n, k),
+               ([b, m, k], [m * k if which == "right" else 0, k, 1], 0), ([b, k, n], [n * k if which == "left" else 0, 1, k], 0))
+    a, w = np.broadcast_to(a, (b, m, k)), np.broadcast_to(w.transpose(0, 2, 1), (b, k, n))
+    got, want = out.to_vec().reshape(b, m, n), a.astype(np.float64) @ w.astype(np.float64)
+    assert np.all(np.abs(got - want) <= _bound(a, w)) and np.linalg.norm(got - want) <= 3e-7 * np.linalg.norm(want)

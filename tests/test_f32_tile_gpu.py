@@ -1,5 +1,6 @@
 """f32 products of many rows or few columns: edges of the 32- to 128-row tiles, of the 128-column tiles and 16-deep slices, products so small
-that k is split inside a CTA and over a cluster, and every layout of both operands, against float64."""
+that k is split inside a CTA and over a cluster, and every layout of both operands, against float64.  Sizes that run on the tensor cores on
+148 SMs (test_f32_split_gpu.py has their edges) are here beside those that do not: FFMA and FFMA_KM."""
 import numpy as np
 import pytest
 
@@ -7,6 +8,15 @@ from ug_b200 import DType, synth
 
 pytestmark = pytest.mark.gpu
 TURNED = [(20000, 17, 64), (8193, 8, 512), (3000, 5, 1999), (2600, 36, 1000), (5000, 64, 300), (1301, 33, 597)]   # few columns: the rows of the tile
+
+# (b, m, n, k) -> (warps over rows, over a slice's k, CTAs along k, turned) on 148 SMs, what stays on the FFMA kernel: whatever the left layout, and
+# with the left operand stored [k, m]; test_f32_split_plan_cpu.py holds the rules to these
+FFMA = {(1, 33, 132, 20): (1, 4, 1, 0), (1, 20, 4, 128): (1, 4, 2, 0), (1, 70, 260, 300): (1, 4, 4, 0), (1, 101, 511, 1030): (1, 4, 8, 0),
+        (38, 100, 4, 88): (1, 4, 1, 1), (1, 8192, 8, 512): (1, 4, 2, 1), (1, 3000, 5, 1999): (1, 4, 4, 1), (11, 36, 4, 524): (1, 4, 8, 1),
+        (1, 779, 667, 36): (2, 2, 1, 0), (1, 1212, 544, 40): (2, 2, 1, 0), (1, 371, 270, 582): (2, 2, 8, 0), (1, 356, 284, 584): (2, 2, 8, 0),
+        (1, 2179, 35, 589): (2, 2, 8, 1), (1, 2200, 36, 584): (2, 2, 8, 1), (38, 100, 4, 20): (4, 1, 1, 0), (1, 1001, 3001, 21): (4, 1, 1, 0)}
+FFMA_KM = {(1, 583, 131, 258): (2, 2, 4, 0), (1, 584, 132, 272): (2, 2, 4, 0), (1, 3876, 45, 289): (2, 2, 4, 1), (1, 3900, 36, 292): (2, 2, 4, 1),
+           (1, 736, 261, 535): (4, 1, 8, 0), (1, 720, 280, 532): (4, 1, 8, 0)}
 
 
 def _check(dev, b, m, n, k, a_km, b_kn, shared=False):
@@ -32,6 +42,13 @@ def _check(dev, b, m, n, k, a_km, b_kn, shared=False):
                                    (65, 63, 1), (130, 129, 15), (64, 65, 16), (63, 200, 17), (5000, 4000, 6)] + TURNED)
 def test_layouts(dev, m, n, k, a_km, b_kn):
     _check(dev, 1, m, n, k, a_km, b_kn)
+
+
+@pytest.mark.parametrize("b_kn", [False, True])
+@pytest.mark.parametrize("b,m,n,k", list(FFMA) + list(FFMA_KM))
+def test_every_instance(dev, b, m, n, k, b_kn):
+    for a_km in (False, True) if (b, m, n, k) in FFMA else (True,):
+        _check(dev, b, m, n, k, a_km, b_kn)
 
 
 @pytest.mark.parametrize("b,m,n,k,shared", [(5, 40, 96, 512, False), (3, 130, 36, 61, False), (16, 20, 200, 256, True), (40, 65, 132, 72, False)])

@@ -134,6 +134,106 @@ template <int R, bool KC, bool VEC> struct Operand {
   }
 };
 
+// Bit j of a worker's `odd`: its sum j is formed again, in f32.  The others keep what they have, so that no result depends on what its
+// neighbours in the tile hold.  Up to LIST of them (a row or a column of the product) are dot products of a warp each; more are
+// formed by all workers from slices in shared memory, eight columns of a warp without one passed over.  Not inlined: a tile comes here once at
+// most, and the arrays would be the main loop's registers.  All threads of the block.
+template <int BN, bool PK, bool QK>
+static __device__ __noinline__ void again_with_ffma(const float *P, const float *Q, long long p_rs, long long p_ks, long long q_rs, long long q_ks, int rows_p, int rows_q,
+                                                    int k_lo, int k_hi, float (&result)[BN * 4 / WARPS], uint32_t odd) {
+  extern __shared__ uint8_t smem_raw[];    // not handed over: its loads would be generic ones
+  uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  constexpr int CK = 32, COLS = BN * 4 / WARPS, NP = (BM * CK + THREADS - 1) / THREADS, NQ = (BN * CK + THREADS - 1) / THREADS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * COLS;
+  const uint32_t needed = __reduce_or_sync(0xffffffffu, odd);
+  {
+    constexpr int LIST = 512;
+    int *count = reinterpret_cast<int *>(smem);
+    uint16_t *list = reinterpret_cast<uint16_t *>(smem + 16);
+    float *sums = reinterpret_cast<float *>(smem + 16 + 2 * LIST);
+    if (threadIdx.x == 0) *count = 0;
+    __syncthreads();
+    const int first = odd ? atomicAdd(count, __popc(odd)) : 0;
+    int at = first;
+#pragma unroll
+    for (int j = 0; j < COLS; ++j)
+      if (odd >> j & 1) {
+        if (at < LIST) list[at] = (uint16_t)((col0 + j) * BM + row);
+        ++at;
+      }
+    __syncthreads();
+    const int n = *count;
+    if (n <= LIST) {
+      for (int i = warp; i < n; i += WARPS + 1) {
+        const float *x = P + (list[i] % BM) * p_rs, *y = Q + (list[i] / BM) * q_rs;
+        float sum = 0.f;
+#pragma unroll 8
+        for (int k = k_lo + lane; k < k_hi; k += 32) sum = fmaf(x[k * p_ks], y[k * q_ks], sum);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) sums[i] = sum;
+      }
+      __syncthreads();
+      at = first;
+#pragma unroll
+      for (int j = 0; j < COLS; ++j)
+        if (odd >> j & 1) result[j] = sums[at++];
+      __syncthreads();                     // the caller writes shared memory
+      return;
+    }
+    __syncthreads();
+  }
+  float(*sp)[BM + 1] = reinterpret_cast<float(*)[BM + 1]>(smem);
+  float(*sq)[BN + 4] = reinterpret_cast<float(*)[BN + 4]>(smem + CK * (BM + 1) * 4 + 64 - CK * (BM + 1) * 4 % 64);
+  float acc[COLS] = {}, np[NP], nq[NQ];    // np, nq: the next slice
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int e = threadIdx.x + i * THREADS, r = PK ? e / CK : e % BM, k = k0 + (PK ? e % CK : e / BM);
+      np[i] = ld1(P + r * p_rs + k * p_ks, e < BM * CK && r < rows_p && k < k_hi);
+    }
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      const int e = threadIdx.x + i * THREADS, r = QK ? e / CK : e % BN, k = k0 + (QK ? e % CK : e / BN);
+      nq[i] = ld1(Q + r * q_rs + k * q_ks, e < BN * CK && r < rows_q && k < k_hi);
+    }
+  };
+  fetch(k_lo);
+  for (int k0 = k_lo; k0 < k_hi; k0 += CK) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int e = threadIdx.x + i * THREADS;
+      if (e < BM * CK) sp[PK ? e % CK : e / BM][PK ? e / CK : e % BM] = np[i];
+    }
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      const int e = threadIdx.x + i * THREADS;
+      if (e < BN * CK) sq[QK ? e % CK : e / BN][QK ? e / CK : e % BN] = nq[i];
+    }
+    __syncthreads();
+    fetch(k0 + CK);
+#pragma unroll
+    for (int j = 0; j < COLS; j += 8) {
+      if (!(needed >> j & 0xff)) continue;
+      float sum[8] = {};                   // of this slice, so that no sum is long
+#pragma unroll 8
+      for (int k = 0; k < CK; ++k) {
+        const float x = sp[k][row];
+        const float4 y = *reinterpret_cast<const float4 *>(&sq[k][col0 + j]), z = *reinterpret_cast<const float4 *>(&sq[k][col0 + j + 4]);
+        sum[0] = fmaf(x, y.x, sum[0]); sum[1] = fmaf(x, y.y, sum[1]); sum[2] = fmaf(x, y.z, sum[2]); sum[3] = fmaf(x, y.w, sum[3]);
+        sum[4] = fmaf(x, z.x, sum[4]); sum[5] = fmaf(x, z.y, sum[5]); sum[6] = fmaf(x, z.z, sum[6]); sum[7] = fmaf(x, z.w, sum[7]);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[j + e] += sum[e];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < COLS; ++j)
+    if (odd >> j & 1) result[j] = acc[j];
+}
+
 template <int BN, bool PK, bool QK, bool VEC>
 __global__ void __launch_bounds__(THREADS, 1)
 f32_split_kernel(const Params p) {
@@ -290,65 +390,21 @@ f32_split_kernel(const Params p) {
   // times the largest value.
   const uint32_t ep = least_p == 0xffffffffu ? 255u : (least_p + 1u) >> 24, eq = least_q == 0xffffffffu ? 255u : (least_q + 1u) >> 24;
   const float floor_ = ep < 24u || eq < 24u || ep + eq < 158u ? (float)p.k * __uint_as_float(most << 16) * 0x1p-97f : 0.f;
+  uint32_t odd = 0;                        // of this worker's sums
   if (worker) {
-    bool odd = false;
 #pragma unroll
     for (int j = 0; j < COLS; ++j)
-      if (p0 + row < p.rows_p && q0 + col0 + j < p.rows_q) odd |= !(fabsf(acc[j]) <= 3.402823466e38f && fabsf(acc[j]) >= floor_);
+      if (p0 + row < p.rows_p && q0 + col0 + j < p.rows_q && !(fabsf(acc[j]) <= 3.402823466e38f && fabsf(acc[j]) >= floor_)) odd |= 1u << j;
     if (__any_sync(0xffffffffu, odd) && lane == 0) atomicOr(&again, 1);
   }
   __syncthreads();
   if (again) {
-    constexpr int CK = 32;
-    float(*sp)[BM + 1] = reinterpret_cast<float(*)[BM + 1]>(smem);
-    float(*sq)[BN + 4] = reinterpret_cast<float(*)[BN + 4]>(smem + CK * (BM + 1) * 4 + 64 - CK * (BM + 1) * 4 % 64);
+    float sums[COLS];
 #pragma unroll
-    for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
-    constexpr int NP = (BM * CK + THREADS - 1) / THREADS, NQ = (BN * CK + THREADS - 1) / THREADS;
-    float np[NP], nq[NQ];                  // the next slice
-    auto fetch = [&](int k0) {
+    for (int j = 0; j < COLS; ++j) sums[j] = acc[j];
+    again_with_ffma<BN, PK, QK>(P, Q, p.p_rs, p.p_ks, p.q_rs, p.q_ks, p.rows_p - p0, p.rows_q - q0, k_lo, k_hi, sums, odd);
 #pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        const int e = threadIdx.x + i * THREADS, r = PK ? e / CK : e % BM, k = k0 + (PK ? e % CK : e / BM);
-        np[i] = ld1(P + r * p.p_rs + k * p.p_ks, e < BM * CK && p0 + r < p.rows_p && k < k_hi);
-      }
-#pragma unroll
-      for (int i = 0; i < NQ; ++i) {
-        const int e = threadIdx.x + i * THREADS, r = QK ? e / CK : e % BN, k = k0 + (QK ? e % CK : e / BN);
-        nq[i] = ld1(Q + r * p.q_rs + k * p.q_ks, e < BN * CK && q0 + r < p.rows_q && k < k_hi);
-      }
-    };
-    fetch(k_lo);
-    for (int k0 = k_lo; k0 < k_hi; k0 += CK) {
-      __syncthreads();
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        const int e = threadIdx.x + i * THREADS;
-        if (e < BM * CK) sp[PK ? e % CK : e / BM][PK ? e / CK : e % BM] = np[i];
-      }
-#pragma unroll
-      for (int i = 0; i < NQ; ++i) {
-        const int e = threadIdx.x + i * THREADS;
-        if (e < BN * CK) sq[QK ? e % CK : e / BN][QK ? e / CK : e % BN] = nq[i];
-      }
-      __syncthreads();
-      fetch(k0 + CK);
-      float sum[COLS] = {};                // of this slice, so that no sum is long
-      if (worker)
-#pragma unroll 8
-        for (int k = 0; k < CK; ++k) {
-          const float x = sp[k][row];
-#pragma unroll
-          for (int j = 0; j < COLS; j += 4) {
-            const float4 y = *reinterpret_cast<const float4 *>(&sq[k][col0 + j]);
-            sum[j] = fmaf(x, y.x, sum[j]); sum[j + 1] = fmaf(x, y.y, sum[j + 1]);
-            sum[j + 2] = fmaf(x, y.z, sum[j + 2]); sum[j + 3] = fmaf(x, y.w, sum[j + 3]);
-          }
-        }
-#pragma unroll
-      for (int j = 0; j < COLS; ++j) acc[j] += sum[j];
-    }
-    __syncthreads();
+    for (int j = 0; j < COLS; ++j) acc[j] = sums[j];
   }
 
   float *C = p.c + (long long)blockIdx.z * p.c_b;
