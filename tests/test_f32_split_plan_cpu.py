@@ -5,7 +5,7 @@ import subprocess
 import pytest
 
 from conftest import ROOT
-from test_f32_split_gpu import SHAPES
+from test_f32_split_gpu import CHAINS, SHAPES
 from test_f32_tile_gpu import FFMA, FFMA_KM
 
 SMS = 148
@@ -44,7 +44,7 @@ def ask(plan):
 def test_tested_sizes_reach_their_tiles(ask, case):
     assert ask(*case, 0) == SHAPES[case]
     bn, split = ask(*case, 1)
-    assert bn in (0, 64, 128) and split in (1, 2, 4, 8)
+    assert bn in (0, 64) and split in (1, 2, 4, 8)
 
 
 @pytest.mark.parametrize("case", [(1, 257, 5632, 2048), (1, 128, 2048, 2048)])
@@ -66,9 +66,21 @@ def test_every_instance_of_the_ffma_kernel_is_reached():
 
 
 def test_every_tile_and_cluster_is_reached():
-    assert {s[0] for s in SHAPES.values()} == {32, 64, 96, 128} and {s[1] for s in SHAPES.values()} == {1, 2, 4, 8}
+    assert {s[0] for s in SHAPES.values()} == {32, 64, 96} and {s[1] for s in SHAPES.values()} == {1, 2, 4, 8}
 
 
 def test_short_k_and_next_to_nothing_stay_where_they_were(ask):
-    assert ask(1, 4096, 4096, 63, 0)[0] == 0 and ask(1, 4096, 4096, 16, 1)[0] == 0
-    assert ask(1, 0, 5, 100, 0)[0] == 0 and ask(5, 3922, 8, 88, 0)[0] == 0 and ask(5, 3922, 33, 88, 0)[0] != 0
+    assert ask(1, 4932, 132, 95, 0)[0] == 0 and ask(1, 4096, 4096, 16, 1)[0] == 0 and ask(1, 4932, 132, 96, 0)[0] != 0
+    assert ask(1, 0, 5, 100, 0)[0] == 0 and ask(5, 3922, 8, 388, 0)[0] == 0 and ask(5, 3922, 33, 388, 0)[0] != 0
+
+
+@pytest.mark.parametrize("case", list(CHAINS))
+def test_chains_beside_which_errors_are_held(plan, case):
+    (bn, split), (wm, wk, cluster, _) = plan(*case, 0)
+    assert CHAINS[case] == wk * cluster and case[3] >= 96 * wk * cluster and 6 * split >= wk * cluster
+
+
+def test_short_chains_and_many_of_them_stay_with_ffma(plan):
+    for case in ((1, 128, 2048, 760), (1, 17, 5632, 2048), (8, 300, 64, 8192)):
+        (bn, _), (_, wk, cluster, _) = plan(*case, 0)
+        assert bn == 0, case

@@ -1,31 +1,39 @@
-// f32 products on the tensor cores: every value is the exact sum of three bf16 parts, and six of the nine products of parts are
+// f32 products on the tensor cores: every value is the exact sum of three bf16 parts, and eight of the nine products of parts are
 // formed by tcgen05.mma with f32 accumulators.
 //
 //   x = hi + mid + lo     hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid: 8 bits each, nothing is lost
-//   a b = hi hi           in accumulators of their own, which leave the tensor memory for f32 registers every 64 k
-//       + hi mid + mid hi + mid mid + hi lo + lo hi          (2^-8 of it and less: one accumulator over all of k)
-//       + mid lo + lo mid + lo lo                            left out: 2^-26 of |a b| at most
+//   a b = hi hi           16 products at a time, each time in an accumulator of its own, from where they are added up in f32 registers
+//       + hi mid + mid hi + mid mid + hi lo + lo hi + mid lo + lo mid          (2^-8 of it and less: one accumulator for 960 k)
+//       + lo lo                                              left out: 2^-33 of |a b|
 //
-// The tensor core cuts a sum off where an FFMA rounds it, so a long sum that stays there drifts towards zero (128 additions of a
-// product of k = 2048: 5e-6 of it); four additions between two transfers and rounded sums in registers leave less error than
-// the FFMA kernel's own sums: 1.3e-7 of the result against 4.1e-7 at k = 2048, 9e-8 against 2.1e-7 at 1000, 6.8e-8 against 8.5e-8 at 64.  What the
-// parts cannot hold is found as it is read and as it is stored, and the tile is then computed again with FFMA: a result that is not
-// finite, and, where parts or products of parts left the normal range (no part product does below 2^-126 as long as the smallest
-// exponents add up to -96 or more), a result so small that what was lost may be 2^-26 of it.
+// The tensor core cuts off what an FFMA rounds: of 16 products and the accumulator, what lies 2^-25 below the largest, and then their sum to
+// f32.  Sums of one sign lose a little of themselves every time, so nothing is added to hi hi there.  The error against 64 bits,
+// beside that of the FFMA kernel, by what is summed (2-norm, 257 x 1024 results):
+//                                     k = 1000                2048                    4096
+//   normal                            8.1e-8 against 2.1e-7   9.8e-8 against 2.2e-7   1.2e-7 against 3.0e-7
+//   uniform in 0 .. 1                 4.6e-8 against 7.0e-8   5.2e-8 against 7.1e-8   5.9e-8 against 8.0e-8
+//   softmax (deviation 3) x uniform   9.7e-8 against 1.1e-7   1.0e-7 against 1.1e-7   1.1e-7 against 1.4e-7
+// With 64 k in an accumulator and six products the last of these was 2.8e-7 to 3.0e-7.  At k = 64 it is 8e-8 here and 6e-8 with FFMA: see
+// ugb_f32_gemm_split_plan for the sums that stay there.
+//
+// What the parts cannot hold is found as it is read and as it is stored, and that result is then formed again with FFMA: one that is not
+// finite, and, where parts left the normal range or products of parts may have lost more than 2^-30 of a product of values (it loses no more as long as
+// the smallest exponents add up to -96 or more), one so small that what was lost may be 2^-26 of it.
 //
 // Tile: 128 columns of the result (lanes of the tensor memory: a warp stores whole lines) x BN rows.  16 warps read both operands, two
 // stages of 32 k ahead in registers, split them into the six swizzled shared-memory planes of a stage, and add what the tensor core
 // has finished to their f32 sums; a warp of its own issues (issued by one of the 16, its conversion and its issuing were in line, and
 // every stage waited for both).  Few tiles: CTAs of a cluster along k, sums through distributed shared memory in rank order.
 //
-// Bound: the conversion (about ten instructions a value on 28 values per thread and stage) and the products' own reads of shared memory
-// (an MMA of 128 x 96 x 16 takes 56 cycles for its operands, twelve a stage), 0.8 us a stage together.  The loads wait in the L1, which is
-// what the stages leave of 256 KB: 32 k a stage, not 64.  The fence between the planes and the tensor core is that of shared memory
-// alone: the general one also waits for the loads ahead (86 -> 59 us on the first of these).  8 warps with twice the work each 68 us there
-// against 56, three stages ahead 61, lines asked into the L2 six stages ahead 59.
-// Against the FFMA kernel: [257, 2048] x [5632, 2048]^T 182 -> 56 us (70 with the matrix from HBM), [2048, 2048] x [4096, 2048]^T 680 -> 298, [777, 5632] x
-// [2048, 5632]^T 481 -> 165, [128, 2048] x [2048, 2048]^T 56 -> 18, [500, 999] x [1001, 999]^T 34 -> 19.  Values that send a tile to FFMA: up to
-// four times the FFMA kernel's time.
+// Bound: the conversion (about ten instructions a value on 28 values per thread and stage), the products' own reads of shared memory
+// (an MMA of 128 x 96 x 16 takes 56 cycles for its operands, sixteen a stage) and the sums' way out of the tensor memory, 1.0 us a stage
+// together.  The loads wait in the L1, which is what the stages leave of 256 KB: 32 k a stage, not 64.  The fence between the planes and the
+// tensor core is that of shared memory alone: the general one also waits for the loads ahead.  Other forms were measured with six products and 64 k in an
+// accumulator, when the first product below took 56 us: the general fence 86, 8 warps with twice the work each 68, three stages ahead 61, lines asked
+// into the L2 six stages ahead 59.  128 rows a tile would leave no room for the accumulators, and were slower (2048 x 4096 x 2048: 299 against 283).
+// Against the FFMA kernel: [257, 2048] x [5632, 2048]^T 182 -> 71 us, [2048, 2048] x [4096, 2048]^T 679 -> 380, [777, 5632] x [2048, 5632]^T 482 -> 208,
+// [128, 2048] x [2048, 2048]^T 56 -> 20, [500, 999] x [1001, 999]^T 35 -> 22.  The first with an infinity or a row of NaN 118 us, with a column of NaN 108;
+// with some in most rows, so that most results are formed again, 590, and the second 2900: three to four and a half times the FFMA kernel's time.
 #include "gemm_f32_split.cuh"
 #include "tc_ptx.cuh"
 
@@ -36,10 +44,11 @@ using namespace ugb_tc;
 constexpr int BM = 128, BK = 32, WORKERS = 512, AHEAD = 2, WARPS = WORKERS / 32, THREADS = WORKERS + 32;
 constexpr int PLANE_P = BM * BK * 2;
 constexpr int RED_LD = BM;                 // floats between a tile's rows of q in shared memory
-constexpr int D_STRIDE = 128, TMEM_COLS = 512;        // hi hi of even and odd stages, the rest
+constexpr int REST_STAGES = 30;            // stages between two transfers of the rest, whole rounds of the workers' loop
+constexpr int D_STRIDE = 96, TMEM_COLS = 512;         // hi hi of the two 16 k of even and of odd stages, the rest
 
 template <int BN> struct Shape {
-  static constexpr int SLOTS = BN <= 96 ? 3 : 2;
+  static constexpr int SLOTS = 3;
   static constexpr int PLANE_Q = BN * BK * 2, STAGE = 3 * (PLANE_P + PLANE_Q), SMEM = SLOTS * STAGE + 1024;
 };
 
@@ -284,16 +293,18 @@ f32_split_kernel(const Params p) {
   const uint64_t pd = desc(smem_u32(smem), PK), qd = desc(smem_u32(smem) + 3 * PLANE_P, QK);
   constexpr uint32_t PSTEP = (PK ? 32 : 2048) >> 4, QSTEP = (QK ? 32 : 2048) >> 4, PP = PLANE_P >> 4, QP = S::PLANE_Q >> 4;
   auto multiply = [&](int s, int slot) { // one thread
-    const uint32_t d0 = tmem + (s >> 1 & 1) * D_STRIDE, d1 = tmem + 2 * D_STRIDE;
+    const uint32_t d0 = tmem + (s & 1) * 2 * D_STRIDE, d1 = tmem + 4 * D_STRIDE;
 #pragma unroll
     for (int j = 0; j < BK / UMMA_K; ++j) {
       const uint64_t a = pd + (uint32_t)slot * (S::STAGE >> 4) + j * PSTEP, b = qd + (uint32_t)slot * (S::STAGE >> 4) + j * QSTEP;
-      umma_bf16(d0, a, b, idesc, (s & 1) || j > 0);
-      umma_bf16(d1, a, b + QP, idesc, s > 0 || j > 0);
+      umma_bf16(d0 + j * D_STRIDE, a, b, idesc, 0);
+      umma_bf16(d1, a, b + QP, idesc, s % REST_STAGES > 0 || j > 0);
       umma_bf16(d1, a + PP, b, idesc, 1);
       umma_bf16(d1, a + PP, b + QP, idesc, 1);
       umma_bf16(d1, a, b + 2 * QP, idesc, 1);
       umma_bf16(d1, a + 2 * PP, b, idesc, 1);
+      umma_bf16(d1, a + PP, b + 2 * QP, idesc, 1);
+      umma_bf16(d1, a + 2 * PP, b + QP, idesc, 1);
     }
     umma_commit(smem_u32(&done[slot]));
   };
@@ -327,30 +338,42 @@ f32_split_kernel(const Params p) {
       oq.load(b, k_hi - k_lo - s * BK);
     };
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    auto add = [&](uint32_t from) {
+    auto add = [&](int s) {                // hi hi of stage s
+#pragma unroll
+      for (int j = 0; j < COLS; j += 8) {
+        uint32_t v[8], w[8];
+        const uint32_t at = tmem + lanes + (uint32_t)((s & 1) * 2 * D_STRIDE + col0 + j);
+        tmem_ld8(at, v);
+        tmem_ld8(at + D_STRIDE, w);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[j + e] += __uint_as_float(v[e]) + __uint_as_float(w[e]);
+      }
+    };
+    auto add_rest = [&]() {
 #pragma unroll
       for (int j = 0; j < COLS; j += 8) {
         uint32_t v[8];
-        tmem_ld8(tmem + lanes + from + (uint32_t)(col0 + j), v);
+        tmem_ld8(tmem + lanes + (uint32_t)(4 * D_STRIDE + col0 + j), v);
         tmem_ld_wait();
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[j + e] += __uint_as_float(v[e]);
       }
     };
     auto stage = [&](int s, int slot, float4 (&a)[OP::N], float4 (&b)[OQ::N]) {
-      const uint32_t parity = s / SLOTS & 1;
-      if (s >= SLOTS && alive) alive = wait(done[slot], parity ^ 1, 0x61);
       if (!alive) return;
       const uint32_t base = smem_u32(smem) + slot * S::STAGE;
       op.store(a, base, PLANE_P);
       oq.store(b, base + 3 * PLANE_P, S::PLANE_Q);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       if (s + AHEAD < stages) load(s + AHEAD, a, b);
-      // Stages come in pairs of 64 k; the pair before last is complete with the stage that was waited for, or before it, and its
-      // accumulator is the one that this stage starts anew.
-      if (!(s & 1) && s >= 4) {
+      // The stage before last: its accumulators are those that this stage starts anew, and the planes of the one before it, waited for
+      // one stage ago, were the ones just written.
+      if (s >= 2) {
+        alive = wait(done[(s - 2) % SLOTS], (s - 2) / SLOTS & 1, 0x61);
+        if (!alive) return;
         tcgen05_fence_after();
-        add((s >> 1 & 1) * D_STRIDE);
+        add(s);
         tcgen05_fence_before();
       }
       __syncwarp();
@@ -360,18 +383,25 @@ f32_split_kernel(const Params p) {
     for (int s = 0; s < AHEAD; ++s)
       if (s < stages) load(s, vp[s], vq[s]);
     constexpr int ROUND = SLOTS % AHEAD ? SLOTS * AHEAD : SLOTS;
-    for (int s = 0; s < stages; s += ROUND)
+    static_assert(REST_STAGES % ROUND == 0, "");
+    for (int s = 0; s < stages; s += ROUND) {
+      if (s > 0 && s % REST_STAGES == 0 && alive) {          // this stage starts the rest anew
+        alive = wait(done[(s - 1) % SLOTS], (s - 1) / SLOTS & 1, 0x65);
+        tcgen05_fence_after();
+        if (alive) add_rest();
+        tcgen05_fence_before();
+      }
 #pragma unroll
       for (int i = 0; i < ROUND; ++i)
         if (s + i < stages) stage(s + i, i % SLOTS, vp[i % AHEAD], vq[i % AHEAD]);
+    }
     if (stages > 0) {
       if (alive) alive = wait(done[(stages - 1) % SLOTS], (stages - 1) / SLOTS & 1, 0x63);   // and all before it
       tcgen05_fence_after();
-      const int pair = (stages - 1) >> 1;
-      if (alive && pair > 0) add((pair - 1 & 1) * D_STRIDE);
-      if (alive) add((pair & 1) * D_STRIDE);
+      if (alive && stages > 1) add(stages - 2);
+      if (alive) add(stages - 1);
+      if (alive) add_rest();
     }
-    if (stages > 0 && alive) add(2 * D_STRIDE);
     const uint32_t lp = __reduce_min_sync(0xffffffffu, op.least), lq = __reduce_min_sync(0xffffffffu, oq.least);
     const uint32_t both = abs_max(op.most, oq.most), top = __reduce_max_sync(0xffffffffu, max(both >> 16 & 0x7fffu, both & 0x7fffu));
     if (lane == 0) {
@@ -475,7 +505,6 @@ int32_t ugb_f32_split(ugb_device *dev, const ugb_f32_split_args &a, int bn, int 
     case 32: if (!qk) return UGB_ERR_UNSUPPORTED; e = launch_any<32>(dev, p, grid, pk, qk, vec, a.pdl); break;
     case 64: e = launch_any<64>(dev, p, grid, pk, qk, vec, a.pdl); break;
     case 96: if (!qk) return UGB_ERR_UNSUPPORTED; e = launch_any<96>(dev, p, grid, pk, qk, vec, a.pdl); break;
-    case 128: e = launch_any<128>(dev, p, grid, pk, qk, vec, a.pdl); break;
     default: return UGB_ERR_UNSUPPORTED;
   }
   if (e != cudaSuccess) return ugb_fail(dev, UGB_ERR_CUDA, "launch of f32_split_kernel failed: %s", cudaGetErrorString(e));

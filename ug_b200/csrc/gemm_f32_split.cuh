@@ -14,6 +14,6 @@ struct ugb_f32_split_args {
   bool pdl;
 };
 
-// On tiles of 128 x bn (32, 64, 96 or 128; 64 or 128 where q's rows are contiguous), k split over clusters of `split` CTAs (up to 8).
+// On tiles of 128 x bn (32, 64 or 96; 64 where q's rows are contiguous), k split over clusters of `split` CTAs (up to 8).
 // UGB_ERR_UNSUPPORTED (last_error untouched) for what it does not take.
 int32_t ugb_f32_split(ugb_device *dev, const ugb_f32_split_args &a, int bn, int split);
