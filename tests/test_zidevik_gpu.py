@@ -171,11 +171,12 @@ def test_wide_steps(dev, batch):
     m.close()
 
 
-@pytest.mark.parametrize("width,ffn,batch", [(264, 72, 1), (1024, 136, 8), (1544, 72, 8), (2112, 264, 3), (1024, None, 2)])
+@pytest.mark.parametrize("width,ffn,batch", [(264, 72, 1), (1024, 136, 8), (1544, 72, 8), (2112, 264, 3), (1024, None, 2),
+                                             (1024, 136, 9), (264, 72, 16), (1024, None, 9)])
 def test_steps_that_run_ahead(dev, width, ffn, batch):
     """Products, attention and experts' rows that run beside the kernels before them (up to two chunks of k with a warp that waits for
-    them, more chunks, k in several pieces, no shared feed-forward) give what they give one behind the other, bit by bit: where a
-    kernel waits changes no operand and no order of a sum."""
+    them, more chunks, k in several pieces, no shared feed-forward; attention and experts' rows beside products of more than 8 rows) give
+    what they give one behind the other, bit by bit: where a kernel waits changes no operand and no order of a sum."""
     cfg = Config(vocab=64, width=width, eps=1e-5, layers=[
         layer((4, 2, 64, 64, 64, 5000.0, 0.3), (256, 16, 4, 32), Experts(16, 2, 40, ffn)), layer((8, 2, 64, 64, 32, 900.0, 0.3), (1032, 8, 3, 16), 200)])
     w = separate_experts(cfg, synth.zidevik_weights(cfg, 502))
