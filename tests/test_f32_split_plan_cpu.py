@@ -70,17 +70,17 @@ def test_every_tile_and_cluster_is_reached():
 
 
 def test_short_k_and_next_to_nothing_stay_where_they_were(ask):
-    assert ask(1, 4932, 132, 95, 0)[0] == 0 and ask(1, 4096, 4096, 16, 1)[0] == 0 and ask(1, 4932, 132, 96, 0)[0] != 0
-    assert ask(1, 0, 5, 100, 0)[0] == 0 and ask(5, 3922, 8, 388, 0)[0] == 0 and ask(5, 3922, 33, 388, 0)[0] != 0
+    assert ask(1, 4932, 132, 99, 0)[0] == 0 and ask(1, 4096, 4096, 16, 1)[0] == 0 and ask(1, 4932, 132, 100, 0)[0] != 0
+    assert ask(1, 0, 5, 100, 0)[0] == 0 and ask(5, 3922, 8, 408, 0)[0] == 0 and ask(5, 3922, 33, 408, 0)[0] != 0
 
 
 @pytest.mark.parametrize("case", list(CHAINS))
 def test_chains_beside_which_errors_are_held(plan, case):
     (bn, split), (wm, wk, cluster, _) = plan(*case, 0)
-    assert CHAINS[case] == wk * cluster and case[3] >= 96 * wk * cluster and 6 * split >= wk * cluster
+    assert CHAINS[case] == wk * cluster and case[3] >= 100 * wk * cluster
 
 
-def test_short_chains_and_many_of_them_stay_with_ffma(plan):
-    for case in ((1, 128, 2048, 760), (1, 17, 5632, 2048), (8, 300, 64, 8192)):
+def test_short_chains_stay_with_ffma(plan):
+    for case in ((1, 128, 2048, 760), (1, 17, 5632, 2048), (1, 70, 3000, 300)):
         (bn, _), (_, wk, cluster, _) = plan(*case, 0)
         assert bn == 0, case

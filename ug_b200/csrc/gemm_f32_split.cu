@@ -3,16 +3,17 @@
 //
 //   x = hi + mid + lo     hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid: 8 bits each, nothing is lost
 //   a b = hi hi           16 products at a time, each time in an accumulator of its own, from where they are added up in f32 registers
-//       + hi mid + mid hi + mid mid + hi lo + lo hi + mid lo + lo mid          (2^-8 of it and less: one accumulator for 960 k)
+//       + hi mid + mid hi + mid mid + hi lo + lo hi + mid lo + lo mid          (2^-8 of it and less: an accumulator for 960 k)
 //       + lo lo                                              left out: 2^-33 of |a b|
 //
-// The tensor core cuts off what an FFMA rounds: of 16 products and the accumulator, what lies 2^-25 below the largest, and then their sum to
-// f32.  Sums of one sign lose a little of themselves every time, so nothing is added to hi hi there.  The error against 64 bits,
-// beside that of the FFMA kernel, by what is summed (2-norm, 257 x 1024 results):
+// The tensor core cuts off what an FFMA rounds: of 16 products and the accumulator what lies 2^-25 below the largest, then their sum to
+// f32 (sums formed that way on a CPU have the errors measured here).  Sums of one sign lose a little of themselves every time, so
+// nothing is added to hi hi there.  The error against 64 bits, beside that of the FFMA kernel, by what is summed (2-norm, 257 x 1024
+// results):
 //                                     k = 1000                2048                    4096
-//   normal                            8.1e-8 against 2.1e-7   9.8e-8 against 2.2e-7   1.2e-7 against 3.0e-7
-//   uniform in 0 .. 1                 4.6e-8 against 7.0e-8   5.2e-8 against 7.1e-8   5.9e-8 against 8.0e-8
-//   softmax (deviation 3) x uniform   9.7e-8 against 1.1e-7   1.0e-7 against 1.1e-7   1.1e-7 against 1.4e-7
+//   normal                            7.6e-8 against 2.1e-7   8.1e-8 against 2.2e-7   9.0e-8 against 3.0e-7
+//   uniform in 0 .. 1                 4.4e-8 against 7.0e-8   4.7e-8 against 7.1e-8   4.8e-8 against 8.0e-8
+//   softmax (deviation 3) x uniform   9.5e-8 against 1.1e-7   9.8e-8 against 1.1e-7   9.9e-8 against 1.4e-7
 // With 64 k in an accumulator and six products the last of these was 2.8e-7 to 3.0e-7.  At k = 64 it is 8e-8 here and 6e-8 with FFMA: see
 // ugb_f32_gemm_split_plan for the sums that stay there.
 //
@@ -22,18 +23,21 @@
 //
 // Tile: 128 columns of the result (lanes of the tensor memory: a warp stores whole lines) x BN rows.  16 warps read both operands, two
 // stages of 32 k ahead in registers, split them into the six swizzled shared-memory planes of a stage, and add what the tensor core
-// has finished to their f32 sums; a warp of its own issues (issued by one of the 16, its conversion and its issuing were in line, and
-// every stage waited for both).  Few tiles: CTAs of a cluster along k, sums through distributed shared memory in rank order.
+// has finished to their f32 sums: hi hi of a stage while its other products are formed.  Every six stages those sums go back into the
+// tensor memory, added to those of the stages before, so that no chain of additions is long.  A warp of its own issues (issued by one of the
+// 16, its conversion and its issuing were in line, and every stage waited for both).  Few tiles: CTAs of a cluster along k, sums through
+// distributed shared memory in rank order.
 //
 // Bound: the conversion (about ten instructions a value on 28 values per thread and stage), the products' own reads of shared memory
 // (an MMA of 128 x 96 x 16 takes 56 cycles for its operands, sixteen a stage) and the sums' way out of the tensor memory, 1.0 us a stage
-// together.  The loads wait in the L1, which is what the stages leave of 256 KB: 32 k a stage, not 64.  The fence between the planes and the
-// tensor core is that of shared memory alone: the general one also waits for the loads ahead.  Other forms were measured with six products and 64 k in an
-// accumulator, when the first product below took 56 us: the general fence 86, 8 warps with twice the work each 68, three stages ahead 61, lines asked
-// into the L2 six stages ahead 59.  128 rows a tile would leave no room for the accumulators, and were slower (2048 x 4096 x 2048: 299 against 283).
-// Against the FFMA kernel: [257, 2048] x [5632, 2048]^T 182 -> 71 us, [2048, 2048] x [4096, 2048]^T 679 -> 380, [777, 5632] x [2048, 5632]^T 482 -> 208,
-// [128, 2048] x [2048, 2048]^T 56 -> 20, [500, 999] x [1001, 999]^T 35 -> 22.  The first with an infinity or a row of NaN 118 us, with a column of NaN 108;
-// with some in most rows, so that most results are formed again, 590, and the second 2900: three to four and a half times the FFMA kernel's time.
+// together (with hi hi waited for together with the rest of its stage the first product below took 85 us).  The loads wait in the L1, which
+// is what the stages leave of 256 KB: 32 k a stage, not 64.  The fence between the planes and the tensor core is that of shared memory
+// alone: the general one also waits for the loads ahead.  Other forms were measured with six products and 64 k in an accumulator, when the
+// first product below took 56 us: the general fence 86, 8 warps with twice the work each 68, three stages ahead 61, lines asked into the
+// L2 six stages ahead 59, and tiles of 128 rows for 2048 x 4096 x 2048 299 against 283.
+// Against the FFMA kernel: [257, 2048] x [5632, 2048]^T 182 -> 73 us, [2048, 2048] x [4096, 2048]^T 679 -> 352, [777, 5632] x [2048, 5632]^T 482 -> 205,
+// [128, 2048] x [2048, 2048]^T 56 -> 20, [500, 999] x [1001, 999]^T 35 -> 22.  The first with an infinity or a row of NaN 120 us, with a column of NaN 111;
+// with some in most rows, so that most results are formed again, 595, and the second 2900: three to four and a half times the FFMA kernel's time.
 #include "gemm_f32_split.cuh"
 #include "tc_ptx.cuh"
 
@@ -44,8 +48,8 @@ using namespace ugb_tc;
 constexpr int BM = 128, BK = 32, WORKERS = 512, AHEAD = 2, WARPS = WORKERS / 32, THREADS = WORKERS + 32;
 constexpr int PLANE_P = BM * BK * 2;
 constexpr int RED_LD = BM;                 // floats between a tile's rows of q in shared memory
-constexpr int REST_STAGES = 30;            // stages between two transfers of the rest, whole rounds of the workers' loop
-constexpr int D_STRIDE = 96, TMEM_COLS = 512;         // hi hi of the two 16 k of even and of odd stages, the rest
+constexpr int GROUP = 6, REST = 30;        // stages whose sums stay in registers; between two transfers of the rest
+constexpr int D_STRIDE = 96, TMEM_COLS = 512;         // hi hi of the two 16 k of a stage, the rest, the sums of whole groups
 
 template <int BN> struct Shape {
   static constexpr int SLOTS = 3;
@@ -87,6 +91,10 @@ static __device__ __forceinline__ void st2(uint32_t at, uint32_t a, uint32_t b) 
 static __device__ __forceinline__ void tmem_ld8(uint32_t at, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(at) : "memory");
+}
+static __device__ __forceinline__ void tmem_st8(uint32_t at, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               :: "r"(at), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
 // R rows x 32 k of an operand in pieces of four values along its contiguous direction (KC: k), N of them per worker:
@@ -250,7 +258,7 @@ f32_split_kernel(const Params p) {
   constexpr int SLOTS = S::SLOTS, COLS = BN * 4 / WARPS;              // COLS: of a worker's sums
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t full[SLOTS], done[SLOTS], last;
+  __shared__ uint64_t full[SLOTS], lead[SLOTS], rest, last;               // lead: hi hi of a stage
   __shared__ uint32_t tmem_slot, least_p, least_q, most;
   __shared__ int aborted, again;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -261,8 +269,9 @@ f32_split_kernel(const Params p) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < SLOTS; ++i) {
       mbar_init(smem_u32(&full[i]), WARPS);
-      mbar_init(smem_u32(&done[i]), 1);
+      mbar_init(smem_u32(&lead[i]), 1);
     }
+    mbar_init(smem_u32(&rest), 1);
     mbar_init(smem_u32(&last), 1);
     aborted = again = 0;
     least_p = least_q = 0xffffffffu;
@@ -293,12 +302,15 @@ f32_split_kernel(const Params p) {
   const uint64_t pd = desc(smem_u32(smem), PK), qd = desc(smem_u32(smem) + 3 * PLANE_P, QK);
   constexpr uint32_t PSTEP = (PK ? 32 : 2048) >> 4, QSTEP = (QK ? 32 : 2048) >> 4, PP = PLANE_P >> 4, QP = S::PLANE_Q >> 4;
   auto multiply = [&](int s, int slot) { // one thread
-    const uint32_t d0 = tmem + (s & 1) * 2 * D_STRIDE, d1 = tmem + 4 * D_STRIDE;
+    const uint32_t d0 = tmem, d1 = tmem + 2 * D_STRIDE;
+    const uint64_t p0 = pd + (uint32_t)slot * (S::STAGE >> 4), q0 = qd + (uint32_t)slot * (S::STAGE >> 4);
+#pragma unroll
+    for (int j = 0; j < BK / UMMA_K; ++j) umma_bf16(d0 + j * D_STRIDE, p0 + j * PSTEP, q0 + j * QSTEP, idesc, 0);
+    umma_commit(smem_u32(&lead[slot]));
 #pragma unroll
     for (int j = 0; j < BK / UMMA_K; ++j) {
-      const uint64_t a = pd + (uint32_t)slot * (S::STAGE >> 4) + j * PSTEP, b = qd + (uint32_t)slot * (S::STAGE >> 4) + j * QSTEP;
-      umma_bf16(d0 + j * D_STRIDE, a, b, idesc, 0);
-      umma_bf16(d1, a, b + QP, idesc, s % REST_STAGES > 0 || j > 0);
+      const uint64_t a = p0 + j * PSTEP, b = q0 + j * QSTEP;
+      umma_bf16(d1, a, b + QP, idesc, s % REST > 0 || j > 0);
       umma_bf16(d1, a + PP, b, idesc, 1);
       umma_bf16(d1, a + PP, b + QP, idesc, 1);
       umma_bf16(d1, a, b + 2 * QP, idesc, 1);
@@ -306,7 +318,7 @@ f32_split_kernel(const Params p) {
       umma_bf16(d1, a + PP, b + 2 * QP, idesc, 1);
       umma_bf16(d1, a + 2 * PP, b + QP, idesc, 1);
     }
-    umma_commit(smem_u32(&done[slot]));
+    if (s + 1 == stages || (s + 1) % REST == 0) umma_commit(smem_u32(&rest));
   };
   const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * COLS;            // of this worker's sums
   const bool worker = warp < WARPS;
@@ -338,11 +350,11 @@ f32_split_kernel(const Params p) {
       oq.load(b, k_hi - k_lo - s * BK);
     };
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    auto add = [&](int s) {                // hi hi of stage s
+    auto add = [&]() {                     // hi hi of the last stage
 #pragma unroll
       for (int j = 0; j < COLS; j += 8) {
         uint32_t v[8], w[8];
-        const uint32_t at = tmem + lanes + (uint32_t)((s & 1) * 2 * D_STRIDE + col0 + j);
+        const uint32_t at = tmem + lanes + (uint32_t)(col0 + j);
         tmem_ld8(at, v);
         tmem_ld8(at + D_STRIDE, w);
         tmem_ld_wait();
@@ -350,30 +362,47 @@ f32_split_kernel(const Params p) {
         for (int e = 0; e < 8; ++e) acc[j + e] += __uint_as_float(v[e]) + __uint_as_float(w[e]);
       }
     };
-    auto add_rest = [&]() {
+    auto add_from = [&](uint32_t from) {   // 2: the rest; 3: the groups before, which no one else touches
 #pragma unroll
       for (int j = 0; j < COLS; j += 8) {
         uint32_t v[8];
-        tmem_ld8(tmem + lanes + (uint32_t)(4 * D_STRIDE + col0 + j), v);
+        tmem_ld8(tmem + lanes + from * D_STRIDE + (uint32_t)(col0 + j), v);
         tmem_ld_wait();
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[j + e] += __uint_as_float(v[e]);
       }
     };
-    auto stage = [&](int s, int slot, float4 (&a)[OP::N], float4 (&b)[OQ::N]) {
+    uint32_t rests = 0;                    // transfers of the rest so far
+    auto put_away = [&]() {
+#pragma unroll
+      for (int j = 0; j < COLS; j += 8) {
+        uint32_t v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { v[e] = __float_as_uint(acc[j + e]); acc[j + e] = 0.f; }
+        tmem_st8(tmem + lanes + (uint32_t)(3 * D_STRIDE + col0 + j), v);
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    };
+    auto stage = [&](int s, int slot, bool new_group, float4 (&a)[OP::N], float4 (&b)[OQ::N]) {
       if (!alive) return;
       const uint32_t base = smem_u32(smem) + slot * S::STAGE;
       op.store(a, base, PLANE_P);
       oq.store(b, base + 3 * PLANE_P, S::PLANE_Q);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       if (s + AHEAD < stages) load(s + AHEAD, a, b);
-      // The stage before last: its accumulators are those that this stage starts anew, and the planes of the one before it, waited for
-      // one stage ago, were the ones just written.
-      if (s >= 2) {
-        alive = wait(done[(s - 2) % SLOTS], (s - 2) / SLOTS & 1, 0x61);
+      // hi hi of the stage before, which this one starts anew; its other products are still being formed, and with it all of the stage before that
+      // is complete, whose planes the next stage writes over.
+      if (s >= 1) {
+        alive = wait(lead[(s - 1) % SLOTS], (s - 1) / SLOTS & 1, 0x61);
+        if (new_group && s % REST == 0 && alive) alive = wait(rest, rests++ & 1, 0x65);
         if (!alive) return;
         tcgen05_fence_after();
-        add(s);
+        add();
+        if (new_group) {
+          if (s % REST == 0) add_from(2);
+          if (s > GROUP) add_from(3);
+          put_away();
+        }
         tcgen05_fence_before();
       }
       __syncwarp();
@@ -382,25 +411,19 @@ f32_split_kernel(const Params p) {
 #pragma unroll
     for (int s = 0; s < AHEAD; ++s)
       if (s < stages) load(s, vp[s], vq[s]);
-    constexpr int ROUND = SLOTS % AHEAD ? SLOTS * AHEAD : SLOTS;
-    static_assert(REST_STAGES % ROUND == 0, "");
-    for (int s = 0; s < stages; s += ROUND) {
-      if (s > 0 && s % REST_STAGES == 0 && alive) {          // this stage starts the rest anew
-        alive = wait(done[(s - 1) % SLOTS], (s - 1) / SLOTS & 1, 0x65);
-        tcgen05_fence_after();
-        if (alive) add_rest();
-        tcgen05_fence_before();
-      }
+    static_assert(GROUP % SLOTS == 0 && GROUP % AHEAD == 0 && REST % GROUP == 0, "");
+    for (int s = 0; s < stages; s += GROUP)
 #pragma unroll
-      for (int i = 0; i < ROUND; ++i)
-        if (s + i < stages) stage(s + i, i % SLOTS, vp[i % AHEAD], vq[i % AHEAD]);
-    }
+      for (int i = 0; i < GROUP; ++i)
+        if (s + i < stages) stage(s + i, i % SLOTS, i == 0, vp[i % AHEAD], vq[i % AHEAD]);
     if (stages > 0) {
-      if (alive) alive = wait(done[(stages - 1) % SLOTS], (stages - 1) / SLOTS & 1, 0x63);   // and all before it
+      if (alive) alive = wait(rest, rests & 1, 0x63);        // and all before it
       tcgen05_fence_after();
-      if (alive && stages > 1) add(stages - 2);
-      if (alive) add(stages - 1);
-      if (alive) add_rest();
+      if (alive) {
+        add();
+        add_from(2);
+        if (stages > GROUP) add_from(3);
+      }
     }
     const uint32_t lp = __reduce_min_sync(0xffffffffu, op.least), lq = __reduce_min_sync(0xffffffffu, oq.least);
     const uint32_t both = abs_max(op.most, oq.most), top = __reduce_max_sync(0xffffffffu, max(both >> 16 & 0x7fffu, both & 0x7fffu));

@@ -84,28 +84,26 @@ inline ugb_f32_shape ugb_f32_gemm_shape(int sm_count, size_t b, size_t m, size_t
 // stages that widen with the tile and slow down a little as more SMs are at work, and the exchange of sums.  Clusters of 4 and 8 find fewer
 // SMs: those of a cluster have to be neighbours.
 //
-// Short sums stay with the FFMA kernel, whose error is smaller there.  It forms a result in `ways` chains; the tensor core's cut-off sums of
-// 16 products are ahead of chains of 96 additions and more whatever is summed.  Softmax probabilities with an exponent of deviation 3 times values of one
-// sign are the worst kind found: 1.35 times the FFMA kernel's error at chains of 16, 1.25 at 32, 1.03 at 64, 0.96 at 96; values of normal
-// distribution 0.63, 0.60, 0.54, 0.54 (2-norms against 64 bits, 90 sizes).  And k is split at least a sixth as often as there: deviation 8, 8 of [300, 8192] x [8192, 64] in 32
-// chains there, 4 CTAs along k here: 1.13.
-constexpr size_t UGB_F32_SPLIT_CHAIN = 96;
+// Short sums stay with the FFMA kernel, whose error may be the smaller one there.  It forms a result in wk * split chains of additions; the tensor
+// core's cut-off sums of 16 products are ahead of chains of 100 and more whatever is summed.  Worst are softmax probabilities (of
+// deviation 3 and 8) times values of one sign: at chains of 30 to 40 additions up to 1.26 times the FFMA kernel's error, 40 to 56 1.18, 56 to 80 1.09, 80 to
+// 96 1.04, above 0.93; values of normal distribution 0.4 to 0.5, uniform ones 0.7 to 0.8 (2-norms against 64 bits, 2400 products of 130 sizes).
+constexpr size_t UGB_F32_SPLIT_CHAIN = 100;
 struct ugb_f32_split_plan { int bn = 0, split = 1; };          // bn 0: not on the tensor cores
 inline ugb_f32_split_plan ugb_f32_gemm_split_plan(int sm_count, size_t b, size_t m, size_t n, size_t k, bool rows_contiguous) {
   ugb_f32_split_plan best;
   if (m == 0 || n == 0 || b == 0) return best;
   if (n <= 32 && n < m) return best;       // a quarter of the 128 lanes: the FFMA kernel's turned tiles (5 of [3922, 88] x [88, 8] 14.9 us here, 11.2 there)
   const ugb_f32_shape ffma = ugb_f32_gemm_shape(sm_count, b, m, n, k);
-  const int ways = ffma.wk * ffma.split;
-  if (k < UGB_F32_SPLIT_CHAIN * ways) return best;
+  if (k < UGB_F32_SPLIT_CHAIN * ffma.wk * ffma.split) return best;
   double least = 0.93 * (ffma.cost / 1900 + 2.5);
   for (int split = 1; split <= 8 && (split == 1 || k / split >= 64); split *= 2)
     for (int bn : {32, 64, 96}) {
-      if (6 * split < ways || (rows_contiguous && bn != 64)) continue;
+      if (rows_contiguous && bn != 64) continue;
       const size_t tiles = (n + 127) / 128 * ((m + bn - 1) / bn) * b * split, slots = std::max<size_t>(split, split <= 2 ? sm_count : sm_count * (split == 4 ? 92 : 75) / 100);
       if (split > 1 && tiles > slots) continue;                        // several rounds are better spent on whole sums (2048 x 4096 x 2048, 96 rows: 420 against 369)
       const double stages = (double)(((k + split - 1) / split + 31) / 32), busy = std::min(1.0, (double)tiles / sm_count);
-      const double us = 1.8 + (double)((tiles + slots - 1) / slots) * (3.4 + stages * (0.585 + 0.0049 * bn) * (0.908 + 0.092 * busy)) + (split > 1 ? 1.3 + 0.0155 * bn : 0);
+      const double us = 2.0 + (double)((tiles + slots - 1) / slots) * (3.6 + stages * (0.521 + 0.0056 * bn) * (0.9 + 0.1 * busy)) + (split > 1 ? 1.3 + 0.0145 * bn : 0);
       if (us < least) { least = us; best = {bn, split}; }
     }
   return best;
