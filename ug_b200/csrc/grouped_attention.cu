@@ -348,8 +348,9 @@ template <int DQ, int DV> cudaError_t launch_one(dim3 grid, int sms, cudaStream_
 
 int ugb_grouped_attention_splits(const ugb_grouped_attention_args &a, int sms) {
   const int pairs = a.rows * a.kv_heads * ((a.heads / a.kv_heads + 15) / 16);
-  // CTAs that are resident together; beside a product of few rows (early) one per SM, which is what finds room there (8 sequences of 544
-  // keys in 8 slices each 87.9 ms for a request of 32 steps, in 4 86.2, in 2 87.4)
+  // CTAs that are resident together; beside a product of few rows or the scan (early) one per SM, which is what finds room there (8 sequences of 544
+  // keys in 8 slices each 87.9 ms for a request of 32 steps, in 4 86.2, in 2 87.4; 8 layers, 8 of 8192 keys, 888, 881, 1028 us a step; beside the scan,
+  // 8 of 512 and of 8192 in 8 and 4 slices, 446 and 424, 611 and 596; worst 5 of 8192, 789 in the rule's 7 slices, 772 in 8)
   const int slots = a.early && ugb_skinny_rows((size_t)a.rows) ? sms : a.dq + a.dv <= 128 ? 4 * sms : 2 * sms;
   return std::max(1, std::min(UGB_GROUPED_MAX_SPLITS, slots / std::max(1, pairs)));
 }

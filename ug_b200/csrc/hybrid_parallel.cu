@@ -13,7 +13,7 @@
 //   [experts]  blocks: GEMM router, route;  expert_rows (rows by expert, times their weight);  grouped GEMMs up and down
 //   GEMM cat -> f32                                     output projections of mixer and feed-forward as one product
 //   row_update      stream += product + experts' rows;  copy -> T (token input or loop) or norm -> h
-//   (a step runs feed-forward, experts and attention ahead of the scan, see run())
+//   (a step runs feed-forward and experts ahead of the scan, and attention too where a layer has a gate | up product, see run())
 //   [token input]  GEMM gate;  token_gate (a step of few rows: inside proj);  GEMM proj -> f32;  row_update  stream += norm(product);  copy or norm
 // The factors of attention and scan are applied where their f32 results are rounded to T.  Products with a f32 result are
 // split over k in a step; the consumer sums the partials.
@@ -98,12 +98,13 @@ int32_t run(ugb_hybrid *m, ugb_hybrid_work &w, const int *tok, int t_block, int 
   ugb_device *dev = m->dev;
   const bool pdl = m->pdl != 0;
   // In a bf16 decode step every kernel lets its successor start only after its own wait: when a kernel starts, everything up
-  // to its predecessor's predecessor is complete (see row_update_kernel).  Attention beside the gate | up product is the one that does not:
-  // when its successor starts, that product may still run, and everything before it is complete.
+  // to its predecessor's predecessor is complete (see row_update_kernel).  Attention is the one that does not: when its
+  // successor starts, the kernel before it (the gate | up product or the scan) may still run, and everything before that is complete.
   const bool early = decode && pdl && !m->f32;
   // What does not depend on its predecessor runs beside it, and only its end waits: the gate | up product beside mixer_inputs
   // and the scan's input product beside attention or the experts' last product (a_ahead, up to 8 rows), attention beside the gate | up
-  // product, the experts' rows beside both (request 8x512+32: 94.3 -> 88.0 ms).  What runs ahead reads mixer_inputs' results and older ones,
+  // product or the scan, the experts' rows beside both (request 8x512+32: 94.3 -> 88.0 ms; 8 layers without a feed-forward, 8 sequences of 512
+  // keys, 473 -> 425 us a step for attention beside the scan).  What runs ahead reads mixer_inputs' results and older ones,
   // and writes what neither that product nor attention touches.
   const int B = m->batch, rows = B * t, wl = m->wl, n_runs = (int)m->runs.size();
   const bool whole = m->only == UGB_HYBRID_K_ALL;            // kernels timed alone leave the counts of the last whole pass as they are

@@ -8,7 +8,7 @@
 //     declared in gemm_tcgen05.cuh, and
 //   * for f32 (the dtype ug-llama casts every weight to, model.rs:118,140,313) two FP32-pipe kernels, a
 //     warp-per-column streaming kernel for the skinny products of a decode step and a register-blocked FFMA kernel
-//     for short k, and for the rest the tensor cores on three bf16 parts of every value (gemm_f32_split.cu), and
+//     for short sums, and for the rest the tensor cores on three bf16 parts of every value (gemm_f32_split.cu), and
 //   * the same FFMA kernel on 16-bit operands for the shapes and layouts the tensor-core kernels do not take.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
